@@ -167,7 +167,7 @@ def test_tiki_taka_benchmark_tile_deterministic():
             c_or = rt.get_weights()
         else:
             orc.update(X, Dm, lr)
-            a_or, c_or = orc.w_fast, orc.w
+            a_or, c_or = orc.a, orc.c
         a = t.get_hidden_parameters().numpy()[ia]
         c = t.get_weights().numpy()
         assert np.abs(a - a_or).max() <= 1e-6, f"fast tile, update {step}"
