@@ -339,6 +339,7 @@ void Tile::updateIndexed(const float *x, const float *d, long long total_input_s
     upd_gather_.idx = rowMajorIndices(m_batch, trans, s);
     upd_gather_.m_batch = m_batch;
     upd_gather_.ld = x_size_;
+    upd_gather_.idx_t = trans ? idx_ : nullptr;
     upd_gather_.image_size = in_mat;
     try {
       update(x, src, false, (int)b, false, false, s);

@@ -1,0 +1,245 @@
+// Pieces of the pulsed update that its kernels share: update management, pulse trains and the
+// device rules (one pulse with the clip behind it).
+#pragma once
+
+#include "mvm_common.cuh"
+#include "tile.h"
+
+namespace ab200 {
+
+__device__ __forceinline__ float blockMax(float v, float *sh) {
+  for (int o = 16; o > 0; o >>= 1) {
+    v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
+  }
+  int w = threadIdx.x >> 5;
+  if ((threadIdx.x & 31) == 0) {
+    sh[w] = v;
+  }
+  __syncthreads();
+  float r = 0.0f;
+  for (int i = 0; i < (int)(blockDim.x >> 5); i++) {
+    r = fmaxf(r, sh[i]);
+  }
+  __syncthreads();
+  return r;
+}
+
+// calculateBlAB + performUpdateManagement, fp32 with the reference's association
+// (rpu_pulsed_meta_parameter.cpp:153-236). BL == 0 means "no update for this sample".
+__device__ __forceinline__ void
+blAB(const UpEff &up, float lr, float dw_min, float xm, float dm, int &BL, float &A, float &B) {
+  if (lr == 0.0f) {
+    BL = 0;
+    A = B = 0.0f;
+    return;
+  }
+  if (up.fixed_bl || up.update_bl_management) {
+    BL = up.desired_bl;
+    A = __fsqrt_rn(__fdiv_rn(lr, __fmul_rn(dw_min, (float)BL)));
+    B = A;
+  } else {
+    if (__fmul_rn(dw_min, (float)up.desired_bl) < lr) {
+      A = B = 1.0f;
+      BL = max((int)ceilf(__fdiv_rn(lr, dw_min)), 1);
+    } else {
+      BL = up.desired_bl;
+      A = __fsqrt_rn(__fdiv_rn(lr, __fmul_rn(dw_min, (float)BL)));
+      B = A;
+    }
+  }
+  if (up.update_bl_management || up.update_management) {
+    if (xm == 0.0f || dm == 0.0f) {
+      BL = 0;
+      A = B = 1.0f;
+      return;
+    }
+    float x_val = xm;
+    float d_val = __fmul_rn(up.um_grad_scale, dm);
+    float k_val = __fdiv_rn(__fmul_rn(__fmul_rn(lr, x_val), d_val), dw_min);
+    if (up.update_bl_management) {
+      BL = (int)ceilf(k_val);
+      if (BL > up.desired_bl) {
+        BL = up.desired_bl;
+      }
+      A = __fsqrt_rn(__fdiv_rn(lr, __fmul_rn(dw_min, (float)BL)));
+      B = A;
+    }
+    if (up.update_management) {
+      if (k_val > (float)up.desired_bl) {
+        d_val = __fmul_rn(d_val, __fdiv_rn((float)up.desired_bl, k_val));
+      }
+      A = __fmul_rn(A, __fsqrt_rn(__fdiv_rn(x_val, d_val)));
+      B = __fmul_rn(B, __fsqrt_rn(__fdiv_rn(d_val, x_val)));
+    }
+  }
+}
+
+// A draw u of 16 bits gives a pulse when u + 0.5 < 65536 pp; as a comparison u < threshold of integers,
+// which keeps the draws off the conversion pipe.
+__device__ __forceinline__ int pulseThreshold(float pp) {
+  return __float2int_ru(__fadd_rn(__fmul_rn(pp, 65536.0f), -0.5f));
+}
+
+// One stochastic pulse train (generateCounts, sparse_bit_line_maker.cpp:200-238): BL Bernoulli
+// draws with probability pp; each draw compares pp against a 16-bit uniform, 8 draws per
+// Philox call. (A bit-serial comparison of all slots at once - one random word per bit of pp until
+// every slot is decided - needs fewer calls per lane but as many per warp, and measured slower.)
+__device__ __forceinline__ uint32_t
+pulseTrain(float pp, int BL, int seg, PhiloxKey key, uint32_t line, uint32_t sample, uint32_t call,
+           uint32_t tag) {
+  // slots [seg * 31, min(BL, seg * 31 + 31)) of the train, as bits 1.. of one word
+  const int k0 = seg * kPulseSegSlots;
+  const int nk = min(BL - k0, kPulseSegSlots);
+  const int thr = pulseThreshold(pp);
+  uint32_t bits = 0;
+  int k = 0;
+  for (int q = 0; q * 8 < nk; q++) {
+    uint32_t r[4];
+    philox4x32<7>(line, sample, call, tag + (uint32_t)(seg * 4 + q), key, r);
+#pragma unroll
+    for (int h = 0; h < 8; h++) {
+      const int u16 = (int)((r[h >> 1] >> ((h & 1) * 16)) & 0xFFFFu);
+      if (k < nk && u16 < thr) {
+        bits |= 1u << (k + 1);
+      }
+      k++;
+    }
+  }
+  return bits;
+}
+
+// getDiscretizedValue of a pulse probability (src/rpucuda/utility_functions.h:186-193): to the
+// nearest multiple of `res`, or - with sto_round - up or down at random in proportion to the
+// remainder; the uniform of a line is a function of (line, sample, call).
+__device__ __forceinline__ float
+pulseProb(const UpdateProblem &p, float v, float res, uint32_t line, uint32_t sample, uint32_t tag) {
+  if (!p.up.sto_round || !(res > 0.0f)) {
+    return discretize(v, res);
+  }
+  uint32_t r[4];
+  philox4x32<7>(line, sample, p.call, tag ^ 0x08000000u, p.key, r);
+  return __fmul_rn(rintf(__fadd_rn(__fdiv_rn(v, res), __fadd_rn(u01(r[0]), -0.5f))), res);
+}
+
+// ---------------------------------------------------------------------------------------------
+// device rules: one pulse, clipped immediately. `down` = weight decreases.
+// par4 = {scale_up, scale_down, max_bound, min_bound}
+// ---------------------------------------------------------------------------------------------
+template <int KIND>
+__device__ __forceinline__ float pulseOnce(float w, bool down, const float4 &q, const float2 &e,
+                                           float xi, int mult_noise, const float4 &es0,
+                                           const float4 &es1, const float *pw = nullptr,
+                                           int pw_n = 0) {
+  if (KIND == AB200_DEVICE_PIECEWISE_STEP) {
+    // PiecewiseStepRPUDevice update_once (rpu_piecewisestep_device.cpp:30-80): the step factor is
+    // interpolated linearly between pw_n nodes spread evenly over [min_bound, max_bound];
+    // pw[0..pw_n) are the up factors, pw[pw_n..2 pw_n) the down factors
+    const float *tab = down ? pw + pw_n : pw;
+    const int n_sec = pw_n - 1;
+    float f;
+    if (n_sec <= 0 || q.z <= q.w) {
+      f = __ldg(tab);
+    } else {
+      const float ws = fmaxf(
+          __fmul_rn(__fdiv_rn(__fsub_rn(w, q.w), __fsub_rn(q.z, q.w)), (float)n_sec), 0.0f);
+      const int idx = min((int)floorf(ws), n_sec - 1);
+      const float t = fminf(__fsub_rn(ws, (float)idx), 1.0f);
+      const float t1 = __fsub_rn(1.0f, t);
+      f = __fadd_rn(__fmul_rn(t1, __ldg(tab + idx)), __fmul_rn(t, __ldg(tab + idx + 1)));
+    }
+    const float step = __fmul_rn(__fmul_rn(down ? q.y : q.x, f), __fadd_rn(1.0f, xi));
+    w = down ? __fsub_rn(w, step) : __fadd_rn(w, step);
+    w = fmaxf(w, q.w);
+    w = fminf(w, q.z);
+    return w;
+  } else if (KIND == AB200_DEVICE_EXP_STEP) {
+    // ExpStepRPUDevice update_once / update_once_complex_noise (rpu_expstep_device.cpp:18-100):
+    // z = 2 w / (max - min) * a + b;  step = scale * max(1 - A exp(+-gamma z), 0)
+    // es0 = {a, b, A_up, A_down}, es1 = {gamma_up, gamma_down, std_add, std_slope}; xi = std * N
+    const float b_diff = __fsub_rn(q.z, q.w);
+    if (!(b_diff > 0.0f)) {
+      return w;
+    }
+    const float z = __fadd_rn(__fmul_rn(__fdiv_rn(__fmul_rn(2.0f, w), b_diff), es0.x), es0.y);
+    const float y = down ? fmaxf(__fsub_rn(1.0f, __fmul_rn(es0.w, expf(__fmul_rn(es1.y, -z)))), 0.0f)
+                         : fmaxf(__fsub_rn(1.0f, __fmul_rn(es0.z, expf(__fmul_rn(es1.x, z)))), 0.0f);
+    if (es1.z != 0.0f || es1.w != 0.0f) {
+      const float dw = down ? -__fmul_rn(y, q.y) : __fmul_rn(y, q.x);
+      const float spread =
+          __fadd_rn(__fadd_rn(fabsf(dw), es1.z), __fmul_rn(es1.w, fabsf(w)));
+      w = __fadd_rn(w, __fadd_rn(dw, __fmul_rn(spread, xi)));
+    } else {
+      const float step = __fmul_rn(__fmul_rn(y, __fadd_rn(1.0f, xi)), down ? q.y : q.x);
+      w = down ? __fsub_rn(w, step) : __fadd_rn(w, step);
+    }
+    w = fminf(w, q.z);
+    w = fmaxf(w, q.w);
+    return w;
+  } else if (KIND == AB200_DEVICE_POW_STEP) {
+    // PowStepRPUDevice update_once (rpu_powstep_device.cpp:91-121): the step shrinks with a power
+    // of the distance to the bound, e = {gamma_up, gamma_down}
+    const float range = __fsub_rn(q.z, q.w);
+    if (range == 0.0f) {
+      return w;
+    }
+    if (down) {
+      const float f = powf(__fdiv_rn(__fsub_rn(w, q.w), range), e.y);
+      w = __fsub_rn(w, __fmul_rn(__fmul_rn(q.y, f), __fadd_rn(1.0f, xi)));
+    } else {
+      const float f = powf(__fdiv_rn(__fsub_rn(q.z, w), range), e.x);
+      w = __fadd_rn(w, __fmul_rn(__fmul_rn(q.x, f), __fadd_rn(1.0f, xi)));
+    }
+    w = fmaxf(w, q.w);
+    w = fminf(w, q.z);
+    return w;
+  } else if (KIND == AB200_DEVICE_CONSTANT_STEP) {
+    float dw = __fmul_rn(__fadd_rn(1.0f, xi), down ? q.y : q.x);
+    w = down ? __fsub_rn(w, dw) : __fadd_rn(w, dw);
+    w = fminf(w, q.z);
+    w = fmaxf(w, q.w);
+    return w;
+  } else if (KIND == AB200_DEVICE_LINEAR_STEP) {
+    float slope = down ? e.y : e.x;
+    float sc = down ? q.y : q.x;
+    float dw;
+    if (mult_noise) {
+      dw = __fmul_rn(__fadd_rn(__fmul_rn(slope, w), sc), __fadd_rn(1.0f, xi));
+    } else {
+      dw = __fadd_rn(__fmul_rn(slope, w), __fmul_rn(sc, __fadd_rn(1.0f, xi)));
+    }
+    w = down ? __fsub_rn(w, dw) : __fadd_rn(w, dw);
+    w = fmaxf(w, q.w);
+    w = fminf(w, q.z);
+    return w;
+  } else { // SOFT_BOUNDS_REFERENCE
+    float ref = e.x;
+    w = __fadd_rn(w, ref);
+    float bound = down ? q.w : q.z;
+    bool ok = down ? (bound < 0.0f) : (bound > 0.0f);
+    float a = ok ? __fdiv_rn(w, bound) : 0.0f;
+    float sc = down ? q.y : q.x;
+    float dw;
+    if (mult_noise) {
+      dw = __fmul_rn(__fmul_rn(sc, __fsub_rn(1.0f, a)), __fadd_rn(1.0f, xi));
+    } else {
+      dw = __fmul_rn(sc, __fadd_rn(__fsub_rn(1.0f, a), xi));
+    }
+    w = down ? __fsub_rn(w, dw) : __fadd_rn(w, dw);
+    w = fmaxf(w, q.w);
+    w = fminf(w, q.z);
+    return __fsub_rn(w, ref);
+  }
+}
+
+// the same problem in rows of pulse words: a sample has nseg of them
+static inline UpdateProblem inRows(const UpdateProblem &p0) {
+  UpdateProblem p = p0;
+  const int nseg = p0.nseg > 0 ? p0.nseg : 1;
+  p.m = p0.m * nseg;
+  p.s_begin = p0.s_begin * nseg;
+  p.s_end = p0.s_end * nseg;
+  p.nseg = 1;
+  return p;
+}
+
+} // namespace ab200

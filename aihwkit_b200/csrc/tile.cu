@@ -640,9 +640,9 @@ Tile::~Tile() {
     cudaFree(drift_w0_);
     cudaFree(drift_t_);
     cudaFree(drift_nu_);
-    cudaFree(xls_);
-    cudaFree(xlx_);
-    cudaFree(xloff_);
+    cudaFree(plane_bl_);
+    cudaFree(plane_nk_);
+    cudaFree(plane_ab_);
     cudaFree(chop_in_);
     cudaFree(chop_out_);
     cudaFree(nm_state_);
@@ -654,8 +654,6 @@ Tile::~Tile() {
     cudaFree(b_onv_);
     cudaFree(xw_);
     cudaFree(dw_);
-    cudaFree(xwt_);
-    cudaFree(xnzt_);
     cudaFree(onehot_);
     cudaFree(tread_);
     cudaFree(t_words_);
@@ -949,7 +947,13 @@ void Tile::ensureScratch(int m) {
   cudaFree(flags_);
   cudaFree(xw_);
   cudaFree(dw_);
-  int cap = m + m / 4 + 16;
+  cudaFree(plane_bl_);
+  cudaFree(plane_nk_);
+  cudaFree(plane_ab_);
+  plane_bl_ = plane_nk_ = nullptr;
+  plane_ab_ = nullptr;
+  // whole blocks of 32 rows: the bit planes of the pulse trains come in those
+  int cap = (m + m / 4 + 16 + 31) / 32 * 32;
   AB200_CUDA(cudaMalloc(&scale_, (size_t)cap * sizeof(float)));
   AB200_CUDA(cudaMalloc(&factor_, (size_t)cap * sizeof(float)));
   AB200_CUDA(cudaMalloc(&vnorm_, (size_t)cap * sizeof(float)));
@@ -961,29 +965,11 @@ void Tile::ensureScratch(int m) {
   if (cfg_.device_kind != AB200_DEVICE_IDEAL && up_.pulse_type != AB200_PULSE_NONE) {
     AB200_CUDA(cudaMalloc(&xw_, (size_t)cap * x_size_ * sizeof(uint32_t)));
     AB200_CUDA(cudaMalloc(&dw_, (size_t)cap * d_size_ * sizeof(uint32_t)));
+    AB200_CUDA(cudaMalloc(&plane_bl_, (size_t)cap * sizeof(int)));
+    AB200_CUDA(cudaMalloc(&plane_nk_, (size_t)(cap / 32 + 1) * sizeof(int)));
+    AB200_CUDA(cudaMalloc(&plane_ab_, (size_t)cap * sizeof(float2)));
   }
   scratch_m_ = cap;
-}
-
-void Tile::ensureStreamScratch(int m_pad) {
-  const size_t need = (size_t)m_pad * x_size_;
-  if (need <= xwt_words_) {
-    return;
-  }
-  AB200_CUDA(cudaDeviceSynchronize());
-  cudaFree(xwt_);
-  cudaFree(xnzt_);
-  cudaFree(xls_);
-  cudaFree(xlx_);
-  cudaFree(xloff_);
-  xwt_ = xnzt_ = xls_ = xlx_ = xloff_ = nullptr;
-  const size_t cap = need + need / 8;
-  AB200_CUDA(cudaMalloc(&xwt_, cap * sizeof(uint32_t)));
-  AB200_CUDA(cudaMalloc(&xnzt_, (cap / 32 + x_size_) * sizeof(uint32_t)));
-  AB200_CUDA(cudaMalloc(&xls_, cap * sizeof(uint32_t)));
-  AB200_CUDA(cudaMalloc(&xlx_, cap * sizeof(uint32_t)));
-  AB200_CUDA(cudaMalloc(&xloff_, (cap / 32 + 2 * (size_t)x_size_) * sizeof(uint32_t)));
-  xwt_words_ = cap;
 }
 
 void Tile::ensureStage(size_t n_floats) {
@@ -1859,17 +1845,23 @@ void Tile::updateCore(const float *x, long long x_ss, long long x_fs, int x_in, 
     u.chop_d = chop_out_;
   }
   u.gather = upd_gather_;
-  launchPulsePrepare(u, s);
-  const bool stream_upd = streamUpdateEligible(u);
-  const int m_pad = (m * u.nseg + 31) / 32 * 32;
-  if (stream_upd) {
-    ensureStreamScratch(m_pad);
-    launchPulseTranspose(u, xwt_, xnzt_, m_pad, s);
-    launchPulseCompact(u, xwt_, xnzt_, m_pad, xls_, xlx_, xloff_, s);
+  u.plane_bl = plane_bl_;
+  u.plane_ab = plane_ab_;
+  u.plane_nk = plane_nk_ ? plane_nk_ + 1 : nullptr; // the first word holds the longest of all
+  u.plane_max = plane_nk_;
+  const bool planes = streamUpdateEligible(u);
+  if (!planes || pulses_up_) {
+    launchPulsePrepare(u, s);
+  }
+  if (pulses_up_) { // single devices only: counted on the pulse words, which the planes then replace
+    launchPulseCounter(u, pulses_up_, pulses_down_, s);
+  }
+  if (planes) {
+    launchPulsePlanes(u, s);
   }
   auto applyRange = [&](UpdateProblem &r) {
-    if (stream_upd) {
-      launchPulsedUpdateStream(r, xwt_, xnzt_, m_pad, s, xls_, xlx_, xloff_);
+    if (planes) {
+      launchPulsedUpdatePlanes(r, s);
     } else {
       launchPulsedUpdate(r, s);
     }
@@ -1877,9 +1869,6 @@ void Tile::updateCore(const float *x, long long x_ss, long long x_fs, int x_in, 
 
   if (cfg_.device_kind != AB200_DEVICE_TRANSFER) {
     u.w = w_;
-    if (pulses_up_) {
-      launchPulseCounter(u, pulses_up_, pulses_down_, s);
-    }
     applyRange(u);
     return;
   }

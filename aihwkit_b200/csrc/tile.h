@@ -89,6 +89,7 @@ struct RowGather {
   int m_batch = 0;
   int ld = 0;
   long long image_size = 0; // elements between two images
+  const int32_t *idx_t = nullptr; // the same array as [ld][m_batch], where the caller's has that order
 };
 
 struct MvmProblem {
@@ -188,6 +189,12 @@ struct UpdateProblem {
   // scratch
   uint32_t *xw; // [m][x_size] pulse words (or float bit patterns for implicit pulses)
   uint32_t *dw; // [m][d_size]
+  // stochastic trains on bit planes (update_planes.cu): xw / dw then hold [rows / 32][32][lines], and per
+  // sample the train length and the factors {A, B}, per block of 32 rows the longest train, and the
+  // longest of all (zero where none is longer than three slots)
+  int *plane_bl;
+  float2 *plane_ab;
+  int *plane_nk, *plane_max;
   // target
   float *w;
   const float4 *par4;
@@ -207,23 +214,15 @@ struct UpdateProblem {
 };
 
 void launchPulsePrepare(const UpdateProblem &p, cudaStream_t stream);
-// Stochastic pulse trains: the update streams over the non-empty samples of an x-line (transposed
-// x words, their bitmaps and compacted lists) instead of staging blocks of samples per weight
-// tile. Measured faster from a batch of 64 (256 x 256 tile) upwards; below one bitmap word of
-// samples the three extra launches are not worth it.
+// Stochastic pulse trains: the update works on bit planes of 32 rows (update_planes.cu). Below one block of
+// rows the planes are mostly empty and the staged kernel's two launches are the shorter way.
 constexpr int kStreamUpdateMinBatch = 32;
 bool streamUpdateEligible(const UpdateProblem &p);
 // kernel selection of the pulsed update: 0 = automatic, 1 = always the staged kernel, 2 = the
-// streaming kernel whenever the pulse type allows it (any batch size)
+// bit-plane kernel whenever the pulse type allows it (any batch size)
 void setUpdatePath(int mode);
-void launchPulseTranspose(const UpdateProblem &p, uint32_t *xwT, uint32_t *xnzT, int m_pad,
-                          cudaStream_t stream);
-// compacted (sample, word) lists of every x-line, from the transposed words and their bitmaps
-void launchPulseCompact(const UpdateProblem &p, const uint32_t *xwT, const uint32_t *xnzT, int m_pad,
-                        uint32_t *list_s, uint32_t *list_x, uint32_t *list_off, cudaStream_t stream);
-void launchPulsedUpdateStream(const UpdateProblem &p, const uint32_t *xwT, const uint32_t *xnzT,
-                              int m_pad, cudaStream_t stream, const uint32_t *list_s,
-                              const uint32_t *list_x, const uint32_t *list_off);
+void launchPulsePlanes(const UpdateProblem &p, cudaStream_t stream);
+void launchPulsedUpdatePlanes(const UpdateProblem &p, cudaStream_t stream);
 void launchPulsedUpdate(const UpdateProblem &p, cudaStream_t stream);
 void launchCoincidences(const UpdateProblem &p, int32_t *counts_dx, cudaStream_t stream);
 // pulses of the samples [s_begin, s_end) of a prepared batch, added per weight to `up` (the weight
@@ -454,7 +453,6 @@ private:
     std::uniform_real_distribution<float> ud{0.0f, 1.0f};
     float uniform() { return ud(gen); }
   } chop_rng_;
-  uint32_t *xls_ = nullptr, *xlx_ = nullptr, *xloff_ = nullptr; // compacted x lists (stream update)
   // per-line tables of a direction (MVParameter, rpu_forward_backward_pass.h:14-22)
   struct LineTables {
     std::vector<float> h_voff, h_nl, h_onv;
@@ -478,10 +476,9 @@ private:
   float *drift_prev_ = nullptr, *drift_w0_ = nullptr, *drift_t_ = nullptr, *drift_nu_ = nullptr;
   float drift_now_ = 0.0f;
   uint32_t *xw_ = nullptr, *dw_ = nullptr;
-  // transposed x words [x_size][m_pad] and their bitmaps, for the streaming update of large batches
-  uint32_t *xwt_ = nullptr, *xnzt_ = nullptr;
-  size_t xwt_words_ = 0;
-  void ensureStreamScratch(int m_pad);
+  // bit-plane update: per-sample train parameters, longest train per 32 rows
+  int *plane_bl_ = nullptr, *plane_nk_ = nullptr;
+  float2 *plane_ab_ = nullptr;
   float *onehot_ = nullptr, *tread_ = nullptr;
   uint32_t *t_words_ = nullptr; // Tiki-Taka write: pulse words of its single sample
   // tensor-core engines (forward / backward operand caches), rebuilt when the weights change

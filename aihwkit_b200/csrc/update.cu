@@ -16,118 +16,9 @@
 //   ConstantStep           src/rpucuda/rpu_constantstep_device.cpp:28-78
 //   LinearStep/SoftBounds  src/rpucuda/rpu_linearstep_device.cpp:113-164
 //   SoftBoundsReference    src/rpucuda/rpu_softbounds_reference_device.cpp:107-175
-#include "mvm_common.cuh"
-#include "tile.h"
+#include "pulse_common.cuh"
 
 namespace ab200 {
-
-__device__ __forceinline__ float blockMax(float v, float *sh) {
-  for (int o = 16; o > 0; o >>= 1) {
-    v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
-  }
-  int w = threadIdx.x >> 5;
-  if ((threadIdx.x & 31) == 0) {
-    sh[w] = v;
-  }
-  __syncthreads();
-  float r = 0.0f;
-  for (int i = 0; i < (int)(blockDim.x >> 5); i++) {
-    r = fmaxf(r, sh[i]);
-  }
-  __syncthreads();
-  return r;
-}
-
-// calculateBlAB + performUpdateManagement, fp32 with the reference's association
-// (rpu_pulsed_meta_parameter.cpp:153-236). BL == 0 means "no update for this sample".
-__device__ __forceinline__ void
-blAB(const UpEff &up, float lr, float dw_min, float xm, float dm, int &BL, float &A, float &B) {
-  if (lr == 0.0f) {
-    BL = 0;
-    A = B = 0.0f;
-    return;
-  }
-  if (up.fixed_bl || up.update_bl_management) {
-    BL = up.desired_bl;
-    A = __fsqrt_rn(__fdiv_rn(lr, __fmul_rn(dw_min, (float)BL)));
-    B = A;
-  } else {
-    if (__fmul_rn(dw_min, (float)up.desired_bl) < lr) {
-      A = B = 1.0f;
-      BL = max((int)ceilf(__fdiv_rn(lr, dw_min)), 1);
-    } else {
-      BL = up.desired_bl;
-      A = __fsqrt_rn(__fdiv_rn(lr, __fmul_rn(dw_min, (float)BL)));
-      B = A;
-    }
-  }
-  if (up.update_bl_management || up.update_management) {
-    if (xm == 0.0f || dm == 0.0f) {
-      BL = 0;
-      A = B = 1.0f;
-      return;
-    }
-    float x_val = xm;
-    float d_val = __fmul_rn(up.um_grad_scale, dm);
-    float k_val = __fdiv_rn(__fmul_rn(__fmul_rn(lr, x_val), d_val), dw_min);
-    if (up.update_bl_management) {
-      BL = (int)ceilf(k_val);
-      if (BL > up.desired_bl) {
-        BL = up.desired_bl;
-      }
-      A = __fsqrt_rn(__fdiv_rn(lr, __fmul_rn(dw_min, (float)BL)));
-      B = A;
-    }
-    if (up.update_management) {
-      if (k_val > (float)up.desired_bl) {
-        d_val = __fmul_rn(d_val, __fdiv_rn((float)up.desired_bl, k_val));
-      }
-      A = __fmul_rn(A, __fsqrt_rn(__fdiv_rn(x_val, d_val)));
-      B = __fmul_rn(B, __fsqrt_rn(__fdiv_rn(d_val, x_val)));
-    }
-  }
-}
-
-// One stochastic pulse train (generateCounts, sparse_bit_line_maker.cpp:200-238): BL Bernoulli
-// draws with probability pp; each draw compares pp against a 16-bit uniform, 8 draws per
-// Philox call. (A bit-serial comparison of all slots at once - one random word per bit of pp until
-// every slot is decided - needs fewer calls per lane but as many per warp, and measured slower.)
-__device__ __forceinline__ uint32_t
-pulseTrain(float pp, int BL, int seg, PhiloxKey key, uint32_t line, uint32_t sample, uint32_t call,
-           uint32_t tag) {
-  // slots [seg * 31, min(BL, seg * 31 + 31)) of the train, as bits 1.. of one word
-  const int k0 = seg * kPulseSegSlots;
-  const int nk = min(BL - k0, kPulseSegSlots);
-  float thr = pp * 65536.0f;
-  uint32_t bits = 0;
-  int k = 0;
-  for (int q = 0; q * 8 < nk; q++) {
-    uint32_t r[4];
-    philox4x32<7>(line, sample, call, tag + (uint32_t)(seg * 4 + q), key, r);
-#pragma unroll
-    for (int h = 0; h < 8; h++) {
-      uint32_t u16 = (r[h >> 1] >> ((h & 1) * 16)) & 0xFFFFu;
-      if (k < nk && ((float)u16 + 0.5f) < thr) {
-        bits |= 1u << (k + 1);
-      }
-      k++;
-    }
-  }
-  return bits;
-}
-
-// getDiscretizedValue of a pulse probability (src/rpucuda/utility_functions.h:186-193): to the
-// nearest multiple of `res`, or - with sto_round - up or down at random in proportion to the
-// remainder; the uniform of a line is a function of (line, sample, call).
-__device__ __forceinline__ float
-pulseProb(const UpdateProblem &p, float v, float res, uint32_t line, uint32_t sample, uint32_t tag) {
-  if (!p.up.sto_round || !(res > 0.0f)) {
-    return discretize(v, res);
-  }
-  uint32_t r[4];
-  philox4x32<7>(line, sample, p.call, tag ^ 0x08000000u, p.key, r);
-  return __fmul_rn(rintf(__fadd_rn(__fdiv_rn(v, res), __fadd_rn(u01(r[0]), -0.5f))), res);
-}
 
 __global__ void __launch_bounds__(256) pulsePrepareKernel(UpdateProblem p) {
   pdlEnter();
@@ -236,116 +127,6 @@ __global__ void __launch_bounds__(256) pulsePrepareKernel(UpdateProblem p) {
       continue;
     }
     (is_x ? xw : dw)[idx] = word;
-  }
-}
-
-// ---------------------------------------------------------------------------------------------
-// device rules: one pulse, clipped immediately. `down` = weight decreases.
-// par4 = {scale_up, scale_down, max_bound, min_bound}
-// ---------------------------------------------------------------------------------------------
-template <int KIND>
-__device__ __forceinline__ float pulseOnce(float w, bool down, const float4 &q, const float2 &e,
-                                           float xi, int mult_noise, const float4 &es0,
-                                           const float4 &es1, const float *pw = nullptr,
-                                           int pw_n = 0) {
-  if (KIND == AB200_DEVICE_PIECEWISE_STEP) {
-    // PiecewiseStepRPUDevice update_once (rpu_piecewisestep_device.cpp:30-80): the step factor is
-    // interpolated linearly between pw_n nodes spread evenly over [min_bound, max_bound];
-    // pw[0..pw_n) are the up factors, pw[pw_n..2 pw_n) the down factors
-    const float *tab = down ? pw + pw_n : pw;
-    const int n_sec = pw_n - 1;
-    float f;
-    if (n_sec <= 0 || q.z <= q.w) {
-      f = __ldg(tab);
-    } else {
-      const float ws = fmaxf(
-          __fmul_rn(__fdiv_rn(__fsub_rn(w, q.w), __fsub_rn(q.z, q.w)), (float)n_sec), 0.0f);
-      const int idx = min((int)floorf(ws), n_sec - 1);
-      const float t = fminf(__fsub_rn(ws, (float)idx), 1.0f);
-      const float t1 = __fsub_rn(1.0f, t);
-      f = __fadd_rn(__fmul_rn(t1, __ldg(tab + idx)), __fmul_rn(t, __ldg(tab + idx + 1)));
-    }
-    const float step = __fmul_rn(__fmul_rn(down ? q.y : q.x, f), __fadd_rn(1.0f, xi));
-    w = down ? __fsub_rn(w, step) : __fadd_rn(w, step);
-    w = fmaxf(w, q.w);
-    w = fminf(w, q.z);
-    return w;
-  } else if (KIND == AB200_DEVICE_EXP_STEP) {
-    // ExpStepRPUDevice update_once / update_once_complex_noise (rpu_expstep_device.cpp:18-100):
-    // z = 2 w / (max - min) * a + b;  step = scale * max(1 - A exp(+-gamma z), 0)
-    // es0 = {a, b, A_up, A_down}, es1 = {gamma_up, gamma_down, std_add, std_slope}; xi = std * N
-    const float b_diff = __fsub_rn(q.z, q.w);
-    if (!(b_diff > 0.0f)) {
-      return w;
-    }
-    const float z = __fadd_rn(__fmul_rn(__fdiv_rn(__fmul_rn(2.0f, w), b_diff), es0.x), es0.y);
-    const float y = down ? fmaxf(__fsub_rn(1.0f, __fmul_rn(es0.w, expf(__fmul_rn(es1.y, -z)))), 0.0f)
-                         : fmaxf(__fsub_rn(1.0f, __fmul_rn(es0.z, expf(__fmul_rn(es1.x, z)))), 0.0f);
-    if (es1.z != 0.0f || es1.w != 0.0f) {
-      const float dw = down ? -__fmul_rn(y, q.y) : __fmul_rn(y, q.x);
-      const float spread =
-          __fadd_rn(__fadd_rn(fabsf(dw), es1.z), __fmul_rn(es1.w, fabsf(w)));
-      w = __fadd_rn(w, __fadd_rn(dw, __fmul_rn(spread, xi)));
-    } else {
-      const float step = __fmul_rn(__fmul_rn(y, __fadd_rn(1.0f, xi)), down ? q.y : q.x);
-      w = down ? __fsub_rn(w, step) : __fadd_rn(w, step);
-    }
-    w = fminf(w, q.z);
-    w = fmaxf(w, q.w);
-    return w;
-  } else if (KIND == AB200_DEVICE_POW_STEP) {
-    // PowStepRPUDevice update_once (rpu_powstep_device.cpp:91-121): the step shrinks with a power
-    // of the distance to the bound, e = {gamma_up, gamma_down}
-    const float range = __fsub_rn(q.z, q.w);
-    if (range == 0.0f) {
-      return w;
-    }
-    if (down) {
-      const float f = powf(__fdiv_rn(__fsub_rn(w, q.w), range), e.y);
-      w = __fsub_rn(w, __fmul_rn(__fmul_rn(q.y, f), __fadd_rn(1.0f, xi)));
-    } else {
-      const float f = powf(__fdiv_rn(__fsub_rn(q.z, w), range), e.x);
-      w = __fadd_rn(w, __fmul_rn(__fmul_rn(q.x, f), __fadd_rn(1.0f, xi)));
-    }
-    w = fmaxf(w, q.w);
-    w = fminf(w, q.z);
-    return w;
-  } else if (KIND == AB200_DEVICE_CONSTANT_STEP) {
-    float dw = __fmul_rn(__fadd_rn(1.0f, xi), down ? q.y : q.x);
-    w = down ? __fsub_rn(w, dw) : __fadd_rn(w, dw);
-    w = fminf(w, q.z);
-    w = fmaxf(w, q.w);
-    return w;
-  } else if (KIND == AB200_DEVICE_LINEAR_STEP) {
-    float slope = down ? e.y : e.x;
-    float sc = down ? q.y : q.x;
-    float dw;
-    if (mult_noise) {
-      dw = __fmul_rn(__fadd_rn(__fmul_rn(slope, w), sc), __fadd_rn(1.0f, xi));
-    } else {
-      dw = __fadd_rn(__fmul_rn(slope, w), __fmul_rn(sc, __fadd_rn(1.0f, xi)));
-    }
-    w = down ? __fsub_rn(w, dw) : __fadd_rn(w, dw);
-    w = fmaxf(w, q.w);
-    w = fminf(w, q.z);
-    return w;
-  } else { // SOFT_BOUNDS_REFERENCE
-    float ref = e.x;
-    w = __fadd_rn(w, ref);
-    float bound = down ? q.w : q.z;
-    bool ok = down ? (bound < 0.0f) : (bound > 0.0f);
-    float a = ok ? __fdiv_rn(w, bound) : 0.0f;
-    float sc = down ? q.y : q.x;
-    float dw;
-    if (mult_noise) {
-      dw = __fmul_rn(__fmul_rn(sc, __fsub_rn(1.0f, a)), __fadd_rn(1.0f, xi));
-    } else {
-      dw = __fmul_rn(sc, __fadd_rn(__fsub_rn(1.0f, a), xi));
-    }
-    w = down ? __fsub_rn(w, dw) : __fadd_rn(w, dw);
-    w = fmaxf(w, q.w);
-    w = fminf(w, q.z);
-    return __fsub_rn(w, ref);
   }
 }
 
@@ -667,288 +448,6 @@ static void launchUpdateInstance(const UpdateProblem &p, dim3 grid, cudaStream_t
   }
 }
 
-// ---------------------------------------------------------------------------------------------
-// Stochastic pulse trains: the update as a stream over the samples of one x-line.
-//
-// A warp owns 32 consecutive d-lines of ONE x-line. The x-line's pulse words are the same for all
-// its lanes, so the walk over the samples is uniform across the warp: it visits the samples
-// where the x word is not empty (a compacted list per x-line, built from the transposed x words
-// and their bitmaps), loads the 32 d words of that sample with one coalesced access, and every
-// lane counts its coincidences with AND + popc. No lane waits for another lane's candidates. The
-// rare expensive part - applying the pulses - is decoupled: a lane queues its events (count,
-// direction) and the warp applies the queued events together, so that most lanes have work in
-// every round.
-// ---------------------------------------------------------------------------------------------
-constexpr int USP_POOL = 256; // Gaussians per warp pool (eight per lane and refill)
-
-// xwT[line][sample] = xw[sample][line] for one 32 x 32 tile, plus the line's bitmap word of the
-// non-empty samples
-__global__ void __launch_bounds__(256)
-    pulseTransposeKernel(const uint32_t *words, int n_lines, int m, int m_pad, uint32_t *wordsT,
-                         uint32_t *nzT) {
-  pdlEnter();
-  __shared__ uint32_t tile[32][33];
-  const int l0 = blockIdx.x * 32, s0 = blockIdx.y * 32;
-  for (int r = threadIdx.y; r < 32; r += 8) {
-    const int s = s0 + r, l = l0 + threadIdx.x;
-    tile[r][threadIdx.x] = (s < m && l < n_lines) ? words[(long long)s * n_lines + l] : 0u;
-  }
-  __syncthreads();
-  for (int r = threadIdx.y; r < 32; r += 8) {
-    const int l = l0 + r, sidx = s0 + threadIdx.x;
-    const uint32_t w = tile[threadIdx.x][r];
-    const uint32_t nz = __ballot_sync(0xffffffffu, w != 0u);
-    if (l < n_lines) {
-      wordsT[(long long)l * m_pad + sidx] = w;
-      if (threadIdx.x == 0) {
-        nzT[(long long)l * (m_pad / 32) + blockIdx.y] = nz;
-      }
-    }
-  }
-}
-
-struct StreamUpdate {
-  const uint32_t *xwT; // [x_size][m_pad]
-  const uint32_t *xnzT; // [x_size][m_pad / 32]
-  int m_pad;
-  // compacted form of the same: per x-line the samples whose word is not empty, in order, and
-  // their words with the sign bit flipped ([x_size][m_pad] each), and the number of entries before
-  // every bitmap word ([x_size][m_pad / 32 + 1])
-  const uint32_t *list_s, *list_x, *list_off;
-};
-
-// Compaction of the transposed x words of a line: the streaming kernel then reads (sample, word)
-// pairs instead of walking a bitmap. One warp per line and segment of UCS_SEG_WORDS bitmap words;
-// the warp first counts the entries of the line's earlier segments (a sum of popcounts over the
-// bitmap, which stays in L2), then handles its bitmap words one at a time with the whole warp
-// (lane = sample), so reads and writes are contiguous.
-constexpr int UCS_SEG_WORDS = 128; // 4096 samples per warp
-
-__global__ void __launch_bounds__(256)
-    pulseCompactKernel(const uint32_t *wordsT, const uint32_t *nzT, int n_lines, int m_pad,
-                       uint32_t *list_s, uint32_t *list_x, uint32_t *list_off) {
-  pdlEnter();
-  const int nw = m_pad >> 5;
-  const int n_seg = (nw + UCS_SEG_WORDS - 1) / UCS_SEG_WORDS;
-  const long long wid = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (wid >= (long long)n_lines * n_seg) {
-    return;
-  }
-  const int line = (int)(wid / n_seg), seg = (int)(wid - (long long)line * n_seg);
-  const uint32_t *nz = nzT + (long long)line * nw;
-  const uint32_t *xw = wordsT + (long long)line * m_pad;
-  uint32_t *ls = list_s + (long long)line * m_pad, *lx = list_x + (long long)line * m_pad;
-  uint32_t *off = list_off + (long long)line * (nw + 1);
-  const uint32_t lt_mask = (1u << lane) - 1u;
-  const int w_begin = seg * UCS_SEG_WORDS;
-  const int w_end = w_begin + UCS_SEG_WORDS < nw ? w_begin + UCS_SEG_WORDS : nw;
-  // entries of this line before the segment
-  uint32_t run = 0;
-  for (int wd = lane; wd < w_begin; wd += 32) {
-    run += (uint32_t)__popc(nz[wd]);
-  }
-  run = __reduce_add_sync(0xffffffffu, run);
-  for (int w0 = w_begin; w0 < w_end; w0 += 32) {
-    const int wd = w0 + lane;
-    const uint32_t bits = wd < w_end ? nz[wd] : 0u;
-    const uint32_t c = (uint32_t)__popc(bits);
-    uint32_t incl = c;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
-      if (lane >= o) {
-        incl += v;
-      }
-    }
-    const uint32_t excl = run + incl - c;
-    if (wd < w_end) {
-      off[wd] = excl;
-    }
-    const int nj = w_end - w0 < 32 ? w_end - w0 : 32;
-    for (int j = 0; j < nj; j++) {
-      const uint32_t bj = __shfl_sync(0xffffffffu, bits, j);
-      if (bj == 0u) {
-        continue;
-      }
-      const uint32_t basej = __shfl_sync(0xffffffffu, excl, j);
-      const int smp = (w0 + j) * 32 + lane;
-      const uint32_t xv = xw[smp];
-      if ((bj >> lane) & 1u) {
-        const uint32_t pos = basej + (uint32_t)__popc(bj & lt_mask);
-        ls[pos] = (uint32_t)smp;
-        lx[pos] = xv ^ 1u; // (x ^ d) & 1 is then the direction bit of an event
-      }
-    }
-    run += __shfl_sync(0xffffffffu, incl, 31);
-  }
-  if (lane == 0 && w_end == nw) {
-    off[nw] = run;
-  }
-}
-
-// The update itself: per walked sample two shuffles (sample, x word), the d word, AND, and - for
-// the lanes with coincidences - one byte (count, direction) pushed into the lane's column of a
-// queue in shared memory. The queues are drained together when one is nearly full, oldest event
-// first: one pulse at a time with the clip after each, as in rpu_weight_updater.cpp:243-291. The
-// Gaussians of the device noise come from a pool per warp in shared memory that all lanes refill
-// together and take from without gaps (ballot + prefix count).
-constexpr int USL_QCAP = 24; // events per lane between two drains
-
-template <int KIND, bool NOISY>
-__global__ void __launch_bounds__(256) pulsedUpdateListKernel(UpdateProblem p, StreamUpdate st) {
-  pdlEnter();
-  __shared__ float pool[8][USP_POOL];
-  // rows padded by one word: lanes at different fill levels then fall into different banks
-  __shared__ uint8_t evq[USL_QCAP][256 + 4];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int n_dblk = (p.d_size + 31) >> 5;
-  const long long task = (long long)blockIdx.x * 8 + warp;
-  if (task >= (long long)n_dblk * p.x_size) {
-    return;
-  }
-  const int j = (int)(task / n_dblk);
-  const int i = (int)(task - (long long)j * n_dblk) * 32 + lane;
-  const bool i_ok = i < p.d_size;
-  const long long idx = (long long)j * p.d_size + (i_ok ? i : 0);
-  float w = 0.0f;
-  float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
-  float2 e = make_float2(0.f, 0.f);
-  if (i_ok) {
-    w = p.w[idx];
-    q = p.par4[idx];
-    if (KIND != AB200_DEVICE_CONSTANT_STEP && KIND != AB200_DEVICE_EXP_STEP &&
-        KIND != AB200_DEVICE_PIECEWISE_STEP) {
-      e = p.par2[idx];
-    }
-  }
-  const float w_in = w;
-  const float std = p.dw_min_std;
-  // chopped transfer compound: direction flipped when exactly one of the two lines is chopped
-  uint32_t chop_flip = 0u;
-  if (p.chop_x != nullptr) {
-    chop_flip = (p.chop_x[j] != 0 ? 1u : 0u) ^ ((i_ok && p.chop_d[i] != 0) ? 1u : 0u);
-  }
-  int cnt = 0;
-  int pool_pos = USP_POOL; // empty
-  uint32_t refills = 0;
-  const uint32_t lt_mask = (1u << lane) - 1u;
-
-  auto drain = [&]() {
-    const int rounds = __reduce_max_sync(0xffffffffu, cnt);
-    for (int r = 0; r < rounds; r++) {
-      int n = 0;
-      bool down = false;
-      if (r < cnt) {
-        const uint32_t ev = evq[r][threadIdx.x];
-        n = (int)(ev >> 1);
-        down = (ev & 1u) != 0u;
-      }
-      for (int k = 0; __any_sync(0xffffffffu, k < n); k++) {
-        const bool act = k < n;
-        float xi = 0.0f;
-        if (NOISY) {
-          const uint32_t takers = __ballot_sync(0xffffffffu, act);
-          if (pool_pos + __popc(takers) > USP_POOL) {
-            // all lanes refill together; what is left of the old pool is dropped
-            float z[8];
-            gauss8(p.key, (uint64_t)(task * 32 + lane) | ((uint64_t)refills << 40), p.call, TAG_DEVICE, z);
-            __syncwarp();
-#pragma unroll
-            for (int rr = 0; rr < 8; rr++) {
-              pool[warp][rr * 32 + lane] = z[rr];
-            }
-            __syncwarp();
-            refills++;
-            pool_pos = 0;
-          }
-          if (act) {
-            xi = std * pool[warp][pool_pos + __popc(takers & lt_mask)];
-          }
-          pool_pos += __popc(takers);
-        }
-        if (act) {
-          w = pulseOnce<KIND>(w, down, q, e, xi, p.mult_noise, p.es0, p.es1, p.pw, p.pw_n);
-        }
-      }
-    }
-    cnt = 0;
-  };
-
-  const int nw = st.m_pad >> 5;
-  const uint32_t *off = st.list_off + (long long)j * (nw + 1);
-  const uint32_t *nz_line = st.xnzT + (long long)j * nw;
-  const uint32_t *ls = st.list_s + (long long)j * st.m_pad;
-  const uint32_t *lx = st.list_x + (long long)j * st.m_pad;
-  // entries of the samples in [s_begin, s_end)
-  auto entriesBefore = [&](int smp) -> uint32_t {
-    const int wd = smp >> 5;
-    if (wd >= nw) {
-      return off[nw];
-    }
-    return off[wd] + (uint32_t)__popc(nz_line[wd] & ((1u << (smp & 31)) - 1u));
-  };
-  const uint32_t k_begin = entriesBefore(p.s_begin), k_end = entriesBefore(p.s_end);
-  for (uint32_t k = k_begin; k < k_end; k += 32) {
-    const uint32_t kk = k + lane;
-    const uint32_t my_s = kk < k_end ? ls[kk] : 0u;
-    const uint32_t my_x = kk < k_end ? lx[kk] : 0u;
-    const int n_in = (int)(k_end - k < 32u ? k_end - k : 32u);
-    for (int t = 0; t < n_in; t += 4) {
-      // four samples at a time, so that their d words are in flight together
-      uint32_t sv[4], xv[4], dwv[4];
-#pragma unroll
-      for (int c = 0; c < 4; c++) {
-        sv[c] = __shfl_sync(0xffffffffu, my_s, (t + c) & 31);
-        xv[c] = __shfl_sync(0xffffffffu, my_x, (t + c) & 31);
-      }
-#pragma unroll
-      for (int c = 0; c < 4; c++) {
-        dwv[c] = (t + c < n_in && i_ok) ? p.dw[(long long)sv[c] * p.d_size + i] : 0u;
-      }
-#pragma unroll
-      for (int c = 0; c < 4; c++) {
-        const uint32_t both = xv[c] & dwv[c] & ~1u;
-        if (both != 0u) {
-          // equal line signs = decrease (rpu_weight_updater.cpp:246-268); the x sign is stored flipped
-          evq[cnt][threadIdx.x] =
-              (uint8_t)(((uint32_t)__popc(both) << 1) | (((xv[c] ^ dwv[c]) & 1u) ^ chop_flip));
-          cnt++;
-        }
-      }
-      if (__any_sync(0xffffffffu, cnt > USL_QCAP - 4)) {
-        drain();
-      }
-    }
-  }
-  drain();
-  if (i_ok && w != w_in) {
-    p.w[idx] = w;
-  }
-}
-
-template <int KIND>
-static void launchStreamKind(const UpdateProblem &p, const StreamUpdate &st, cudaStream_t stream) {
-  const long long tasks = (long long)((p.d_size + 31) / 32) * p.x_size;
-  const unsigned blocks = (unsigned)((tasks + 7) / 8);
-  if (p.dw_min_std > 0.0f) {
-    AB200_CUDA(launchChained(pulsedUpdateListKernel<KIND, true>, dim3(blocks), dim3(256), 0, stream, p, st));
-  } else {
-    AB200_CUDA(launchChained(pulsedUpdateListKernel<KIND, false>, dim3(blocks), dim3(256), 0, stream, p, st));
-  }
-}
-
-// the same problem in rows of pulse words: a sample has nseg of them
-static UpdateProblem inRows(const UpdateProblem &p0) {
-  UpdateProblem p = p0;
-  const int nseg = p0.nseg > 0 ? p0.nseg : 1;
-  p.m = p0.m * nseg;
-  p.s_begin = p0.s_begin * nseg;
-  p.s_end = p0.s_end * nseg;
-  p.nseg = 1;
-  return p;
-}
-
 static int g_update_path = 0;
 void setUpdatePath(int mode) { g_update_path = mode; }
 
@@ -957,59 +456,6 @@ bool streamUpdateEligible(const UpdateProblem &p) {
     return false;
   }
   return g_update_path == 2 || p.m * (p.nseg > 0 ? p.nseg : 1) >= kStreamUpdateMinBatch;
-}
-
-void launchPulseTranspose(const UpdateProblem &p0, uint32_t *xwT, uint32_t *xnzT, int m_pad,
-                          cudaStream_t stream) {
-  const UpdateProblem p = inRows(p0);
-  dim3 grid((p.x_size + 31) / 32, m_pad / 32), block(32, 8);
-  AB200_CUDA(launchChained(pulseTransposeKernel, grid, block, 0, stream, p.xw, p.x_size, p.m, m_pad, xwT,
-                           xnzT));
-  AB200_LAUNCH_CHECK();
-}
-
-void launchPulseCompact(const UpdateProblem &p0, const uint32_t *xwT, const uint32_t *xnzT, int m_pad,
-                        uint32_t *list_s, uint32_t *list_x, uint32_t *list_off, cudaStream_t stream) {
-  const UpdateProblem p = inRows(p0);
-  const int n_seg = (m_pad / 32 + UCS_SEG_WORDS - 1) / UCS_SEG_WORDS;
-  const unsigned blocks = (unsigned)(((long long)p.x_size * n_seg * 32 + 255) / 256);
-  AB200_CUDA(launchChained(pulseCompactKernel, dim3(blocks), dim3(256), 0, stream, xwT, xnzT, p.x_size, m_pad,
-                           list_s, list_x, list_off));
-  AB200_LAUNCH_CHECK();
-}
-
-void launchPulsedUpdateStream(const UpdateProblem &p0, const uint32_t *xwT, const uint32_t *xnzT,
-                              int m_pad, cudaStream_t stream, const uint32_t *list_s,
-                              const uint32_t *list_x, const uint32_t *list_off) {
-  const UpdateProblem p = inRows(p0);
-  if (p.s_end <= p.s_begin) {
-    return;
-  }
-  StreamUpdate st{xwT, xnzT, m_pad, list_s, list_x, list_off};
-  switch (p.kind) {
-  case AB200_DEVICE_CONSTANT_STEP:
-    launchStreamKind<AB200_DEVICE_CONSTANT_STEP>(p, st, stream);
-    break;
-  case AB200_DEVICE_LINEAR_STEP:
-  case AB200_DEVICE_SOFT_BOUNDS:
-    launchStreamKind<AB200_DEVICE_LINEAR_STEP>(p, st, stream);
-    break;
-  case AB200_DEVICE_SOFT_BOUNDS_REFERENCE:
-    launchStreamKind<AB200_DEVICE_SOFT_BOUNDS_REFERENCE>(p, st, stream);
-    break;
-  case AB200_DEVICE_POW_STEP:
-    launchStreamKind<AB200_DEVICE_POW_STEP>(p, st, stream);
-    break;
-  case AB200_DEVICE_EXP_STEP:
-    launchStreamKind<AB200_DEVICE_EXP_STEP>(p, st, stream);
-    break;
-  case AB200_DEVICE_PIECEWISE_STEP:
-    launchStreamKind<AB200_DEVICE_PIECEWISE_STEP>(p, st, stream);
-    break;
-  default:
-    AB200_FATAL("pulsed update: device kind not implemented");
-  }
-  AB200_LAUNCH_CHECK();
 }
 
 void launchPulsePrepare(const UpdateProblem &p, cudaStream_t stream) {

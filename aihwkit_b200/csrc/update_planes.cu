@@ -1,0 +1,614 @@
+// Pulsed update with stochastic trains, on bit planes.
+//
+//   pulseStatsKernel / pulseStatsGatherKernel
+//                      per sample |x|max, |d|max -> train length BL and the probabilities' factors
+//                      A, B (update management).
+//   pulsePlanesKernel  the trains of 32 rows of every line as bit planes: plane 0 holds the signs of the 32
+//                      rows, plane k their pulses in slot k. A row is a sample, or a segment of at most
+//                      31 slots of it. Four planes of a line lie side by side, [block][plane / 4][line][4], so
+//                      that one 16-byte load brings trains of up to three slots.
+//   pulsedUpdatePlanesKernel
+//                      a warp owns 32 d-lines of ONE x-line; AND of the two lines' planes gives the
+//                      coincidences of 32 rows at a time.
+//
+// Update management shortens the trains to what a sample needs (BL = ceil(lr |x|max |d|max / dw_min)), one
+// or two slots in ordinary training, so 32 rows take one or two ANDs where words per row took 32 ANDs,
+// 32 population counts and 32 loads. Only planes up to the longest train of a block are written and read.
+// Before, the words of a line were transposed and compacted to lists of (sample, word), two launches more.
+// Measured, update of a 256 x 2304 SoftBounds tile with 131072 rows: 27.4 -> 19.1 ms; 1024 x 1024 Tiki-Taka step
+// with 256 rows 407 -> 257 us.
+#include "pulse_common.cuh"
+
+namespace ab200 {
+
+// ---------------------------------------------------------------------------------------------
+// update management per sample
+// ---------------------------------------------------------------------------------------------
+__device__ __forceinline__ void storeSampleParams(const UpdateProblem &p, int s, float xm, float dm) {
+  if (s == 0) {
+    *p.plane_max = 0; // the planes' kernel raises it
+  }
+  int BL;
+  float A, B;
+  blAB(p.up, p.lr, p.dw_min, xm, dm, BL, A, B);
+  p.plane_bl[s] = BL;
+  p.plane_ab[s] = make_float2(A, B);
+}
+
+// plain rows (any strides) and rows gathered through a row-major index array: one CTA per sample
+__global__ void __launch_bounds__(128) pulseStatsKernel(UpdateProblem p) {
+  pdlEnter();
+  __shared__ float sh[4];
+  const int s = blockIdx.x;
+  float xm = 0.0f, dm = 0.0f;
+  if (p.up.update_management || p.up.update_bl_management) {
+    if (p.gather.idx != nullptr) {
+      for (int j = threadIdx.x; j < p.x_size; j += 128) {
+        xm = fmaxf(xm, fabsf(gatherRowElement(p.gather, p.x, s, j)));
+      }
+    } else {
+      const float *xr = p.x + (long long)s * p.x_ss;
+#pragma unroll 8
+      for (int j = threadIdx.x; j < p.x_real; j += 128) {
+        xm = fmaxf(xm, fabsf(xr[(long long)j * p.x_fs]));
+      }
+      if (p.x_real < p.x_size) {
+        xm = fmaxf(xm, 1.0f); // the bias line
+      }
+    }
+    const float *dr = p.d + (long long)s * p.d_ss;
+#pragma unroll 8
+    for (int i = threadIdx.x; i < p.d_size; i += 128) {
+      dm = fmaxf(dm, fabsf(dr[(long long)i * p.d_fs]));
+    }
+    xm = blockMax(xm, sh);
+    dm = blockMax(dm, sh);
+  }
+  if (threadIdx.x == 0) {
+    storeSampleParams(p, s, xm, dm);
+  }
+}
+
+// Images gathered through an index array [x_size][m_batch]: lanes are 32 neighbouring positions, whose
+// indices are contiguous and whose pixels nearly are, and the warps of the CTA share the x-lines.
+__global__ void __launch_bounds__(1024) pulseStatsGatherKernel(UpdateProblem p) {
+  pdlEnter();
+  __shared__ float shx[32][33], shd[32];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int s = blockIdx.x * 32 + lane;
+  float xm = 0.0f;
+  if (s < p.m) {
+    const int n = s / p.gather.m_batch, l = s - n * p.gather.m_batch;
+    const float *img = p.x + (long long)n * p.gather.image_size - 2;
+    const int32_t *col = p.gather.idx_t + l;
+#pragma unroll 6
+    for (int k = warp; k < p.x_size; k += 32) {
+      const int e = __ldg(col + (long long)k * p.gather.m_batch);
+      xm = fmaxf(xm, e <= 1 ? (float)e : fabsf(__ldg(img + e)));
+    }
+  }
+  shx[warp][lane] = xm;
+  const int sd = blockIdx.x * 32 + warp;
+  float dm = 0.0f;
+  if (sd < p.m) {
+    const float *dr = p.d + (long long)sd * p.d_ss;
+#pragma unroll 8
+    for (int i = lane; i < p.d_size; i += 32) {
+      dm = fmaxf(dm, fabsf(dr[(long long)i * p.d_fs]));
+    }
+  }
+  for (int o = 16; o > 0; o >>= 1) {
+    dm = fmaxf(dm, __shfl_xor_sync(0xffffffffu, dm, o));
+  }
+  if (lane == 0) {
+    shd[warp] = dm;
+  }
+  __syncthreads();
+  if (warp == 0 && s < p.m) {
+    xm = 0.0f;
+#pragma unroll 8
+    for (int w = 0; w < 32; w++) {
+      xm = fmaxf(xm, shx[w][lane]);
+    }
+    storeSampleParams(p, s, xm, shd[lane]);
+  }
+}
+
+// ---------------------------------------------------------------------------------------------
+// trains of 32 rows as planes
+// ---------------------------------------------------------------------------------------------
+constexpr int PP_LINES = 64; // lines per CTA, eight per warp
+
+// Lane = row: a ballot then yields one plane word of one line. The values are staged through shared
+// memory where the rows are contiguous along the lines, and read directly where they are contiguous
+// along the rows (transposed inputs, index arrays [x_size][m_batch]).
+__global__ void __launch_bounds__(256) pulsePlanesKernel(UpdateProblem p, int n_xchunk) {
+  pdlEnter();
+  __shared__ float tile[PP_LINES][33];
+  __shared__ uint32_t planes[32][PP_LINES + 1];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int nseg = p.nseg > 0 ? p.nseg : 1;
+  const int n_chunk = n_xchunk + (p.d_size + PP_LINES - 1) / PP_LINES;
+  const int blk = blockIdx.x / n_chunk, chunk = blockIdx.x - blk * n_chunk;
+  const bool is_x = chunk < n_xchunk;
+  const int line0 = (is_x ? chunk : chunk - n_xchunk) * PP_LINES;
+  const int n_lines = is_x ? p.x_size : p.d_size;
+  const int real = is_x ? p.x_real : p.d_size;
+  const float *src = is_x ? p.x : p.d;
+  const long long ss = is_x ? p.x_ss : p.d_ss, fs = is_x ? p.x_fs : p.d_fs;
+  const bool gathered = is_x && p.gather.idx != nullptr;
+  const bool gather_t = gathered && p.gather.idx_t != nullptr;
+  const bool direct = gather_t || (!gathered && ss == 1 && fs != 1);
+
+  const int row = blk * 32 + lane;
+  const int s = nseg == 1 ? row : row / nseg;
+  const int seg = nseg == 1 ? 0 : row - s * nseg;
+  const bool row_ok = s < p.m;
+  const int BL = row_ok ? p.plane_bl[s] : 0;
+  float P = 0.0f;
+  if (row_ok) {
+    const float2 ab = p.plane_ab[s];
+    P = is_x ? ab.y : ab.x;
+  }
+  const int nk = max(min(BL - seg * kPulseSegSlots, kPulseSegSlots), 0);
+  const int nk_max = __reduce_max_sync(0xffffffffu, nk);
+  if (chunk == 0 && threadIdx.x == 0) {
+    p.plane_nk[blk] = nk_max;
+    if (nk_max > 3) {
+      atomicMax(p.plane_max, nk_max);
+    }
+  }
+
+  if (!direct) {
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      const int rr = warp * 4 + q;
+      const int rs = (blk * 32 + rr) / nseg;
+#pragma unroll
+      for (int h = 0; h < PP_LINES; h += 32) {
+        const int line = line0 + h + lane;
+        float v = 0.0f;
+        if (rs < p.m && line < n_lines) {
+          if (gathered) {
+            v = gatherRowElement(p.gather, p.x, rs, line);
+          } else {
+            v = line < real ? src[(long long)rs * ss + (long long)line * fs] : 1.0f;
+          }
+        }
+        tile[h + lane][rr] = v;
+      }
+    }
+    __syncthreads();
+  }
+  int img_n = 0, img_l = 0;
+  if (gather_t && row_ok) {
+    img_n = s / p.gather.m_batch;
+    img_l = s - img_n * p.gather.m_batch;
+  }
+  float v[PP_LINES / 8];
+#pragma unroll
+  for (int q = 0; q < PP_LINES / 8; q++) {
+    const int ll = warp * (PP_LINES / 8) + q, line = line0 + ll;
+    v[q] = 0.0f;
+    if (!direct) {
+      v[q] = tile[ll][lane];
+    } else if (row_ok && line < n_lines) {
+      if (gather_t) {
+        const int e = __ldg(p.gather.idx_t + (long long)line * p.gather.m_batch + img_l);
+        v[q] = e <= 1 ? (float)e : __ldg(p.x + (long long)img_n * p.gather.image_size + (e - 2));
+      } else {
+        v[q] = line < real ? src[s + (long long)line * fs] : 1.0f;
+      }
+    }
+  }
+  const uint32_t tag = is_x ? TAG_PULSE_X : TAG_PULSE_D;
+  const uint32_t flip = (!is_x && p.lr_neg) ? 1u : 0u;
+  const bool plain = !(p.up.res > 0.0f);
+#pragma unroll
+  for (int q = 0; q < PP_LINES / 8; q++) {
+    const int ll = warp * (PP_LINES / 8) + q;
+    const uint32_t line = (uint32_t)(line0 + ll);
+    // the train of pulseTrain (pulse_common.cuh), slot by slot across the 32 rows
+    float pp = __fmul_rn(fabsf(v[q]), P);
+    if (!plain) {
+      pp = pulseProb(p, pp, p.up.res, line, (uint32_t)s, tag);
+    }
+    const int thr = pulseThreshold(pp);
+    const uint32_t signs = __ballot_sync(0xffffffffu, ((v[q] > 0.0f ? 0u : 1u) ^ flip) != 0u);
+    uint32_t mine = lane == 0 ? signs : 0u;
+    for (int k0 = 0; k0 < nk_max; k0 += 8) {
+      uint32_t r[4];
+      philox4x32<7>(line, (uint32_t)s, p.call, tag + (uint32_t)(seg * 4 + (k0 >> 3)), p.key, r);
+#pragma unroll
+      for (int h = 0; h < 4; h++) {
+        if (k0 + 2 * h < nk_max) {
+          const uint32_t lo =
+              __ballot_sync(0xffffffffu, k0 + 2 * h < nk && (int)(r[h] & 0xffffu) < thr);
+          const uint32_t hi =
+              __ballot_sync(0xffffffffu, k0 + 2 * h + 1 < nk && (int)(r[h] >> 16) < thr);
+          mine = lane == k0 + 2 * h + 1 ? lo : mine;
+          mine = lane == k0 + 2 * h + 2 ? hi : mine;
+        }
+      }
+    }
+    planes[lane][ll] = mine;
+  }
+  __syncthreads();
+  uint4 *dst = reinterpret_cast<uint4 *>(is_x ? p.xw : p.dw) + (long long)blk * 8 * n_lines + line0;
+  for (int t = threadIdx.x; t < (nk_max / 4 + 1) * PP_LINES; t += 256) {
+    const int g = t / PP_LINES, l = t % PP_LINES;
+    if (line0 + l < n_lines) {
+      dst[(long long)g * n_lines + l] =
+          make_uint4(planes[4 * g][l], planes[4 * g + 1][l], planes[4 * g + 2][l], planes[4 * g + 3][l]);
+    }
+  }
+}
+
+// ---------------------------------------------------------------------------------------------
+// the update
+// ---------------------------------------------------------------------------------------------
+constexpr int UP_WARPS = 4;   // x-lines per CTA (neighbours share the sectors of the x planes)
+constexpr int UP_POOL = 256;  // Gaussians per warp pool (eight per lane and refill)
+constexpr int UP_DRAIN = 20;  // a lane with more events than this has the warp apply all events
+constexpr int UP_EVENTS = 24; // most events of a lane between two drains
+
+struct UpdatePlanesSmem {
+  float pool[UP_WARPS][UP_POOL]; // (lanes without an event read up to 31 values past the end)
+  uint8_t counts[UP_WARPS][UP_EVENTS][32]; // pulses of the events that have more than one
+};
+
+// What a pulse needs of its element, by direction, with the sign of the direction in it: w += signed
+// step instead of w -= step (round-to-nearest is symmetric, so the bits are those of pulseOnce).
+template <int KIND> struct PulseStep {
+  float4 q;
+  float2 e;
+  float scale_dn, slope_dn;
+  __device__ __forceinline__ void set(const float4 &q_, const float2 &e_) {
+    q = q_;
+    e = e_;
+    scale_dn = -q.y;
+    slope_dn = -e.y;
+  }
+  // the noise of a pulse enters the rule as 1 + xi; kept in that form from the draw on
+  static constexpr bool kOnePlus =
+      KIND == AB200_DEVICE_CONSTANT_STEP || KIND == AB200_DEVICE_LINEAR_STEP;
+  __device__ __forceinline__ float apply(const UpdateProblem &p, float w, bool down, float xi) const {
+    if (KIND == AB200_DEVICE_CONSTANT_STEP) {
+      w = __fadd_rn(w, __fmul_rn(xi, down ? scale_dn : q.x));
+      return fmaxf(fminf(w, q.z), q.w);
+    } else if (KIND == AB200_DEVICE_LINEAR_STEP) {
+      const float sc = down ? scale_dn : q.x, sl = __fmul_rn(down ? slope_dn : e.x, w);
+      const float dw = p.mult_noise ? __fmul_rn(__fadd_rn(sl, sc), xi) : __fadd_rn(sl, __fmul_rn(sc, xi));
+      return fminf(fmaxf(__fadd_rn(w, dw), q.w), q.z);
+    } else {
+      return pulseOnce<KIND>(w, down, q, e, xi, p.mult_noise, p.es0, p.es1, p.pw, p.pw_n);
+    }
+  }
+};
+
+// Eight fresh Gaussians per lane for a warp's pool, as offset + std * z. Out of line: rare against the pulses
+// that take from the pool at two places, and the largest piece of code among them.
+__device__ __noinline__ void refillPool(PhiloxKey key, uint64_t pair, uint32_t call, float std, float offset,
+                                        float *column) {
+  float z[8];
+  gauss8(key, pair, call, TAG_DEVICE, z);
+#pragma unroll
+  for (int rr = 0; rr < 8; rr++) {
+    column[rr * 32] = __fadd_rn(offset, __fmul_rn(std, z[rr]));
+  }
+}
+
+// Per block of 32 rows a lane gets one word of coincidences and appends their directions to a queue of
+// bits in a register. The pulses are applied in rounds, one event per
+// lane and round, oldest first, one pulse at a time with the clip after each as in
+// rpu_weight_updater.cpp:243-291; Gaussians of the device noise come from a pool per warp that all lanes
+// refill together and take from without gaps (ballot + prefix count). Rounds start when, after a group of
+// four rows in which the x-line pulsed, a lane holds more than UP_DRAIN events: that point fixes
+// which Gaussian an event gets, so it is found exactly, also inside a word.
+//
+// Bound by instructions (0.75 of the issue slots used): about 60 per block of 32 rows, 45 per round, and 150 per
+// refill; the busiest lane sets the number of rounds, 0.66 of the lanes have an event in one. A list of
+// {coincidences, directions} words in shared memory instead of the queue of bits took 7 % fewer instructions
+// and the same time (24 instead of 32 warps per SM).
+template <int KIND, bool NOISY>
+__global__ void __launch_bounds__(32 * UP_WARPS, 8) pulsedUpdatePlanesKernel(UpdateProblem p) {
+  pdlEnter();
+  __shared__ UpdatePlanesSmem sm;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int n_dblk = (p.d_size + 31) >> 5;
+  const int jg = (int)(blockIdx.x / (unsigned)n_dblk), dblk = (int)(blockIdx.x - (unsigned)jg * n_dblk);
+  const int j = jg * UP_WARPS + warp;
+  if (j >= p.x_size) {
+    return;
+  }
+  const long long task = (long long)j * n_dblk + dblk;
+  const int i = dblk * 32 + lane;
+  const bool i_ok = i < p.d_size;
+  const long long idx = (long long)j * p.d_size + (i_ok ? i : 0);
+  float w = 0.0f;
+  PulseStep<KIND> step;
+  {
+    float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
+    float2 e = make_float2(0.f, 0.f);
+    if (i_ok) {
+      w = p.w[idx];
+      q = p.par4[idx];
+      if (KIND != AB200_DEVICE_CONSTANT_STEP && KIND != AB200_DEVICE_EXP_STEP &&
+          KIND != AB200_DEVICE_PIECEWISE_STEP) {
+        e = p.par2[idx];
+      }
+    }
+    step.set(q, e);
+  }
+  const float w_in = w;
+  const float std = p.dw_min_std;
+  // chopped transfer compound: direction flipped when exactly one of the two lines is chopped
+  uint32_t flip = 0xffffffffu; // equal line signs = decrease (rpu_weight_updater.cpp:246-268)
+  if (p.chop_x != nullptr && (p.chop_x[j] != 0) != (i_ok && p.chop_d[i] != 0)) {
+    flip = 0u;
+  }
+  float *const pool = sm.pool[warp];
+  uint8_t *const counts = &sm.counts[warp][0][lane];
+  int cnt = 0;        // events in the queue
+  uint32_t queue = 0; // their directions, the newest in bit 0
+  uint32_t multi = 0; // events (by ordinal) of more than one pulse
+  int pool_pos = UP_POOL; // empty
+  uint32_t refills = 0;
+  const uint32_t lt_mask = (1u << lane) - 1u;
+
+  // one pulse for the lanes in `act`
+  auto pulse = [&](bool act, bool down) {
+    float xi = PulseStep<KIND>::kOnePlus ? 1.0f : 0.0f;
+    if (NOISY) {
+      const uint32_t takers = __ballot_sync(0xffffffffu, act);
+      const int n_take = __popc(takers);
+      if (pool_pos + n_take > UP_POOL) {
+        // all lanes refill together; what is left of the old pool is dropped
+        __syncwarp();
+        refillPool(p.key, (uint64_t)(task * 32 + lane) | ((uint64_t)refills << 40), p.call, std,
+                   PulseStep<KIND>::kOnePlus ? 1.0f : 0.0f, pool + lane);
+        __syncwarp();
+        refills++;
+        pool_pos = 0;
+      }
+      xi = pool[pool_pos + __popc(takers & lt_mask)];
+      pool_pos += n_take;
+    }
+    const float w_new = step.apply(p, w, down, xi);
+    w = act ? w_new : w;
+  };
+
+  auto drain = [&]() {
+    const int rounds = __reduce_max_sync(0xffffffffu, cnt);
+    uint32_t multi_any = __reduce_or_sync(0xffffffffu, multi);
+    queue = __funnelshift_lc(0u, queue, 32 - cnt); // the oldest first
+    for (int r = 0; r < rounds; r++) {
+      const bool down = (int)queue < 0;
+      queue <<= 1;
+      pulse(r < cnt, down);
+      if ((multi_any & 1u) != 0u) {
+        const int n = ((multi >> r) & 1u) != 0u ? counts[r * 32] : 0;
+        for (int k = 1; __any_sync(0xffffffffu, k < n); k++) {
+          pulse(k < n, down);
+        }
+      }
+      multi_any >>= 1;
+    }
+    cnt = 0;
+    queue = 0u;
+    multi = 0u;
+  };
+
+  const int b_first = p.s_begin >> 5, b_last = (p.s_end - 1) >> 5;
+  const uint4 *xb = reinterpret_cast<const uint4 *>(p.xw) + (long long)b_first * 8 * p.x_size + j;
+  const uint4 *db = reinterpret_cast<const uint4 *>(p.dw) + (long long)b_first * 8 * p.d_size + (i_ok ? i : 0);
+  const long long x_step = 8LL * p.x_size, d_step = 8LL * p.d_size;
+  const bool deep = *p.plane_max > 3; // some train has more slots than the first four planes hold
+  // rows of the first / last block outside of [s_begin, s_end)
+  const uint32_t rows_first = 0xffffffffu << (p.s_begin & 31);
+  const uint32_t rows_last = 0xffffffffu >> (31 - ((p.s_end - 1) & 31));
+  const uint32_t lane_on = i_ok ? 0xffffffffu : 0u;
+  uint32_t rank0 = 0; // pulsing rows of the x-line before this block, from s_begin on
+  uint32_t group = 0; // group in which a lane has passed the mark
+
+  auto push = [&](uint32_t ev, uint32_t dir) {
+    while (ev != 0u) {
+      const uint32_t rest = ev & (ev - 1u);
+      queue = queue * 2u + ((dir & (ev ^ rest)) != 0u ? 1u : 0u);
+      ev = rest;
+    }
+  };
+  auto pushCounts = [&](uint32_t more, uint32_t ev, int before, uint32_t c0, uint32_t c1, uint32_t c2,
+                        uint32_t c3, uint32_t c4) {
+    while (more != 0u) {
+      const uint32_t bit = more & (0u - more);
+      more ^= bit;
+      const int at = before + __popc(ev & (bit - 1u));
+      counts[at * 32] = (uint8_t)(((c0 & bit) ? 1 : 0) + ((c1 & bit) ? 2 : 0) + ((c2 & bit) ? 4 : 0) +
+                                  ((c3 & bit) ? 8 : 0) + ((c4 & bit) ? 16 : 0));
+      multi |= 1u << at;
+    }
+  };
+
+  int b = b_first;
+  while (true) {
+    // Two inner blocks at a time as long as no lane fills up in them and no train is longer than three slots.
+    while (!deep && b > b_first && b + 1 < b_last) {
+      const uint4 x0 = xb[0], x1 = xb[x_step], d0 = db[0], d1 = db[d_step];
+      const uint32_t p0 = x0.y & d0.y, p1 = x0.z & d0.z, p2 = x0.w & d0.w;
+      const uint32_t q0 = x1.y & d1.y, q1 = x1.z & d1.z, q2 = x1.w & d1.w;
+      const uint32_t any0 = (p0 | p1 | p2) & lane_on, any1 = (q0 | q1 | q2) & lane_on;
+      const int n0 = __popc(any0), n1 = __popc(any1);
+      if (__any_sync(0xffffffffu, cnt + n0 + n1 > UP_DRAIN)) {
+        break;
+      }
+      push(any0, x0.x ^ d0.x ^ flip);
+      push(any1, x1.x ^ d1.x ^ flip);
+      const uint32_t m0 = (p0 & p1) | (p0 & p2) | (p1 & p2), m1 = (q0 & q1) | (q0 & q2) | (q1 & q2);
+      if (((m0 | m1) & lane_on) != 0u) {
+        pushCounts(m0 & lane_on, any0, cnt, p0 ^ p1 ^ p2, m0, 0u, 0u, 0u);
+        pushCounts(m1 & lane_on, any1, cnt + n0, q0 ^ q1 ^ q2, m1, 0u, 0u, 0u);
+      }
+      cnt += n0 + n1;
+      rank0 += (uint32_t)(__popc(x0.y | x0.z | x0.w) + __popc(x1.y | x1.z | x1.w));
+      b += 2;
+      xb += 2 * x_step;
+      db += 2 * d_step;
+    }
+    // One block; after the last one a turn that applies what is left.
+    const bool end = b > b_last;
+    uint32_t any = 0, dir = 0, xnz = 0, c0 = 0, c1 = 0, c2 = 0, c3 = 0, c4 = 0;
+    if (!end) {
+      const uint4 xv = *xb, dv = *db;
+      // coincidences and, in c0..c4, the bits of their pulse counts
+      dir = xv.x ^ dv.x ^ flip;
+      xnz = xv.y | xv.z | xv.w;
+      const uint32_t a1 = xv.y & dv.y, a2 = xv.z & dv.z, a3 = xv.w & dv.w;
+      any = a1 | a2 | a3;
+      c0 = a1 ^ a2 ^ a3;
+      c1 = (a1 & a2) | (a1 & a3) | (a2 & a3);
+      if (deep) {
+        const int nk = p.plane_nk[b];
+        const uint4 *xg = xb, *dg = db;
+        for (int k = 4; k <= nk; k += 4) {
+          xg += p.x_size;
+          dg += p.d_size;
+          const uint4 xk = *xg, dk = *dg;
+          const uint32_t a[4] = {xk.x & dk.x, xk.y & dk.y, xk.z & dk.z, xk.w & dk.w};
+          xnz |= xk.x | xk.y | xk.z | xk.w;
+#pragma unroll
+          for (int u = 0; u < 4; u++) {
+            any |= a[u];
+            const uint32_t t0 = c0 & a[u];
+            c0 ^= a[u];
+            const uint32_t t1 = c1 & t0;
+            c1 ^= t0;
+            const uint32_t t2 = c2 & t1;
+            c2 ^= t1;
+            const uint32_t t3 = c3 & t2;
+            c3 ^= t2;
+            c4 ^= t3;
+          }
+        }
+      }
+      xnz &= b == b_first ? rows_first : 0xffffffffu;
+      xnz &= b == b_last ? rows_last : 0xffffffffu;
+      any &= xnz & lane_on;
+    }
+    const uint32_t rank_end = rank0 + (uint32_t)__popc(xnz);
+    while (true) {
+      // events of this word that belong to the list being filled
+      uint32_t ev = any;
+      const int total = cnt + __popc(any);
+      bool full = __any_sync(0xffffffffu, total > UP_DRAIN);
+      if (full && !end) {
+        // the group of four pulsing rows in which the first lane passes the mark
+        uint32_t g = 0xffffffffu;
+        if (total > UP_DRAIN) {
+          if (cnt > UP_DRAIN) {
+            g = group; // passed it in an earlier word, in a group that goes on in this one
+          } else {
+            uint32_t t = any;
+            for (int k = cnt; k < UP_DRAIN; k++) {
+              t &= t - 1u;
+            }
+            const uint32_t at = t & (0u - t);
+            g = (rank0 + (uint32_t)__popc(xnz & (at - 1u))) >> 2;
+          }
+        }
+        group = __reduce_min_sync(0xffffffffu, g);
+        full = rank_end >= 4u * group + 4u; // else the group ends in a later word
+        if (full) {
+          // rows of this word up to the end of the group
+          ev &= __ballot_sync(0xffffffffu, rank0 + (uint32_t)__popc(xnz & lt_mask) < 4u * group + 4u);
+        }
+      }
+      if (ev != 0u) {
+        push(ev, dir);
+        pushCounts(ev & (c1 | c2 | c3 | c4), ev, cnt, c0, c1, c2, c3, c4);
+        cnt += __popc(ev);
+      }
+      if (!full && !end) {
+        break;
+      }
+      drain();
+      any ^= ev;
+      if (end) {
+        break;
+      }
+    }
+    if (end) {
+      break;
+    }
+    rank0 = rank_end;
+    b++;
+    xb += x_step;
+    db += d_step;
+  }
+  if (i_ok && w != w_in) {
+    p.w[idx] = w;
+  }
+}
+
+template <int KIND, bool NOISY>
+static void launchPlanesInstance(const UpdateProblem &p, cudaStream_t stream) {
+  const long long blocks =
+      (long long)((p.d_size + 31) / 32) * ((p.x_size + UP_WARPS - 1) / UP_WARPS);
+  AB200_CUDA(launchChained(pulsedUpdatePlanesKernel<KIND, NOISY>, dim3((unsigned)blocks), dim3(32 * UP_WARPS),
+                           0, stream, p));
+}
+
+template <int KIND> static void launchPlanesKind(const UpdateProblem &p, cudaStream_t stream) {
+  if (p.dw_min_std > 0.0f) {
+    launchPlanesInstance<KIND, true>(p, stream);
+  } else {
+    launchPlanesInstance<KIND, false>(p, stream);
+  }
+}
+
+void launchPulsePlanes(const UpdateProblem &p, cudaStream_t stream) {
+  if (p.gather.idx != nullptr && p.gather.idx_t != nullptr) {
+    AB200_CUDA(launchChained(pulseStatsGatherKernel, dim3((p.m + 31) / 32), dim3(1024), 0, stream, p));
+  } else {
+    AB200_CUDA(launchChained(pulseStatsKernel, dim3(p.m), dim3(128), 0, stream, p));
+  }
+  AB200_LAUNCH_CHECK();
+  const int n_blk = (p.m * (p.nseg > 0 ? p.nseg : 1) + 31) / 32;
+  const int n_x = (p.x_size + PP_LINES - 1) / PP_LINES, n_d = (p.d_size + PP_LINES - 1) / PP_LINES;
+  AB200_CUDA(launchChained(pulsePlanesKernel, dim3((unsigned)((long long)n_blk * (n_x + n_d))), dim3(256), 0,
+                           stream, p, n_x));
+  AB200_LAUNCH_CHECK();
+}
+
+void launchPulsedUpdatePlanes(const UpdateProblem &p0, cudaStream_t stream) {
+  const UpdateProblem p = inRows(p0);
+  if (p.s_end <= p.s_begin) {
+    return;
+  }
+  switch (p.kind) {
+  case AB200_DEVICE_CONSTANT_STEP:
+    launchPlanesKind<AB200_DEVICE_CONSTANT_STEP>(p, stream);
+    break;
+  case AB200_DEVICE_LINEAR_STEP:
+  case AB200_DEVICE_SOFT_BOUNDS:
+    launchPlanesKind<AB200_DEVICE_LINEAR_STEP>(p, stream);
+    break;
+  case AB200_DEVICE_SOFT_BOUNDS_REFERENCE:
+    launchPlanesKind<AB200_DEVICE_SOFT_BOUNDS_REFERENCE>(p, stream);
+    break;
+  case AB200_DEVICE_POW_STEP:
+    launchPlanesKind<AB200_DEVICE_POW_STEP>(p, stream);
+    break;
+  case AB200_DEVICE_EXP_STEP:
+    launchPlanesKind<AB200_DEVICE_EXP_STEP>(p, stream);
+    break;
+  case AB200_DEVICE_PIECEWISE_STEP:
+    launchPlanesKind<AB200_DEVICE_PIECEWISE_STEP>(p, stream);
+    break;
+  default:
+    AB200_FATAL("pulsed update: device kind not implemented");
+  }
+  AB200_LAUNCH_CHECK();
+}
+
+} // namespace ab200

@@ -1,0 +1,150 @@
+"""The bit-plane update kernel against an event-by-event restatement, device noise on: trains, order of
+the pulses and the Gaussian every pulse gets (pools of 256 per 32 weights, taken in rounds that start
+once a weight holds more than 20 events after a group of four rows in which its input line pulsed)."""
+
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+TAG_X, TAG_D, TAG_DEVICE = 0x30000000, 0x40000000, 0x50000000
+
+
+def _philox7(c, key):
+    """Philox4x32 with seven rounds; ``c``: four uint32 arrays."""
+    c = [np.asarray(v, np.uint64) & 0xFFFFFFFF for v in np.broadcast_arrays(*c)]
+    k0, k1 = key
+    for _ in range(7):
+        p0, p1 = c[0] * np.uint64(0xD2511F53), c[2] * np.uint64(0xCD9E8D57)
+        c = [(p1 >> np.uint64(32)) ^ c[1] ^ np.uint64(k0), p1 & np.uint64(0xFFFFFFFF),
+             (p0 >> np.uint64(32)) ^ c[3] ^ np.uint64(k1), p0 & np.uint64(0xFFFFFFFF)]
+        k0, k1 = (k0 + 0x9E3779B9) & 0xFFFFFFFF, (k1 + 0xBB67AE85) & 0xFFFFFFFF
+    return c
+
+
+def _trains(v, strength, bl, key, tag):
+    """Pulses ``[sample, line, slot]`` of a batch ``[sample, line]``."""
+    m, n = v.shape
+    p = (np.abs(v) * np.float32(strength)).astype(np.float32)
+    thr = np.ceil((p * np.float32(65536) - np.float32(0.5)).astype(np.float32))
+    out = np.zeros((m, n, bl), bool)
+    line, smp = np.arange(n)[None, :], np.arange(m)[:, None]
+    for k in range(bl):
+        seg, slot = divmod(k, 31)
+        r = _philox7((line, smp, 0, tag + seg * 4 + slot // 8), key)[(slot % 8) >> 1]
+        out[:, :, k] = ((r >> np.uint64(16 * (slot & 1))) & np.uint64(0xFFFF)).astype(np.float64) < thr
+    return out
+
+
+def _pool(task, refill, key):
+    pair = (task * 32 + np.arange(32)).astype(np.uint64) | np.uint64(refill << 40)
+    r = _philox7((pair & np.uint64(0xFFFFFFFF), pair >> np.uint64(32), 0, TAG_DEVICE), key)
+    z = np.zeros((8, 32))
+    for h in range(4):
+        u1 = 1.0 - (r[h] >> np.uint64(16)).astype(np.float64) / 65536.0
+        ang = 2 * np.pi * (r[h] & np.uint64(0xFFFF)).astype(np.float64) / 65536.0
+        rad = np.sqrt(-2.0 * np.log(u1))
+        z[2 * h], z[2 * h + 1] = rad * np.cos(ang), rad * np.sin(ang)
+    return z.reshape(-1).astype(np.float32)
+
+
+def _apply_task(w, hi, lo, up, down, counts, dirs, rows, std, task, key):
+    """One x-line and up to 32 d-lines: ``counts`` / ``dirs`` ``[row, lane]``, ``rows`` those in which the
+    x-line pulsed.  Returns the number of pulses of the busiest weight."""
+    one, n_lanes = np.float32(1), w.size
+    state = {"pool": None, "pos": 256, "refills": 0}
+
+    def take(n):
+        if state["pos"] + n > 256:
+            state["pool"] = _pool(task, state["refills"], key)
+            state["refills"] += 1
+            state["pos"] = 0
+        state["pos"] += n
+        return state["pool"][state["pos"] - n : state["pos"]]
+
+    def drain(q):
+        for r in range(max(len(e) for e in q)):
+            n = [e[r][0] if r < len(e) else 0 for e in q]
+            for k in range(max(n)):
+                lanes = [l for l in range(n_lanes) if k < n[l]]
+                for l, z in zip(lanes, take(len(lanes))):
+                    f = one + np.float32(std) * z
+                    w[l] = w[l] - f * down[l] if q[l][r][1] else w[l] + f * up[l]
+                    w[l] = max(min(w[l], hi[l]), lo[l])
+
+    q = [[] for _ in range(n_lanes)]
+    for g in range(0, len(rows), 4):
+        for s in rows[g : g + 4]:
+            for l in range(n_lanes):
+                if counts[s, l]:
+                    q[l].append((int(counts[s, l]), bool(dirs[s, l])))
+        if max(len(e) for e in q) > 20:
+            drain(q)
+            q = [[] for _ in range(n_lanes)]
+    drain(q)
+    return int(counts.sum(0).max())
+
+
+@pytest.mark.parametrize("x_size,d_size,m,bl,scale,layout", [
+    (3, 33, 32, 1, 0.9, "rows"),     # one block, one slot, lines past a warp
+    (5, 31, 33, 1, 1.0, "rows"),     # every row pulses: rounds start inside words
+    (2, 64, 97, 2, 0.6, "trans"),    # ragged last block, two slots, transposed inputs
+    (65, 7, 130, 3, 0.3, "rows"),    # sparse: a group of four rows spans words
+    (4, 40, 70, 4, 0.8, "rows"),     # the first train of more than three slots
+    (3, 32, 45, 31, 0.7, "trans"),   # longest train of one segment, many pulses per event
+    (2, 35, 40, 40, 0.5, "rows"),    # two segments per sample
+])
+def test_pulses_and_noise_event_by_event(x_size, d_size, m, bl, scale, layout):
+    from aihwkit_b200.rpu_base import devices as D
+    from aihwkit_b200.rpu_base import tiles as T
+
+    rng = np.random.default_rng(x_size * 1000 + m)
+    p = D.AnalogTileParameter()
+    p.update.pulse_type, p.update.desired_bl = D.PulseType.StochasticCompressed, bl
+    p.update.update_management = p.update.update_bl_management = False
+    p.update.fixed_bl = True
+    dp = D.ConstantStepResistiveDeviceParameter()
+    dp.dw_min, dp.dw_min_std, dp.construction_seed, dp.enforce_consistency = 0.002, 0.3, 11, True
+    t = T.AnalogTile(p._config(x_size, d_size, dp, seed=17), cuda_device=0)
+    seed = (5 << 32) | 1234567
+    t.set_seed(seed)
+    key = (seed & 0xFFFFFFFF, (seed >> 32) ^ 0x5BD1E995)
+    lr = 0.002 * bl  # strength sqrt(lr / (dw_min * bl)) = 1
+    t.set_learning_rate(lr)
+    strength = np.sqrt(np.float32(lr) / (np.float32(0.002) * np.float32(bl))).astype(np.float32)
+    x = (rng.uniform(0.2, 1, (m, x_size)) * rng.choice([-1, 1], (m, x_size)) * scale).astype(np.float32)
+    d = (rng.uniform(0.2, 1, (m, d_size)) * rng.choice([-1, 1], (m, d_size)) * scale).astype(np.float32)
+    x[rng.random((m, x_size)) < 0.2] = 0.0
+    names = t.get_hidden_parameter_names()
+    hp = t.get_hidden_parameters().numpy()
+    hi, lo, up, down = (hp[names.index(k)] for k in ("max_bound", "min_bound", "dwmin_up", "dwmin_down"))
+    w = np.clip(rng.uniform(-0.3, 0.3, (d_size, x_size)), lo, hi).astype(np.float32)
+    t.set_weights(torch.from_numpy(w))
+    xt, dt = torch.from_numpy(x).cuda(), torch.from_numpy(d).cuda()
+    if layout == "trans":
+        t.update(xt.t().contiguous(), dt.t().contiguous(), False, True, True)
+    else:
+        t.update(xt, dt)
+    got = t.get_weights().numpy()
+
+    # rows: samples, or the segments of at most 31 slots of each
+    n_seg = (bl + 30) // 31
+    px, pd = _trains(x, strength, bl, key, TAG_X), _trains(d, strength, bl, key, TAG_D)
+    busiest = 0
+    for j in range(x_size):
+        cut = [slice(31 * g, min(bl, 31 * g + 31)) for g in range(n_seg)]
+        counts = np.stack([(px[:, j, None, c] & pd[:, :, c]).sum(-1) for c in cut], 1).reshape(m * n_seg, d_size)
+        rows = np.flatnonzero(np.stack([px[:, j, c].any(-1) for c in cut], 1).reshape(-1))
+        dirs = np.repeat((x[:, j, None] > 0) == (d > 0), n_seg, axis=0)  # equal signs: decrease
+        for i0 in range(0, d_size, 32):
+            s = slice(i0, min(i0 + 32, d_size))
+            task = j * ((d_size + 31) // 32) + i0 // 32
+            col = w[s, j].copy()
+            busiest = max(busiest, _apply_task(col, hi[s, j], lo[s, j], up[s, j], down[s, j], counts[:, s],
+                                               dirs[:, s], rows, 0.3, task, key))
+            w[s, j] = col
+    # one rounding of a value below 1 per pulse may fall the other way (the device's logarithm, sine and
+    # cosine are approximations); a Gaussian given to another pulse moves a weight by about 6e-4
+    assert np.abs(got - w).max() <= busiest * 2.0 ** -24
+    assert busiest > 3
