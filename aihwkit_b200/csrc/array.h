@@ -88,8 +88,10 @@ private:
   std::unique_ptr<TcEngine> tc_;
   std::vector<uint64_t> tc_versions_;
   bool tcEligible(int m);
+  bool smallEligible(int m);
   // x0 points at the first locally owned column of row 0, x_ss is the row pitch
   void forwardImpl(const float *x0, long long x_ss, float *y, int m, cudaStream_t s);
+  void forwardSmall(const float *x0, long long x_ss, float *y, int m, cudaStream_t s);
   void forwardTc(const float *x0, long long x_ss, float *y, int m, cudaStream_t s);
   // host-buffer path: the batch is cut into row chunks that flow through a three-stage pipeline
   // (host -> device copy, kernels, device -> host copy) on three streams with two buffers each

@@ -194,6 +194,17 @@ gauss4(PhiloxKey key, uint64_t blk, uint32_t call, uint32_t tag, float z[4]) {
   boxMuller16(odd ? r[3] : r[1], z[2], z[3]);
 }
 
+// normal number q (0..3) of noise block `blk`, without the others
+__device__ __forceinline__ float gaussOf4(PhiloxKey key, uint64_t blk, uint32_t call, uint32_t tag, int q) {
+  uint32_t r[4];
+  const uint64_t pair = blk >> 1;
+  philox4x32<7>((uint32_t)pair, (uint32_t)(pair >> 32), call, tag, key, r);
+  const uint32_t lo = q < 2 ? r[0] : r[1], hi = q < 2 ? r[2] : r[3];
+  float z0, z1;
+  boxMuller16((blk & 1) != 0 ? hi : lo, z0, z1);
+  return (q & 1) != 0 ? z1 : z0;
+}
+
 // eight standard normals for the block pair `pair` (blocks 2 * pair and 2 * pair + 1 of gauss4)
 __device__ __forceinline__ void
 gauss8(PhiloxKey key, uint64_t pair, uint32_t call, uint32_t tag, float z[8]) {

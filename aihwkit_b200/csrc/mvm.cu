@@ -14,6 +14,8 @@
 #include "mvm_common.cuh"
 #include "tile.h"
 
+#include <algorithm>
+
 namespace ab200 {
 
 // ---------------------------------------------------------------------------------------------
@@ -123,15 +125,11 @@ __global__ void nmAverageKernel(float *sval, int m, float decay, float *state) {
 // PCM ("line chain"): also accumulate per output sum_k |w| v^2 (variance factor of the PCMRead
 // weight noise), sum_k |w| |v| (line current) and sum_k w v posw(k) (position-weighted product) for
 // the IR drop, and run the long output chain (lineChain) instead of the merged noise draw.
-// NMF (small problems, T = 1): the noise management of the CTA's sixteen rows runs in the prologue
-// instead of a kernel of its own - sixteen threads per row reduce the row's statistics, every
-// column CTA of a row block repeats that (a few KB), and the first one leaves the per-row values
-// for the bound-management re-run. One launch less per pass where launches are what a pass costs.
 // PN (with PCM): the negative and the positive prepared inputs accumulate separately, with the
 // norm of each half, and the epilogue runs the analog chain of the line once per half before it
 // adds them in front of (pos_neg = 1) or behind (pos_neg = 2) the output stage
 // (computeAnalogMV, rpu_forward_backward_pass.cpp:820-876).
-template <bool A_K_FAST, bool B_N_FAST, int T, bool PCM, bool NMF = false, bool PN = false>
+template <bool A_K_FAST, bool B_N_FAST, int T, bool PCM, bool PN = false>
 __global__ void __launch_bounds__(256) mvmSimtKernel(MvmProblem p) {
   static_assert(!PN || PCM, "separate passes use the line-chain variant");
   constexpr int S = PN ? 2 : 1; // accumulator sets: [negative inputs, positive inputs] or one
@@ -141,7 +139,6 @@ __global__ void __launch_bounds__(256) mvmSimtKernel(MvmProblem p) {
   __shared__ float As[BK][BM + 4];
   __shared__ float Bs[BK][BN + 4];
   __shared__ float s_scale[BM];
-  __shared__ float s_fac[NMF ? BM : 1];
   const IOEff &io = p.io;
   const int tid = threadIdx.x;
   const int tx = tid & 15, ty = tid >> 4;
@@ -149,47 +146,7 @@ __global__ void __launch_bounds__(256) mvmSimtKernel(MvmProblem p) {
   const int K = p.in_size, N = p.out_size;
   const ElemRng g{p.key, p.call, (p.backward ? TAG_BWD_IN : TAG_FWD_IN) + p.noise_id};
 
-  if (NMF) {
-    // BM = 16 rows, 16 threads per row
-    const int r = tid >> 4, part = tid & 15;
-    const int gr = row0 + r;
-    NmStats st;
-    if (gr < p.m && nmNeedsStats(io)) {
-      const float *row = p.in + (long long)gr * p.in_ss;
-      for (int k = part; k < K; k += 16) {
-        st.add(k < p.in_real ? row[(long long)k * p.in_fs] : 1.0f);
-      }
-    }
-#pragma unroll
-    for (int o = 8; o > 0; o >>= 1) {
-      st.amax = fmaxf(st.amax, __shfl_xor_sync(0xffffffffu, st.amax, o));
-      st.vmax = fmaxf(st.vmax, __shfl_xor_sync(0xffffffffu, st.vmax, o));
-      st.psum += __shfl_xor_sync(0xffffffffu, st.psum, o);
-      st.nsum += __shfl_xor_sync(0xffffffffu, st.nsum, o);
-    }
-    if (part == 0) {
-      float scale = 0.0f, fac = 0.0f;
-      if (gr < p.m) {
-        const float sval = nmValue(io, st);
-        scale = inputScale(io, sval, /*reduction=*/1.0f, !p.backward);
-        fac = outputFactor(io, p.alpha, sval, scale, p.backward);
-        if (blockIdx.x == 0) {
-          // what the bound-management re-run reads; the flags are zero between passes (the
-          // re-run clears the ones it has served)
-          p.scale[gr] = scale;
-          p.sval[gr] = sval;
-          p.factor[gr] = fac;
-          p.vnorm[gr] = 0.0f;
-        }
-      }
-      s_scale[r] = scale;
-      s_fac[NMF ? r : 0] = fac;
-    }
-    if (blockIdx.x == 0 && blockIdx.y == 0 && tid == 0 && !p.backward && p.bm_stats) {
-      p.bm_stats[0] = 0;
-      p.bm_stats[1] = 0;
-    }
-  } else if (tid < BM) {
+  if (tid < BM) {
     int r = row0 + tid;
     s_scale[tid] = r < p.m ? p.scale[r] : 0.0f;
   }
@@ -304,7 +261,7 @@ __global__ void __launch_bounds__(256) mvmSimtKernel(MvmProblem p) {
       continue;
     }
     float sc = s_scale[ty * T + i];
-    float fac = NMF ? s_fac[NMF ? ty * T + i : 0] : p.factor[r];
+    float fac = p.factor[r];
     float y[T];
 #pragma unroll
     for (int j = 0; j < T; j++) {
@@ -323,7 +280,7 @@ __global__ void __launch_bounds__(256) mvmSimtKernel(MvmProblem p) {
       }
     } else {
       const bool line_sigma = p.out_noise_vals != nullptr;
-      const float vn = NMF ? 0.0f : p.vnorm[r];
+      const float vn = p.vnorm[r];
       float sigma = PCM ? io.out_noise : outputSigma(io, vn);
       const uint64_t blk = (uint64_t)r * n4 + (uint64_t)(c >> 2);
       const bool w_draw = PCM && io.w_noise > 0.0f && io.w_noise_type != AB200_WNOISE_NONE;
@@ -407,16 +364,35 @@ __global__ void __launch_bounds__(256) mvmSimtKernel(MvmProblem p) {
 // is an independent mat-vec with a halved input scale per round, exactly the per-sample loop of
 // the reference CPU tile. Nothing is copied to the host.
 // ---------------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) bmRerunKernel(MvmProblem p) {
+constexpr int BM_THREADS = 1024;
+
+__global__ void __launch_bounds__(BM_THREADS) bmRerunKernel(MvmProblem p, int n_slices, int k_slice) {
   pdlEnter();
-  extern __shared__ float v_sh[]; // K prepared inputs
+  extern __shared__ float v_sh[]; // K prepared inputs, then the partial sums of the K slices
   const IOEff &io = p.io;
   const int K = p.in_size, N = p.out_size;
   const uint64_t n4 = (uint64_t)(((N + 7) >> 3) << 1);
-  for (int r = blockIdx.x; r < p.m; r += gridDim.x) {
-    if (p.flags[r] == 0) {
-      continue;
+  float *const part_sh = v_sh + K;
+  const int n_cb = (N + 31) / 32, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  // The flags of up to blockDim.x of this CTA's rows are read together: in the usual case, no row
+  // clipped, a walk over them one after the other is all the kernel would spend its time on (131072 rows:
+  // 113 us of dependent loads against 25).
+  __shared__ int todo[BM_THREADS], n_todo;
+  for (long long base = blockIdx.x; base < p.m; base += (long long)gridDim.x * BM_THREADS) {
+  if (threadIdx.x == 0) {
+    n_todo = 0;
+  }
+  __syncthreads();
+  {
+    const long long mine = base + (long long)threadIdx.x * gridDim.x;
+    if (mine < p.m && p.flags[mine] != 0) {
+      todo[atomicAdd(&n_todo, 1)] = (int)mine;
     }
+  }
+  __syncthreads();
+  const int n_rows = n_todo;
+  for (int at = 0; at < n_rows; at++) {
+    const int r = todo[at];
     float sval = p.sval[r];
     const float *row = p.in + (long long)r * p.in_ss;
     const bool gathered = p.gather.idx != nullptr; // rows read through an index array
@@ -436,7 +412,7 @@ __global__ void __launch_bounds__(256) bmRerunKernel(MvmProblem p) {
                           : (k < p.in_real ? row[(long long)k * p.in_fs] : 1.0f));
         }
         st.warpReduce();
-        __shared__ float st_sh[8][3];
+        __shared__ float st_sh[BM_THREADS / 32][3];
         if ((threadIdx.x & 31) == 0) {
           st_sh[threadIdx.x >> 5][0] = st.amax;
           st_sh[threadIdx.x >> 5][1] = st.psum;
@@ -475,7 +451,7 @@ __global__ void __launch_bounds__(256) bmRerunKernel(MvmProblem p) {
           nacc_n += __shfl_xor_sync(0xffffffffu, nacc_n, o);
           nacc_p += __shfl_xor_sync(0xffffffffu, nacc_p, o);
         }
-        __shared__ float red2_sh[8][2];
+        __shared__ float red2_sh[BM_THREADS / 32][2];
         if ((threadIdx.x & 31) == 0) {
           red2_sh[threadIdx.x >> 5][0] = nacc_n;
           red2_sh[threadIdx.x >> 5][1] = nacc_p;
@@ -500,6 +476,23 @@ __global__ void __launch_bounds__(256) bmRerunKernel(MvmProblem p) {
       const uint32_t round_tag_u = TAG_FWD_OUT_U + p.noise_id + (uint32_t)round * 0x10000u;
       const bool w_draw = io.w_noise > 0.0f && io.w_noise_type != AB200_WNOISE_NONE;
       int fail = 0;
+      if (n_slices > 1) {
+        // fewer blocks of 32 columns than warps: the warps share slices of K
+        for (int t = warp; t < n_cb * n_slices; t += BM_THREADS / 32) {
+          const int cb = t % n_cb, sl = t / n_cb, n = cb * 32 + lane;
+          const int k1 = min(K, (sl + 1) * k_slice);
+          const float *wp = p.w + (long long)(n < N ? n : 0) * p.wn;
+          float a = 0.0f;
+#pragma unroll 16
+          for (int k = sl * k_slice; k < k1; k++) {
+            a = fmaf(v_sh[k], wp[(long long)k * p.wk], a);
+          }
+          if (n < N) {
+            part_sh[sl * N + n] = a;
+          }
+        }
+        __syncthreads();
+      }
       for (int n = threadIdx.x; n < N; n += blockDim.x) {
         // accumulator sets: [0] the only pass, or the pass over the positive inputs; [1] the
         // pass over the negative inputs
@@ -526,7 +519,12 @@ __global__ void __launch_bounds__(256) bmRerunKernel(MvmProblem p) {
             acc_c[0] = fmaf(fabsf(v), fabsf(wv), acc_c[0]);
             acc_i[0] = fmaf(v * irPosWeight(k, K), wv, acc_i[0]);
           }
+        } else if (n_slices > 1) {
+          for (int sl = 0; sl < n_slices; sl++) {
+            acc[0] += part_sh[sl * N + n];
+          }
         } else {
+#pragma unroll 8
           for (int k = 0; k < K; k++) {
             acc[0] = fmaf(v_sh[k], wp[(long long)k * p.wk], acc[0]);
           }
@@ -599,9 +597,15 @@ __global__ void __launch_bounds__(256) bmRerunKernel(MvmProblem p) {
     }
     __syncthreads();
   }
+  __syncthreads();
+  }
 }
 
 void launchMvmSimt(const MvmProblem &p, cudaStream_t stream) {
+  if (smallMvmEligible(p)) {
+    launchMvmSmallTile(p, stream);
+    return;
+  }
   // noise management
   bool sample_contig = p.in_fs == 1;
   auto nmPass = [&](int mode) {
@@ -615,32 +619,11 @@ void launchMvmSimt(const MvmProblem &p, cudaStream_t stream) {
   };
   const bool running = !p.io.is_perfect && (p.io.nm == AB200_NM_AVERAGE_ABS_MAX ||
                                             p.io.nm == AB200_NM_AVERAGE_ABS_MAX_SINGLE_VALUE);
-  // small problems (the 16 x 16 tile is chosen below) without per-row norms or running values:
-  // the noise management goes into the prologue of the product kernel
   static int n_sm = 0; // SMs of the GPUs of this process (one kind per process)
   if (n_sm == 0) {
     int dev = 0;
     AB200_CUDA(cudaGetDevice(&dev));
     AB200_CUDA(cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev));
-  }
-  const long long ctas2 = (long long)((p.out_size + 31) / 32) * ((p.m + 31) / 32);
-  const bool fused_nm = !running && !ioNeedsLineChain(p.io) && ctas2 < n_sm && p.in_size <= 4096 &&
-                        !(p.io.w_noise_type == AB200_WNOISE_ADDITIVE_CONSTANT && p.io.w_noise > 0.0f &&
-                          !p.io.is_perfect);
-  if (fused_nm) {
-    dim3 grid((p.out_size + 15) / 16, (p.m + 15) / 16);
-    const bool a_k = p.in_fs == 1, b_n = p.wn == 1;
-    if (a_k && b_n) {
-      AB200_CUDA(launchChained(mvmSimtKernel<true, true, 1, false, true>, grid, dim3(256), 0, stream, p));
-    } else if (a_k) {
-      AB200_CUDA(launchChained(mvmSimtKernel<true, false, 1, false, true>, grid, dim3(256), 0, stream, p));
-    } else if (b_n) {
-      AB200_CUDA(launchChained(mvmSimtKernel<false, true, 1, false, true>, grid, dim3(256), 0, stream, p));
-    } else {
-      AB200_CUDA(launchChained(mvmSimtKernel<false, false, 1, false, true>, grid, dim3(256), 0, stream, p));
-    }
-    AB200_LAUNCH_CHECK();
-    return;
   }
   if (running) {
     if (!p.nm_state) {
@@ -680,13 +663,13 @@ void launchMvmSimt(const MvmProblem &p, cudaStream_t stream) {
     // separate passes: two sets of the line-chain accumulators, the 16-wide tile
     dim3 grid((p.out_size + 15) / 16, (p.m + 15) / 16);
     if (a_k_fast && b_n_fast) {
-      AB200_CUDA(launchChained(mvmSimtKernel<true, true, 1, true, false, true>, grid, dim3(256), 0, stream, p));
+      AB200_CUDA(launchChained(mvmSimtKernel<true, true, 1, true, true>, grid, dim3(256), 0, stream, p));
     } else if (a_k_fast) {
-      AB200_CUDA(launchChained(mvmSimtKernel<true, false, 1, true, false, true>, grid, dim3(256), 0, stream, p));
+      AB200_CUDA(launchChained(mvmSimtKernel<true, false, 1, true, true>, grid, dim3(256), 0, stream, p));
     } else if (b_n_fast) {
-      AB200_CUDA(launchChained(mvmSimtKernel<false, true, 1, true, false, true>, grid, dim3(256), 0, stream, p));
+      AB200_CUDA(launchChained(mvmSimtKernel<false, true, 1, true, true>, grid, dim3(256), 0, stream, p));
     } else {
-      AB200_CUDA(launchChained(mvmSimtKernel<false, false, 1, true, false, true>, grid, dim3(256), 0, stream, p));
+      AB200_CUDA(launchChained(mvmSimtKernel<false, false, 1, true, true>, grid, dim3(256), 0, stream, p));
     }
   } else if (pcm) { // the second accumulator doubles the registers of a thread: the 32-wide tile at most
     if (T >= 2) {
@@ -712,16 +695,22 @@ void launchBmRerun(const MvmProblem &p, cudaStream_t stream) {
   if (p.accumulate) {
     AB200_FATAL("bound management cannot be combined with accumulating outputs");
   }
-  size_t smem = (size_t)p.in_size * sizeof(float);
-  if (smem > 200 * 1024) {
+  if ((size_t)p.in_size * sizeof(float) > 200 * 1024) {
     AB200_FATAL("bound management: x_size too large for the re-run kernel");
   }
-  if (smem > 48 * 1024) {
-    AB200_CUDA(cudaFuncSetAttribute(bmRerunKernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    200 * 1024));
+  // K slices: as many as there are more warps than column blocks, 64 features each at the least (785 x 130,
+  // 10 rows of which some clip: 59 -> 23 us)
+  const int n_cb = (p.out_size + 31) / 32;
+  const int n_slices =
+      ioNeedsLineChain(p.io) ? 1 : std::max(1, std::min(BM_THREADS / 32 / n_cb, p.in_size / 64));
+  const int k_slice = (p.in_size + n_slices - 1) / n_slices;
+  const size_t smem =
+      ((size_t)p.in_size + (n_slices > 1 ? (size_t)n_slices * p.out_size : 0)) * sizeof(float);
+  if (smem > 40 * 1024) {
+    AB200_CUDA(cudaFuncSetAttribute(bmRerunKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 204 * 1024));
   }
-  int blocks = p.m < 592 ? p.m : 592;
-  AB200_CUDA(launchChained(bmRerunKernel, dim3(blocks), dim3(256), smem, stream, p));
+  const int blocks = p.m < 296 ? p.m : 296; // two per SM at the most
+  AB200_CUDA(launchChained(bmRerunKernel, dim3(blocks), dim3(BM_THREADS), smem, stream, p, n_slices, k_slice));
   AB200_LAUNCH_CHECK();
 }
 

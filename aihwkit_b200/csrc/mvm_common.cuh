@@ -170,6 +170,24 @@ __device__ __forceinline__ float prepareInput(const IOEff &io, float x, float sc
   return v;
 }
 
+// The plain DAC with the division left out where it cannot matter: v * inv_res and the correctly rounded
+// v / res differ by at most 9e-5 below a quotient of 512 (two roundings and that of inv_res, 2^-24 each, and
+// one of the division), so they round to the same code unless one is within 1e-4 of a half-integer.
+// Same bits as discretize with the clip behind it.
+__device__ __forceinline__ float dacPlain(const IOEff &io, float inv_res, float x, float scale) {
+  float v = __fmul_rn(x, scale);
+  if (io.res_in > 0.0f) {
+    const float q = __fmul_rn(v, inv_res);
+    float code = rintf(q);
+    if (fabsf(__fsub_rn(q, code)) > 0.4999f || !(fabsf(q) < 512.0f)) {
+      code = rintf(__fdiv_rn(v, io.res_in));
+    }
+    v = __fmul_rn(code, io.res_in);
+  }
+  v = v > io.inp_bound ? io.inp_bound : v;
+  return v < -io.inp_bound ? -io.inp_bound : v;
+}
+
 // Std-dev of the Gaussian added before the ADC: output noise (:695-698) and the additive-constant
 // weight noise w_noise * ||v|| (:341-352) are independent zero-mean Gaussians on the same value,
 // so one draw with the combined variance is statistically identical to two draws.

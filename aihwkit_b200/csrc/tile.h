@@ -140,6 +140,30 @@ void launchMvm(const MvmProblem &p, cudaStream_t stream);
 // bound-management re-run of the rows whose first round clipped (forward only; no-op otherwise)
 void launchBmRerun(const MvmProblem &p, cudaStream_t stream);
 
+// Small batches on CUDA cores (mvm_small.cu): the tiles of a mapped layer, or a single one, in one launch.
+struct SmallTile {
+  const float *w;
+  long long ld; // pitch of the weights: of a feature, or of an output where features are contiguous
+  float alpha;
+  uint32_t call, noise_id;
+  PhiloxKey key;
+};
+constexpr int kSmallSplits = 32, kSmallTiles = 72; // per launch
+struct SmallSplits {
+  int n_in, n_out;
+  int in_off[kSmallSplits], in_size[kSmallSplits];
+  int out_off[kSmallSplits], out_size[kSmallSplits];
+  int col_blk[kSmallSplits + 1]; // first column block of every out-split (set by the launch)
+  int vec;                       // weights may be read in fours along k (set by the launch)
+  const float *bias;             // added once per output column, or null
+  SmallTile tile[kSmallTiles];   // [in-split][out-split]
+};
+bool smallMvmIo(const IOEff &io); // IO settings these kernels implement
+int smallMvmMaxCtas();            // column blocks of 32 times row blocks of 16 up to which they are used
+bool smallMvmEligible(const MvmProblem &p);
+void launchMvmSmall(const MvmProblem &p, SmallSplits &sp, cudaStream_t stream);
+void launchMvmSmallTile(const MvmProblem &p, cudaStream_t stream);
+
 // Kernel selection for the MVM: 0 = automatic, 1 = always CUDA cores, 2 = tensor cores whenever
 // the problem can be expressed on them.
 void setMvmPath(int mode);
@@ -377,6 +401,7 @@ public:
   uint64_t weightsVersion() const { return w_version_; }
   PhiloxKey noiseKey() const { return key_; }
   uint32_t nextForwardCall() { return fwd_calls_++; }
+  const float *forwardWeights(bool is_test) const { return fbWeights(is_test); }
 
 private:
   void requireDevice(const char *what) const;

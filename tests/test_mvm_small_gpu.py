@@ -1,0 +1,61 @@
+"""The CUDA-core kernel for small batches at the edges of its tiles: rows 4 / 8 / 16 per CTA, columns in 32s,
+features in steps of 512, and the tiles of a mapped layer in one launch."""
+
+import numpy as np
+import pytest
+import torch
+
+from tests import helpers as H
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("m", [1, 4, 5, 8, 9, 16, 17])
+@pytest.mark.parametrize("x_size,d_size", [(1, 33), (31, 1), (64, 32), (130, 785), (512, 96), (513, 31), (1030, 40)])
+def test_perfect_io_against_float64(m, x_size, d_size):
+    from aihwkit_b200.rpu_base import tiles as T
+
+    g = torch.Generator().manual_seed(m * 10000 + x_size)
+    t = T.FloatingPointTile(x_size, d_size, cuda_device=0)
+    w = torch.rand(d_size, x_size, generator=g) - 0.5
+    t.set_weights(w)
+    x, d = torch.rand(m, x_size, generator=g) - 0.5, torch.rand(m, d_size, generator=g) - 0.5
+    y, gr = t.forward(x.cuda()).cpu().double(), t.backward(d.cuda()).cpu().double()
+    # K products of at most 1/4 and K - 1 additions in fp32, each rounded once
+    for got, a, b, k in ((y, x, w.t(), x_size), (gr, d, w, d_size)):
+        assert (got - a.double() @ b.double()).abs().max() <= k * k * 0.25 * 2.0 ** -24
+
+
+@pytest.mark.parametrize("out_size,in_size,max_tile,m", [
+    (96, 64, 64, 3), (33, 200, 70, 7), (700, 130, 64, 16), (1536, 384, 192, 21), (100, 2300, 64, 2)])
+def test_mapped_layer_against_its_tiles_one_by_one(out_size, in_size, max_tile, m):
+    """Scaled tiles, bias and all noise on: the layer in one launch against single tiles with the same
+    weights, noise streams and rows, added up in the order of the in-splits."""
+    from aihwkit_b200 import _cabi
+    from aihwkit_b200.rpu_base import tiles as T
+
+    rng = np.random.default_rng(out_size + in_size)
+    cfg = H.inference_params(True)._config(max_tile, max_tile, H.D.IdealResistiveDeviceParameter(), seed=3)
+    w = torch.from_numpy(rng.normal(0, 0.1, (out_size, in_size)).astype(np.float32))
+    x = torch.from_numpy(rng.normal(0, 1, (m, in_size)).astype(np.float32)).cuda()
+    bias = torch.from_numpy(rng.normal(0, 0.1, out_size).astype(np.float32))
+    out = []
+    lib = _cabi.lib()
+    try:
+        for path in (0, 2):  # the fp32 kernel for small batches, the tensor-core kernel
+            _cabi.check(lib.ab200_set_mvm_path(path))
+            layer = T.TileArray(cfg, out_size, in_size, max_tile, max_tile, cuda_device=0)
+            layer.set_seed(77)
+            layer.set_weights(w, weight_scaling_omega=1.0)
+            layer.set_bias(bias)
+            layer.forward(x)
+            out.append(layer.forward(x).cpu().double())  # second call: the call counters advanced alike
+            scales = layer.get_tile_scales()
+    finally:
+        _cabi.check(lib.ab200_set_mvm_path(0))
+    # the split-bf16 weights move a sum by less than an ADC step: a code differs by one where the sum is
+    # next to a rounding tie, in the scale of the largest tile and input
+    step = 2 * 10.0 / 254.0 * float(scales.max()) * float(x.abs().max())
+    diff = (out[0] - out[1]).abs()
+    assert diff.max() <= 2.01 * step
+    assert (diff > 1e-4 * step).double().mean() <= 0.002 * scales.size(0) + 2.0 / diff.numel()
