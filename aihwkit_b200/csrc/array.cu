@@ -438,7 +438,7 @@ bool TileArray::smallEligible(int m) {
   for (int oi = out_begin_; oi < out_end_; oi++) {
     blocks += (out_sizes_[oi] + 31) / 32;
   }
-  return blocks * ((m + 15) / 16) <= smallMvmMaxCtas();
+  return blocks * ((m + 15) / 16) <= smallMvmMaxCtas(in_sizes_[in_begin_]);
 }
 
 void TileArray::forwardSmall(const float *x0, long long x_ss, float *y, int m, cudaStream_t s) {

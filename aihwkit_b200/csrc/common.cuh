@@ -258,6 +258,23 @@ gauss8Keyed(const Philox7Keys &k, uint64_t pair, uint32_t call, uint32_t tag, fl
   boxMuller16(r[3], z[6], z[7]);
 }
 
+// T neighbouring values from shared memory in one load
+template <int T> __device__ __forceinline__ void loadRow(const float *src, float *dst) {
+  if (T == 4) {
+    const float4 v = *reinterpret_cast<const float4 *>(src);
+    dst[0] = v.x;
+    dst[T > 1 ? 1 : 0] = v.y;
+    dst[T > 2 ? 2 : 0] = v.z;
+    dst[T > 3 ? 3 : 0] = v.w;
+  } else if (T == 2) {
+    const float2 v = *reinterpret_cast<const float2 *>(src);
+    dst[0] = v.x;
+    dst[T > 1 ? 1 : 0] = v.y;
+  } else {
+    dst[0] = src[0];
+  }
+}
+
 // getDiscretizedValueSR<false> (src/rpucuda/utility_functions.h:204-210): rint(v / res) * res with
 // round-half-to-even, as separate correctly-rounded fp32 operations (no FMA contraction).
 __device__ __forceinline__ float discretize(float v, float res) {

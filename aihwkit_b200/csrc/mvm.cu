@@ -136,8 +136,8 @@ __global__ void __launch_bounds__(256) mvmSimtKernel(MvmProblem p) {
   pdlEnter();
   constexpr int BM = 16 * T, BN = 16 * T;
   constexpr int BK = T == 1 ? 64 : (T == 2 ? 32 : 16);
-  __shared__ float As[BK][BM + 4];
-  __shared__ float Bs[BK][BN + 4];
+  __shared__ __align__(16) float As[2][BK][BM + 4];
+  __shared__ __align__(16) float Bs[2][BK][BN + 4];
   __shared__ float s_scale[BM];
   const IOEff &io = p.io;
   const int tid = threadIdx.x;
@@ -148,7 +148,12 @@ __global__ void __launch_bounds__(256) mvmSimtKernel(MvmProblem p) {
 
   if (tid < BM) {
     int r = row0 + tid;
-    s_scale[tid] = r < p.m ? p.scale[r] : 0.0f;
+    // (perfect IO has no per-row values: no noise-management pass ran)
+    s_scale[tid] = io.is_perfect ? 1.0f : (r < p.m ? p.scale[r] : 0.0f);
+  }
+  if (io.is_perfect && blockIdx.x == 0 && blockIdx.y == 0 && tid == 0 && !p.backward && p.bm_stats) {
+    p.bm_stats[0] = 0;
+    p.bm_stats[1] = 0;
   }
   __syncthreads();
 
@@ -172,54 +177,73 @@ __global__ void __launch_bounds__(256) mvmSimtKernel(MvmProblem p) {
     }
   }
 
-  for (int k0 = 0; k0 < K; k0 += BK) {
+  // Operands of a step go through registers into one of two buffers: the loads of step k + 1 are in flight
+  // while step k is multiplied, one barrier per step.
+  constexpr int NE = BM * BK / 256; // elements of each operand per thread (BM == BN)
+  const bool plain = !io.is_perfect && !inputIsRandom(io) && io.inp_asym == 1.0f;
+  const float inv_res = __fdiv_rn(1.0f, io.res_in); // (read with res_in > 0 only)
+  float ra[NE], rb[NE];
+  auto load = [&](int k0) {
 #pragma unroll
-    for (int e = tid; e < BM * BK; e += 256) {
-      int r, kk;
-      if (A_K_FAST) {
-        kk = e % BK;
-        r = e / BK;
-      } else {
-        r = e % BM;
-        kk = e / BM;
-      }
-      int gr = row0 + r, gk = k0 + kk;
-      float v = 0.0f;
+    for (int u = 0; u < NE; u++) {
+      const int e = tid + u * 256;
+      const int kk = A_K_FAST ? e % BK : e / BM, r = A_K_FAST ? e / BK : e % BM;
+      const int gr = row0 + r, gk = k0 + kk;
+      ra[u] = 0.0f;
       if (gr < p.m && gk < K) {
-        float sc = s_scale[r];
-        if (sc != 0.0f) {
-          float xin = gk < p.in_real ? p.in[(long long)gr * p.in_ss + (long long)gk * p.in_fs] : 1.0f;
-          v = prepareInput(io, xin, sc, g, (uint32_t)gr, (uint32_t)gk);
+        ra[u] = 1.0f; // the bias line
+        if (gk < p.in_real) {
+          ra[u] = p.in[(long long)gr * p.in_ss + (long long)gk * p.in_fs];
         }
       }
-      As[kk][r] = v;
     }
 #pragma unroll
-    for (int e = tid; e < BN * BK; e += 256) {
-      int n, kk;
-      if (B_N_FAST) {
-        n = e % BN;
-        kk = e / BN;
-      } else {
-        kk = e % BK;
-        n = e / BK;
+    for (int u = 0; u < NE; u++) {
+      const int e = tid + u * 256;
+      const int n = B_N_FAST ? e % BN : e / BK, kk = B_N_FAST ? e / BN : e % BK;
+      const int gk = k0 + kk, gn = col0 + n;
+      rb[u] = 0.0f;
+      if (gk < K && gn < N) {
+        rb[u] = p.w[(long long)gk * p.wk + (long long)gn * p.wn];
       }
-      int gk = k0 + kk, gn = col0 + n;
-      Bs[kk][n] = (gk < K && gn < N) ? p.w[(long long)gk * p.wk + (long long)gn * p.wn] : 0.0f;
     }
-    __syncthreads();
+  };
+  auto stage = [&](int buf, int k0) {
+#pragma unroll
+    for (int u = 0; u < NE; u++) {
+      const int e = tid + u * 256;
+      const int kk = A_K_FAST ? e % BK : e / BM, r = A_K_FAST ? e / BK : e % BM;
+      const float sc = s_scale[r];
+      float v = 0.0f;
+      if (io.is_perfect) {
+        v = ra[u];
+      } else if (sc != 0.0f && k0 + kk < K) {
+        v = plain ? dacPlain(io, inv_res, ra[u], sc)
+                  : prepareInput(io, ra[u], sc, g, (uint32_t)(row0 + r), (uint32_t)(k0 + kk));
+      }
+      As[buf][kk][r] = v;
+    }
+#pragma unroll
+    for (int u = 0; u < NE; u++) {
+      const int e = tid + u * 256;
+      const int n = B_N_FAST ? e % BN : e / BK, kk = B_N_FAST ? e / BN : e % BK;
+      Bs[buf][kk][n] = rb[u];
+    }
+  };
+  load(0);
+  stage(0, 0);
+  __syncthreads();
+  for (int k0 = 0, buf = 0; k0 < K; k0 += BK, buf ^= 1) {
+    const bool more = k0 + BK < K;
+    if (more) {
+      load(k0 + BK);
+    }
 #pragma unroll
     for (int kk = 0; kk < BK; kk++) {
       float a[T], b[T];
       const float posw = PCM ? irPosWeight(k0 + kk, K) : 0.0f;
-#pragma unroll
-      for (int i = 0; i < T; i++) {
-        a[i] = As[kk][ty * T + i];
-      }
-#pragma unroll
-      for (int j = 0; j < T; j++) {
-        b[j] = Bs[kk][tx * T + j];
-      }
+      loadRow<T>(&As[buf][kk][ty * T], a);
+      loadRow<T>(&Bs[buf][kk][tx * T], b);
 #pragma unroll
       for (int h = 0; h < S; h++) {
 #pragma unroll
@@ -242,6 +266,9 @@ __global__ void __launch_bounds__(256) mvmSimtKernel(MvmProblem p) {
         }
       }
     }
+    if (more) {
+      stage(buf ^ 1, k0 + BK);
+    }
     __syncthreads();
   }
 
@@ -261,7 +288,7 @@ __global__ void __launch_bounds__(256) mvmSimtKernel(MvmProblem p) {
       continue;
     }
     float sc = s_scale[ty * T + i];
-    float fac = p.factor[r];
+    float fac = io.is_perfect ? __fmul_rn(io.out_scale, p.alpha) : p.factor[r];
     float y[T];
 #pragma unroll
     for (int j = 0; j < T; j++) {
@@ -634,17 +661,17 @@ void launchMvmSimt(const MvmProblem &p, cudaStream_t stream) {
                              p.nm_state));
     AB200_LAUNCH_CHECK();
     nmPass(2);
-  } else {
+  } else if (!p.io.is_perfect) {
     nmPass(0);
   }
 
   const bool a_k_fast = p.in_fs == 1;
   const bool b_n_fast = p.wn == 1;
-  // the largest tile that still gives every SM a CTA
+  // the largest tile that still gives two SMs in three a CTA (64 x 64) or every SM one (32 x 32)
   auto ctas = [&](int t) {
     return (long long)((p.out_size + 16 * t - 1) / (16 * t)) * ((p.m + 16 * t - 1) / (16 * t));
   };
-  const int T = ctas(4) >= n_sm ? 4 : (ctas(2) >= n_sm ? 2 : 1);
+  const int T = 3 * ctas(4) >= 2 * n_sm ? 4 : (ctas(2) >= n_sm ? 2 : 1);
   const bool pcm = ioNeedsLineChain(p.io);
 #define AB200_SIMT(TT, PCM)                                                                        \
   {                                                                                                \

@@ -320,17 +320,19 @@ bool smallMvmIo(const IOEff &io) {
   return !running && !ioNeedsLineChain(io) && !ioLineSigma(io);
 }
 
-int smallMvmMaxCtas() {
+int smallMvmMaxCtas(int in_size) {
   // Four rounds of one CTA per SM; with more, the 64 x 64 tiles of the general kernel fill the GPU as well and
   // load less per product. 2048 x 2048, forward, this kernel against the general one: 16 rows (64 CTAs) 28
   // against 91 us, 64 rows (256) 56 against 179; 4096 x 4096, 32 rows (256) 109 against 367.
+  // Short rows leave most of a CTA's 512 features empty: 64 x 64, 4000 rows (500 CTAs) 22.6 against 17.9 us, but
+  // 128 x 128, 1000 rows (252) 13.3 against 15.4.
   static int n_sm = 0; // SMs of the GPUs of this process (one kind per process)
   if (n_sm == 0) {
     int dev = 0;
     AB200_CUDA(cudaGetDevice(&dev));
     AB200_CUDA(cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev));
   }
-  return 4 * n_sm;
+  return (in_size > 128 ? 4 : 2) * n_sm;
 }
 
 template <int ROWS> static void launchRows(const MvmProblem &p, const SmallSplits &sp, bool k_fast, cudaStream_t stream) {
@@ -370,7 +372,7 @@ bool smallMvmEligible(const MvmProblem &p) {
       !smallMvmIo(p.io)) {
     return false;
   }
-  return (long long)((p.out_size + 31) / 32) * ((p.m + 15) / 16) <= smallMvmMaxCtas();
+  return (long long)((p.out_size + 31) / 32) * ((p.m + 15) / 16) <= smallMvmMaxCtas(p.in_size);
 }
 
 void launchMvmSmallTile(const MvmProblem &p, cudaStream_t stream) {

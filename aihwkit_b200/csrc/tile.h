@@ -159,7 +159,7 @@ struct SmallSplits {
   SmallTile tile[kSmallTiles];   // [in-split][out-split]
 };
 bool smallMvmIo(const IOEff &io); // IO settings these kernels implement
-int smallMvmMaxCtas();            // column blocks of 32 times row blocks of 16 up to which they are used
+int smallMvmMaxCtas(int in_size); // column blocks of 32 times row blocks of 16 up to which they are used
 bool smallMvmEligible(const MvmProblem &p);
 void launchMvmSmall(const MvmProblem &p, SmallSplits &sp, cudaStream_t stream);
 void launchMvmSmallTile(const MvmProblem &p, cudaStream_t stream);

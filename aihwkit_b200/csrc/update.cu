@@ -448,6 +448,111 @@ static void launchUpdateInstance(const UpdateProblem &p, dim3 grid, cudaStream_t
   }
 }
 
+// ---------------------------------------------------------------------------------------------
+// Implicit pulses without device noise: every pair of lines of a sample has a value, so there is nothing to
+// skip and nothing to look up but n = rint(d * BL * x) (dense_bit_line_maker.cpp:240-264). A thread
+// owns EJ weights of one d-line and takes the samples in order; the warp applies pulse k of a sample to the
+// weights with more than k of them, all EJ chains at once, until none is left. Bound by the instructions of
+// that (17 per pair and warp at 1.9 pulses for the busiest of 128 weights). The staged kernel searched bitmaps
+// that are all ones and took one event per lane and round: 512 x 512, 128 samples, 245 -> 39 us.
+// ---------------------------------------------------------------------------------------------
+constexpr int UD_I = 64;    // d-lines per CTA
+constexpr int UD_S = 64;    // samples staged at a time
+constexpr int UD_T = 4;     // groups of 64 threads, EJ x-lines each
+
+template <int KIND, int EJ> __global__ void __launch_bounds__(UD_I *UD_T) pulsedUpdateDenseKernel(UpdateProblem p) {
+  pdlEnter();
+  constexpr int UJ = UD_T * EJ;
+  __shared__ float sd[UD_S][UD_I];
+  __shared__ __align__(16) float sx[UD_S][UJ];
+  const int ti = threadIdx.x % UD_I, tj = threadIdx.x / UD_I;
+  const int i = blockIdx.x * UD_I + ti, j0 = blockIdx.y * UJ;
+  const bool i_ok = i < p.d_size;
+  const bool small = p.up.desired_bl < (1 << 20); // |d BL x| <= BL: rounded by adding 1.5 * 2^23
+  float w[EJ], w_in[EJ];
+  PulseStep<KIND> step[EJ];
+  bool flip[EJ];
+#pragma unroll
+  for (int t = 0; t < EJ; t++) {
+    const int j = j0 + tj * EJ + t;
+    const bool ok = i_ok && j < p.x_size;
+    const long long idx = ok ? (long long)j * p.d_size + i : 0;
+    float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
+    float2 e = make_float2(0.f, 0.f);
+    w[t] = 0.0f;
+    flip[t] = false;
+    if (ok) {
+      w[t] = p.w[idx];
+      q = p.par4[idx];
+      if (KIND != AB200_DEVICE_CONSTANT_STEP && KIND != AB200_DEVICE_EXP_STEP &&
+          KIND != AB200_DEVICE_PIECEWISE_STEP) {
+        e = p.par2[idx];
+      }
+      if (p.chop_x != nullptr) {
+        flip[t] = (p.chop_x[j] != 0) != (p.chop_d[i] != 0);
+      }
+    }
+    step[t].set(q, e);
+    w_in[t] = w[t];
+  }
+  for (int s0 = p.s_begin; s0 < p.s_end; s0 += UD_S) {
+    const int n_s = min(UD_S, p.s_end - s0);
+#pragma unroll 8
+    for (int r = tj; r < UD_S; r += UD_T) {
+      sd[r][ti] = (r < n_s && i_ok) ? __uint_as_float(p.dw[(long long)(s0 + r) * p.d_size + i]) : 0.0f;
+    }
+#pragma unroll
+    for (int e = threadIdx.x; e < UD_S * UJ; e += UD_I * UD_T) {
+      const int r = e / UJ, j = j0 + e % UJ;
+      sx[r][e % UJ] =
+          (r < n_s && j < p.x_size) ? __uint_as_float(p.xw[(long long)(s0 + r) * p.x_size + j]) : 0.0f;
+    }
+    __syncthreads();
+    for (int r = 0; r < n_s; r++) {
+      const float dv = sd[r][ti];
+      float c[EJ], n[EJ], most = 0.0f;
+#pragma unroll
+      for (int t = 0; t < EJ; t++) {
+        c[t] = __fmul_rn(dv, sx[r][tj * EJ + t]);
+        n[t] = fabsf(small ? __fadd_rn(__fadd_rn(c[t], 12582912.0f), -12582912.0f) : rintf(c[t]));
+        most = fmaxf(most, n[t]);
+      }
+      for (float k = 0.5f; __any_sync(0xffffffffu, most > k); k += 1.0f) {
+#pragma unroll
+        for (int t = 0; t < EJ; t++) {
+          // positive = decrease
+          const float w_new = step[t].apply(p, w[t], (c[t] > 0.0f) != flip[t], PulseStep<KIND>::kOnePlus ? 1.0f : 0.0f);
+          w[t] = n[t] > k ? w_new : w[t];
+        }
+      }
+    }
+    __syncthreads();
+  }
+#pragma unroll
+  for (int t = 0; t < EJ; t++) {
+    const int j = j0 + tj * EJ + t;
+    if (i_ok && j < p.x_size && w[t] != w_in[t]) {
+      p.w[(long long)j * p.d_size + i] = w[t];
+    }
+  }
+}
+
+template <int KIND> static void launchUpdateDense(const UpdateProblem &p, cudaStream_t stream) {
+  static int n_sm = 0; // SMs of the GPUs of this process (one kind per process)
+  if (n_sm == 0) {
+    int dev = 0;
+    AB200_CUDA(cudaGetDevice(&dev));
+    AB200_CUDA(cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev));
+  }
+  // four weights per thread where that still gives every SM a CTA, else one
+  const int gx = (p.d_size + UD_I - 1) / UD_I, gy4 = (p.x_size + 15) / 16, gy1 = (p.x_size + 3) / 4;
+  if ((long long)gx * gy4 >= n_sm) {
+    AB200_CUDA(launchChained(pulsedUpdateDenseKernel<KIND, 4>, dim3(gx, gy4), dim3(UD_I * UD_T), 0, stream, p));
+  } else {
+    AB200_CUDA(launchChained(pulsedUpdateDenseKernel<KIND, 1>, dim3(gx, gy1), dim3(UD_I * UD_T), 0, stream, p));
+  }
+}
+
 static int g_update_path = 0;
 void setUpdatePath(int mode) { g_update_path = mode; }
 
@@ -482,8 +587,10 @@ void launchPulsedUpdate(const UpdateProblem &p0, cudaStream_t stream) {
     launchUpdateInstance<KIND, IMPL, false>(p, grid, stream);                                      \
   }
 #define AB200_UPD(KIND)                                                                            \
-  if (implicit) {                                                                                  \
-    AB200_UPD2(KIND, true)                                                                         \
+  if (implicit && !noisy) {                                                                        \
+    launchUpdateDense<KIND>(p, stream);                                                            \
+  } else if (implicit) {                                                                           \
+    launchUpdateInstance<KIND, true, true>(p, grid, stream);                                       \
   } else {                                                                                         \
     AB200_UPD2(KIND, false)                                                                        \
   }
@@ -602,36 +709,124 @@ void launchCoincidences(const UpdateProblem &p, int32_t *counts_dx, cudaStream_t
 // Floating-point update W[x][d] -= lr * sum_s x[s][x] d[s][d] (RPUSimple::updateMatrix,
 // src/rpucuda/rpu.cpp:700-745), used by ideal devices / PulseType::None.
 // `overwrite`: the target receives -lr * sum alone (delta-weight mode: beta = 0, rpu.cpp:1509-1511)
-// CLIP_EACH: PulseType::NoneWithDevice - the rank-one update of every sample is followed by the
-// clip to the element's bounds (rpu_weight_updater.cpp:216-223), so the samples are applied to the
-// weight one after the other instead of being summed first.
-template <bool CLIP_EACH>
+//
+// T x T sums per thread, 16 x 16 threads; the samples come in steps through registers into one of two
+// buffers, so that the loads of a step are in flight while the one before is multiplied. Bound by the fp32
+// units; 64 x 16 sums per CTA with a barrier on each side of an unpipelined load took 194 us for 1024 x 1024 and
+// 512 samples, this takes 48. The sum of an element runs over the samples in order, as before.
+template <int T>
 __global__ void __launch_bounds__(256) fpUpdateKernel(UpdateProblem p, float lr_signed, int overwrite) {
+  pdlEnter();
+  constexpr int BN = 16 * T, BK = 64 / T; // lines and samples per step: four values per thread and operand
+  __shared__ __align__(16) float xs[2][BK][BN + 4], ds[2][BK][BN + 4];
+  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+  const int i0 = blockIdx.x * BN, j0 = blockIdx.y * BN;
+  const bool x_line = p.x_fs == 1 || p.x_ss != 1, d_line = p.d_fs == 1 || p.d_ss != 1;
+  float rx[4], rd[4], acc[T][T];
+#pragma unroll
+  for (int a = 0; a < T; a++) {
+#pragma unroll
+    for (int b = 0; b < T; b++) {
+      acc[a][b] = 0.0f;
+    }
+  }
+  // neighbouring threads take neighbouring lines, or samples where those are contiguous
+  auto load = [&](int s0) {
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+      const int e = tid + u * 256;
+      const int s = s0 + (x_line ? e / BN : e % BK), j = j0 + (x_line ? e % BN : e / BK);
+      rx[u] = 0.0f;
+      if (s < p.m && j < p.x_size) {
+        rx[u] = 1.0f; // the bias line
+        if (j < p.x_real) {
+          rx[u] = p.x[(long long)s * p.x_ss + (long long)j * p.x_fs];
+        }
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+      const int e = tid + u * 256;
+      const int s = s0 + (d_line ? e / BN : e % BK), i = i0 + (d_line ? e % BN : e / BK);
+      rd[u] = 0.0f;
+      if (s < p.m && i < p.d_size) {
+        rd[u] = p.d[(long long)s * p.d_ss + (long long)i * p.d_fs];
+      }
+    }
+  };
+  auto stage = [&](int buf) {
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+      const int e = tid + u * 256;
+      xs[buf][x_line ? e / BN : e % BK][x_line ? e % BN : e / BK] = rx[u];
+      ds[buf][d_line ? e / BN : e % BK][d_line ? e % BN : e / BK] = rd[u];
+    }
+  };
+  load(0);
+  stage(0);
+  __syncthreads();
+  for (int s0 = 0, buf = 0; s0 < p.m; s0 += BK, buf ^= 1) {
+    const bool more = s0 + BK < p.m;
+    if (more) {
+      load(s0 + BK);
+    }
+#pragma unroll
+    for (int s = 0; s < BK; s++) {
+      float a[T], b[T];
+      loadRow<T>(&xs[buf][s][ty * T], a);
+      loadRow<T>(&ds[buf][s][tx * T], b);
+#pragma unroll
+      for (int u = 0; u < T; u++) {
+#pragma unroll
+        for (int v = 0; v < T; v++) {
+          acc[u][v] = fmaf(a[u], b[v], acc[u][v]);
+        }
+      }
+    }
+    if (more) {
+      stage(buf ^ 1);
+    }
+    __syncthreads();
+  }
+#pragma unroll
+  for (int u = 0; u < T; u++) {
+#pragma unroll
+    for (int v = 0; v < T; v++) {
+      const int j = j0 + ty * T + u, i = i0 + tx * T + v;
+      if (j < p.x_size && i < p.d_size) {
+        const long long idx = (long long)j * p.d_size + i;
+        p.w[idx] = overwrite ? -lr_signed * acc[u][v] : p.w[idx] - lr_signed * acc[u][v];
+      }
+    }
+  }
+}
+
+// PulseType::NoneWithDevice: the rank-one update of every sample is followed by the clip to the
+// element's bounds (rpu_weight_updater.cpp:216-223), so the samples are applied to the weight one after the
+// other instead of being summed first.
+__global__ void __launch_bounds__(256) fpUpdateClipKernel(UpdateProblem p, float lr_signed) {
   pdlEnter();
   __shared__ float xs[16][16 + 1];
   __shared__ float ds[16][64 + 1];
   const int ti = threadIdx.x & 63, tj = threadIdx.x >> 6; // 64 d-lines x 4 groups of 4 x-lines
   const int i = blockIdx.x * 64 + ti;
   const int jb = blockIdx.y * 16;
-  float acc[4] = {0.f, 0.f, 0.f, 0.f};
   float wv[4] = {0.f, 0.f, 0.f, 0.f}, hi[4], lo[4];
-  if (CLIP_EACH) {
 #pragma unroll
-    for (int t = 0; t < 4; t++) {
-      const int j = jb + tj * 4 + t;
-      hi[t] = lo[t] = 0.0f;
-      if (i < p.d_size && j < p.x_size) {
-        const long long idx = (long long)j * p.d_size + i;
-        wv[t] = p.w[idx];
-        if (p.par4 != nullptr) {
-          const float4 q = p.par4[idx];
-          hi[t] = q.z;
-          lo[t] = q.w;
-        } else {
-          // no bounds: the digital accumulator of a mixed-precision compound
-          hi[t] = 3.4e38f;
-          lo[t] = -3.4e38f;
-        }
+  for (int t = 0; t < 4; t++) {
+    const int j = jb + tj * 4 + t;
+    hi[t] = lo[t] = 0.0f;
+    if (i < p.d_size && j < p.x_size) {
+      const long long idx = (long long)j * p.d_size + i;
+      wv[t] = p.w[idx];
+      if (p.par4 != nullptr) {
+        const float4 q = p.par4[idx];
+        hi[t] = q.z;
+        lo[t] = q.w;
+      } else {
+        // no bounds: the digital accumulator of a mixed-precision compound
+        hi[t] = 3.4e38f;
+        lo[t] = -3.4e38f;
       }
     }
   }
@@ -656,12 +851,8 @@ __global__ void __launch_bounds__(256) fpUpdateKernel(UpdateProblem p, float lr_
       float dv = ds[ss][ti];
 #pragma unroll
       for (int t = 0; t < 4; t++) {
-        if (CLIP_EACH) {
-          wv[t] = __fsub_rn(wv[t], __fmul_rn(__fmul_rn(lr_signed, dv), xs[ss][tj * 4 + t]));
-          wv[t] = fmaxf(fminf(wv[t], hi[t]), lo[t]);
-        } else {
-          acc[t] = fmaf(xs[ss][tj * 4 + t], dv, acc[t]);
-        }
+        wv[t] = __fsub_rn(wv[t], __fmul_rn(__fmul_rn(lr_signed, dv), xs[ss][tj * 4 + t]));
+        wv[t] = fmaxf(fminf(wv[t], hi[t]), lo[t]);
       }
     }
     __syncthreads();
@@ -671,12 +862,7 @@ __global__ void __launch_bounds__(256) fpUpdateKernel(UpdateProblem p, float lr_
     for (int t = 0; t < 4; t++) {
       int j = jb + tj * 4 + t;
       if (j < p.x_size) {
-        long long idx = (long long)j * p.d_size + i;
-        if (CLIP_EACH) {
-          p.w[idx] = wv[t];
-        } else {
-          p.w[idx] = overwrite ? -lr_signed * acc[t] : p.w[idx] - lr_signed * acc[t];
-        }
+        p.w[(long long)j * p.d_size + i] = wv[t];
       }
     }
   }
@@ -684,12 +870,28 @@ __global__ void __launch_bounds__(256) fpUpdateKernel(UpdateProblem p, float lr_
 
 void launchFPUpdate(const UpdateProblem &p, float lr_signed, cudaStream_t stream, bool overwrite,
                     bool clip_each) {
-  dim3 grid((p.d_size + 63) / 64, (p.x_size + 15) / 16);
   if (clip_each) {
-    AB200_CUDA(launchChained(fpUpdateKernel<true>, grid, dim3(256), 0, stream, p, lr_signed, 0));
+    dim3 grid((p.d_size + 63) / 64, (p.x_size + 15) / 16);
+    AB200_CUDA(launchChained(fpUpdateClipKernel, grid, dim3(256), 0, stream, p, lr_signed));
+    AB200_LAUNCH_CHECK();
+    return;
+  }
+  static int n_sm = 0; // SMs of the GPUs of this process (one kind per process)
+  if (n_sm == 0) {
+    int dev = 0;
+    AB200_CUDA(cudaGetDevice(&dev));
+    AB200_CUDA(cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev));
+  }
+  // the largest tile that still gives every SM a CTA (or, with many x-lines, fits the grid)
+  auto grid = [&](int t) { return dim3((p.d_size + 16 * t - 1) / (16 * t), (p.x_size + 16 * t - 1) / (16 * t)); };
+  auto fits = [&](int t) { return (long long)grid(t).x * grid(t).y >= n_sm; };
+  const int ow = overwrite ? 1 : 0;
+  if (fits(4) || p.x_size > 65535 * 16) {
+    AB200_CUDA(launchChained(fpUpdateKernel<4>, grid(4), dim3(256), 0, stream, p, lr_signed, ow));
+  } else if (fits(2)) {
+    AB200_CUDA(launchChained(fpUpdateKernel<2>, grid(2), dim3(256), 0, stream, p, lr_signed, ow));
   } else {
-    AB200_CUDA(launchChained(fpUpdateKernel<false>, grid, dim3(256), 0, stream, p, lr_signed,
-                             overwrite ? 1 : 0));
+    AB200_CUDA(launchChained(fpUpdateKernel<1>, grid(1), dim3(256), 0, stream, p, lr_signed, ow));
   }
   AB200_LAUNCH_CHECK();
 }

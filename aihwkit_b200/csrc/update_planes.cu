@@ -257,35 +257,6 @@ struct UpdatePlanesSmem {
   uint8_t counts[UP_WARPS][UP_EVENTS][32]; // pulses of the events that have more than one
 };
 
-// What a pulse needs of its element, by direction, with the sign of the direction in it: w += signed
-// step instead of w -= step (round-to-nearest is symmetric, so the bits are those of pulseOnce).
-template <int KIND> struct PulseStep {
-  float4 q;
-  float2 e;
-  float scale_dn, slope_dn;
-  __device__ __forceinline__ void set(const float4 &q_, const float2 &e_) {
-    q = q_;
-    e = e_;
-    scale_dn = -q.y;
-    slope_dn = -e.y;
-  }
-  // the noise of a pulse enters the rule as 1 + xi; kept in that form from the draw on
-  static constexpr bool kOnePlus =
-      KIND == AB200_DEVICE_CONSTANT_STEP || KIND == AB200_DEVICE_LINEAR_STEP;
-  __device__ __forceinline__ float apply(const UpdateProblem &p, float w, bool down, float xi) const {
-    if (KIND == AB200_DEVICE_CONSTANT_STEP) {
-      w = __fadd_rn(w, __fmul_rn(xi, down ? scale_dn : q.x));
-      return fmaxf(fminf(w, q.z), q.w);
-    } else if (KIND == AB200_DEVICE_LINEAR_STEP) {
-      const float sc = down ? scale_dn : q.x, sl = __fmul_rn(down ? slope_dn : e.x, w);
-      const float dw = p.mult_noise ? __fmul_rn(__fadd_rn(sl, sc), xi) : __fadd_rn(sl, __fmul_rn(sc, xi));
-      return fminf(fmaxf(__fadd_rn(w, dw), q.w), q.z);
-    } else {
-      return pulseOnce<KIND>(w, down, q, e, xi, p.mult_noise, p.es0, p.es1, p.pw, p.pw_n);
-    }
-  }
-};
-
 // Eight fresh Gaussians per lane for a warp's pool, as offset + std * z. Out of line: rare against the pulses
 // that take from the pool at two places, and the largest piece of code among them.
 __device__ __noinline__ void refillPool(PhiloxKey key, uint64_t pair, uint32_t call, float std, float offset,
