@@ -179,55 +179,94 @@ __global__ void __launch_bounds__(256) mvmSimtKernel(MvmProblem p) {
 
   // Operands of a step go through registers into one of two buffers: the loads of step k + 1 are in flight
   // while step k is multiplied, one barrier per step.
-  constexpr int NE = BM * BK / 256; // elements of each operand per thread (BM == BN)
+  constexpr int NE = 4; // elements of each operand per thread
+  static_assert(BM * BK == 256 * NE && BM == BN, "one group of four per thread and operand");
   const bool plain = !io.is_perfect && !inputIsRandom(io) && io.inp_asym == 1.0f;
   const float inv_res = __fdiv_rn(1.0f, io.res_in); // (read with res_in > 0 only)
+  // four neighbours in memory per thread, in one load where alignment and sizes allow
+  constexpr int AV = A_K_FAST ? BK / 4 : BM / 4, BV = B_N_FAST ? BN / 4 : BK / 4;
+  const int a_k = A_K_FAST ? (tid % AV) * 4 : tid / AV, a_r = A_K_FAST ? tid / AV : (tid % AV) * 4;
+  const int b_k = B_N_FAST ? tid / BV : (tid % BV) * 4, b_n = B_N_FAST ? (tid % BV) * 4 : tid / BV;
+  const long long a_ld = A_K_FAST ? p.in_ss : p.in_fs, b_ld = B_N_FAST ? p.wk : p.wn;
+  const bool a_vec = (A_K_FAST ? p.in_fs == 1 && (K & 3) == 0 : p.in_ss == 1 && (p.m & 3) == 0) &&
+                     p.in_real == K && (a_ld & 3) == 0 && (reinterpret_cast<uintptr_t>(p.in) & 15) == 0;
+  const bool b_vec = (B_N_FAST ? p.wn == 1 && (N & 3) == 0 : p.wk == 1 && (K & 3) == 0) && (b_ld & 3) == 0 &&
+                     (reinterpret_cast<uintptr_t>(p.w) & 15) == 0;
+  const float *a_src = p.in + (A_K_FAST ? (long long)(row0 + a_r) * a_ld + a_k : (long long)a_k * a_ld + row0 + a_r);
+  const float *b_src = p.w + (B_N_FAST ? (long long)b_k * b_ld + col0 + b_n : (long long)(col0 + b_n) * b_ld + b_k);
   float ra[NE], rb[NE];
   auto load = [&](int k0) {
+    if (a_vec) {
+      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (row0 + a_r < p.m && k0 + a_k < K) {
+        v = __ldg(reinterpret_cast<const float4 *>(a_src + (A_K_FAST ? (long long)k0 : k0 * a_ld)));
+      }
+      ra[0] = v.x;
+      ra[1] = v.y;
+      ra[2] = v.z;
+      ra[3] = v.w;
+    } else {
 #pragma unroll
-    for (int u = 0; u < NE; u++) {
-      const int e = tid + u * 256;
-      const int kk = A_K_FAST ? e % BK : e / BM, r = A_K_FAST ? e / BK : e % BM;
-      const int gr = row0 + r, gk = k0 + kk;
-      ra[u] = 0.0f;
-      if (gr < p.m && gk < K) {
-        ra[u] = 1.0f; // the bias line
-        if (gk < p.in_real) {
-          ra[u] = p.in[(long long)gr * p.in_ss + (long long)gk * p.in_fs];
+      for (int u = 0; u < NE; u++) {
+        const int gr = row0 + a_r + (A_K_FAST ? 0 : u), gk = k0 + a_k + (A_K_FAST ? u : 0);
+        ra[u] = 0.0f;
+        if (gr < p.m && gk < K) {
+          ra[u] = 1.0f; // the bias line
+          if (gk < p.in_real) {
+            ra[u] = p.in[(long long)gr * p.in_ss + (long long)gk * p.in_fs];
+          }
         }
       }
     }
+    if (b_vec) {
+      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (k0 + b_k < K && col0 + b_n < N) {
+        v = *reinterpret_cast<const float4 *>(b_src + (B_N_FAST ? k0 * b_ld : (long long)k0));
+      }
+      rb[0] = v.x;
+      rb[1] = v.y;
+      rb[2] = v.z;
+      rb[3] = v.w;
+    } else {
 #pragma unroll
-    for (int u = 0; u < NE; u++) {
-      const int e = tid + u * 256;
-      const int n = B_N_FAST ? e % BN : e / BK, kk = B_N_FAST ? e / BN : e % BK;
-      const int gk = k0 + kk, gn = col0 + n;
-      rb[u] = 0.0f;
-      if (gk < K && gn < N) {
-        rb[u] = p.w[(long long)gk * p.wk + (long long)gn * p.wn];
+      for (int u = 0; u < NE; u++) {
+        const int gk = k0 + b_k + (B_N_FAST ? 0 : u), gn = col0 + b_n + (B_N_FAST ? u : 0);
+        rb[u] = 0.0f;
+        if (gk < K && gn < N) {
+          rb[u] = p.w[(long long)gk * p.wk + (long long)gn * p.wn];
+        }
       }
     }
   };
   auto stage = [&](int buf, int k0) {
 #pragma unroll
     for (int u = 0; u < NE; u++) {
-      const int e = tid + u * 256;
-      const int kk = A_K_FAST ? e % BK : e / BM, r = A_K_FAST ? e / BK : e % BM;
-      const float sc = s_scale[r];
-      float v = 0.0f;
-      if (io.is_perfect) {
-        v = ra[u];
-      } else if (sc != 0.0f && k0 + kk < K) {
-        v = plain ? dacPlain(io, inv_res, ra[u], sc)
-                  : prepareInput(io, ra[u], sc, g, (uint32_t)(row0 + r), (uint32_t)(k0 + kk));
+      const int r = a_r + (A_K_FAST ? 0 : u), kk = a_k + (A_K_FAST ? u : 0);
+      if (!io.is_perfect) {
+        const float sc = s_scale[r];
+        float v = 0.0f;
+        if (sc != 0.0f && k0 + kk < K) {
+          v = plain ? dacPlain(io, inv_res, ra[u], sc)
+                    : prepareInput(io, ra[u], sc, g, (uint32_t)(row0 + r), (uint32_t)(k0 + kk));
+        }
+        ra[u] = v;
       }
-      As[buf][kk][r] = v;
     }
+    if (A_K_FAST) {
 #pragma unroll
-    for (int u = 0; u < NE; u++) {
-      const int e = tid + u * 256;
-      const int n = B_N_FAST ? e % BN : e / BK, kk = B_N_FAST ? e / BN : e % BK;
-      Bs[buf][kk][n] = rb[u];
+      for (int u = 0; u < NE; u++) {
+        As[buf][a_k + u][a_r] = ra[u];
+      }
+    } else {
+      *reinterpret_cast<float4 *>(&As[buf][a_k][a_r]) = make_float4(ra[0], ra[1], ra[2], ra[3]);
+    }
+    if (B_N_FAST) {
+      *reinterpret_cast<float4 *>(&Bs[buf][b_k][b_n]) = make_float4(rb[0], rb[1], rb[2], rb[3]);
+    } else {
+#pragma unroll
+      for (int u = 0; u < NE; u++) {
+        Bs[buf][b_k + u][b_n] = rb[u];
+      }
     }
   };
   load(0);
@@ -238,12 +277,22 @@ __global__ void __launch_bounds__(256) mvmSimtKernel(MvmProblem p) {
     if (more) {
       load(k0 + BK);
     }
+    float an[T], bn[T]; // operands of the next k, on their way from shared memory
+    loadRow<T>(&As[buf][0][ty * T], an);
+    loadRow<T>(&Bs[buf][0][tx * T], bn);
 #pragma unroll
     for (int kk = 0; kk < BK; kk++) {
       float a[T], b[T];
       const float posw = PCM ? irPosWeight(k0 + kk, K) : 0.0f;
-      loadRow<T>(&As[buf][kk][ty * T], a);
-      loadRow<T>(&Bs[buf][kk][tx * T], b);
+#pragma unroll
+      for (int i = 0; i < T; i++) {
+        a[i] = an[i];
+        b[i] = bn[i];
+      }
+      if (kk + 1 < BK) {
+        loadRow<T>(&As[buf][kk + 1][ty * T], an);
+        loadRow<T>(&Bs[buf][kk + 1][tx * T], bn);
+      }
 #pragma unroll
       for (int h = 0; h < S; h++) {
 #pragma unroll

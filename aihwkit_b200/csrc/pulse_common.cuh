@@ -233,15 +233,32 @@ __device__ __forceinline__ float pulseOnce(float w, bool down, const float4 &q, 
 
 // What a pulse needs of its element, by direction, with the sign of the direction in it: w += signed
 // step instead of w -= step (round-to-nearest is symmetric, so the bits are those of pulseOnce).
+//
+// SoftBoundsReference divides the weight by its bound in every pulse. Where the bounds are ordinary numbers the
+// quotient comes from their reciprocals, taken once, and two residual corrections q += (w - b q) y, which
+// give the correctly rounded quotient (Markstein, "Computation of elementary functions on the IBM RISC
+// System/6000 processor", 1990: y the rounded reciprocal; the first correction leaves q within an ulp, the second
+// rounds it correctly). Residuals below the normal range only occur for quotients that 1 - q does not see.
 template <int KIND> struct PulseStep {
   float4 q;
   float2 e;
   float scale_dn, slope_dn;
+  bool by_reciprocal = false; // the same for a whole warp
   __device__ __forceinline__ void set(const float4 &q_, const float2 &e_) {
     q = q_;
     e = e_;
     scale_dn = -q.y;
     slope_dn = -e.y;
+  }
+  // for all lanes of a warp together; `used` = the lane owns a weight
+  __device__ __forceinline__ void prepare(float w, bool used) {
+    if (KIND == AB200_DEVICE_SOFT_BOUNDS_REFERENCE) {
+      const float lo = 8.7e-19f, hi = 1.15e18f; // 2^-60, 2^60
+      by_reciprocal = __all_sync(0xffffffffu, !used || (q.z > lo && q.z < hi && q.w < -lo && q.w > -hi &&
+                                                        fabsf(w) < hi && fabsf(e.x) < hi));
+      e.y = __fdiv_rn(1.0f, q.z); // (the rule uses e.x alone)
+      slope_dn = __fdiv_rn(1.0f, q.w);
+    }
   }
   // the noise of a pulse enters the rule as 1 + xi; kept in that form from the draw on
   static constexpr bool kOnePlus =
@@ -254,6 +271,17 @@ template <int KIND> struct PulseStep {
       const float sc = down ? scale_dn : q.x, sl = __fmul_rn(down ? slope_dn : e.x, w);
       const float dw = p.mult_noise ? __fmul_rn(__fadd_rn(sl, sc), xi) : __fadd_rn(sl, __fmul_rn(sc, xi));
       return fminf(fmaxf(__fadd_rn(w, dw), q.w), q.z);
+    } else if (KIND == AB200_DEVICE_SOFT_BOUNDS_REFERENCE && by_reciprocal) {
+      const float bound = down ? q.w : q.z, y = down ? slope_dn : e.y, sc = down ? scale_dn : q.x;
+      w = __fadd_rn(w, e.x);
+      float a = __fmul_rn(w, y);
+      a = __fmaf_rn(__fmaf_rn(-bound, a, w), y, a);
+      a = __fmaf_rn(__fmaf_rn(-bound, a, w), y, a);
+      const float rest = __fsub_rn(1.0f, a);
+      const float dw = p.mult_noise ? __fmul_rn(__fmul_rn(sc, rest), __fadd_rn(1.0f, xi))
+                                    : __fmul_rn(sc, __fadd_rn(rest, xi));
+      w = fminf(fmaxf(__fadd_rn(w, dw), q.w), q.z);
+      return __fsub_rn(w, e.x);
     } else {
       return pulseOnce<KIND>(w, down, q, e, xi, p.mult_noise, p.es0, p.es1, p.pw, p.pw_n);
     }

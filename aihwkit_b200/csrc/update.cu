@@ -721,7 +721,6 @@ __global__ void __launch_bounds__(256) fpUpdateKernel(UpdateProblem p, float lr_
   __shared__ __align__(16) float xs[2][BK][BN + 4], ds[2][BK][BN + 4];
   const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
   const int i0 = blockIdx.x * BN, j0 = blockIdx.y * BN;
-  const bool x_line = p.x_fs == 1 || p.x_ss != 1, d_line = p.d_fs == 1 || p.d_ss != 1;
   float rx[4], rd[4], acc[T][T];
 #pragma unroll
   for (int a = 0; a < T; a++) {
@@ -730,37 +729,62 @@ __global__ void __launch_bounds__(256) fpUpdateKernel(UpdateProblem p, float lr_
       acc[a][b] = 0.0f;
     }
   }
-  // neighbouring threads take neighbouring lines, or samples where those are contiguous
-  auto load = [&](int s0) {
+  // four neighbouring lines of a sample per thread (or four samples of a line where those are contiguous),
+  // in one load where alignment and sizes allow
+  const bool x_line = p.x_fs == 1 || p.x_ss != 1, d_line = p.d_fs == 1 || p.d_ss != 1;
+  const int LV = BN / 4, SV = BK / 4;
+  const int x_s = x_line ? tid / LV : (tid % SV) * 4, x_j = x_line ? (tid % LV) * 4 : tid / SV;
+  const int d_s = d_line ? tid / LV : (tid % SV) * 4, d_i = d_line ? (tid % LV) * 4 : tid / SV;
+  auto vec = [&](const float *v, long long fs, long long ss, bool line, int lines, int real) {
+    return (line ? fs == 1 && (ss & 3) == 0 && (lines & 3) == 0 : ss == 1 && (fs & 3) == 0 && (p.m & 3) == 0) &&
+           real == lines && (reinterpret_cast<uintptr_t>(v) & 15) == 0;
+  };
+  const bool x_vec = vec(p.x, p.x_fs, p.x_ss, x_line, p.x_size, p.x_real);
+  const bool d_vec = vec(p.d, p.d_fs, p.d_ss, d_line, p.d_size, p.d_size);
+  const float *x_src = p.x + (long long)x_s * p.x_ss + (long long)(j0 + x_j) * p.x_fs;
+  const float *d_src = p.d + (long long)d_s * p.d_ss + (long long)(i0 + d_i) * p.d_fs;
+  auto load4 = [&](float *r, bool v4, const float *src, long long ss, long long fs, bool line, int s, int l, int lines,
+                   int real) {
+    if (v4) {
+      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (s < p.m && l < lines) {
+        v = __ldg(reinterpret_cast<const float4 *>(src));
+      }
+      r[0] = v.x;
+      r[1] = v.y;
+      r[2] = v.z;
+      r[3] = v.w;
+    } else {
 #pragma unroll
-    for (int u = 0; u < 4; u++) {
-      const int e = tid + u * 256;
-      const int s = s0 + (x_line ? e / BN : e % BK), j = j0 + (x_line ? e % BN : e / BK);
-      rx[u] = 0.0f;
-      if (s < p.m && j < p.x_size) {
-        rx[u] = 1.0f; // the bias line
-        if (j < p.x_real) {
-          rx[u] = p.x[(long long)s * p.x_ss + (long long)j * p.x_fs];
+      for (int u = 0; u < 4; u++) {
+        const int gs = s + (line ? 0 : u), gl = l + (line ? u : 0);
+        r[u] = 0.0f;
+        if (gs < p.m && gl < lines) {
+          r[u] = 1.0f; // the bias line
+          if (gl < real) {
+            r[u] = src[line ? u * fs : u * ss];
+          }
         }
       }
     }
+  };
+  auto load = [&](int s0) {
+    load4(rx, x_vec, x_src + s0 * p.x_ss, p.x_ss, p.x_fs, x_line, s0 + x_s, j0 + x_j, p.x_size, p.x_real);
+    load4(rd, d_vec, d_src + s0 * p.d_ss, p.d_ss, p.d_fs, d_line, s0 + d_s, i0 + d_i, p.d_size, p.d_size);
+  };
+  auto stage4 = [&](float (*dst)[BN + 4], const float *r, bool line, int s, int l) {
+    if (line) {
+      *reinterpret_cast<float4 *>(&dst[s][l]) = make_float4(r[0], r[1], r[2], r[3]);
+    } else {
 #pragma unroll
-    for (int u = 0; u < 4; u++) {
-      const int e = tid + u * 256;
-      const int s = s0 + (d_line ? e / BN : e % BK), i = i0 + (d_line ? e % BN : e / BK);
-      rd[u] = 0.0f;
-      if (s < p.m && i < p.d_size) {
-        rd[u] = p.d[(long long)s * p.d_ss + (long long)i * p.d_fs];
+      for (int u = 0; u < 4; u++) {
+        dst[s + u][l] = r[u];
       }
     }
   };
   auto stage = [&](int buf) {
-#pragma unroll
-    for (int u = 0; u < 4; u++) {
-      const int e = tid + u * 256;
-      xs[buf][x_line ? e / BN : e % BK][x_line ? e % BN : e / BK] = rx[u];
-      ds[buf][d_line ? e / BN : e % BK][d_line ? e % BN : e / BK] = rd[u];
-    }
+    stage4(xs[buf], rx, x_line, x_s, x_j);
+    stage4(ds[buf], rd, d_line, d_s, d_i);
   };
   load(0);
   stage(0);
@@ -770,11 +794,21 @@ __global__ void __launch_bounds__(256) fpUpdateKernel(UpdateProblem p, float lr_
     if (more) {
       load(s0 + BK);
     }
+    float an[T], bn[T]; // operands of the next sample, on their way from shared memory
+    loadRow<T>(&xs[buf][0][ty * T], an);
+    loadRow<T>(&ds[buf][0][tx * T], bn);
 #pragma unroll
     for (int s = 0; s < BK; s++) {
       float a[T], b[T];
-      loadRow<T>(&xs[buf][s][ty * T], a);
-      loadRow<T>(&ds[buf][s][tx * T], b);
+#pragma unroll
+      for (int u = 0; u < T; u++) {
+        a[u] = an[u];
+        b[u] = bn[u];
+      }
+      if (s + 1 < BK) {
+        loadRow<T>(&xs[buf][s + 1][ty * T], an);
+        loadRow<T>(&ds[buf][s + 1][tx * T], bn);
+      }
 #pragma unroll
       for (int u = 0; u < T; u++) {
 #pragma unroll

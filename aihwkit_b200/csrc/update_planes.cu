@@ -310,6 +310,7 @@ __global__ void __launch_bounds__(32 * UP_WARPS, 8) pulsedUpdatePlanesKernel(Upd
       }
     }
     step.set(q, e);
+    step.prepare(w, i_ok);
   }
   const float w_in = w;
   const float std = p.dw_min_std;
@@ -383,6 +384,14 @@ __global__ void __launch_bounds__(32 * UP_WARPS, 8) pulsedUpdatePlanesKernel(Upd
   uint32_t group = 0; // group in which a lane has passed the mark
 
   auto push = [&](uint32_t ev, uint32_t dir) {
+    // (most words hold no more than a few events: the first three without a branch)
+#pragma unroll
+    for (int u = 0; u < 3; u++) {
+      const uint32_t rest = ev & (ev - 1u);
+      const uint32_t next = queue * 2u + ((dir & (ev ^ rest)) != 0u ? 1u : 0u);
+      queue = ev != 0u ? next : queue;
+      ev = rest;
+    }
     while (ev != 0u) {
       const uint32_t rest = ev & (ev - 1u);
       queue = queue * 2u + ((dir & (ev ^ rest)) != 0u ? 1u : 0u);
