@@ -129,29 +129,38 @@ __global__ void nmAverageKernel(float *sval, int m, float decay, float *state) {
 // norm of each half, and the epilogue runs the analog chain of the line once per half before it
 // adds them in front of (pos_neg = 1) or behind (pos_neg = 2) the output stage
 // (computeAnalogMV, rpu_forward_backward_pass.cpp:820-876).
+// Groups of 256 threads that share the outputs of a CTA, each with every other step along K: the 64 x 64
+// tile leaves an SM one CTA in mid-sized problems, and eight warps do not hide the latency of shared
+// memory (fp32 pipe 26 % active).
+__host__ __device__ constexpr int simtGroups(int T) { return T == 4 ? 2 : 1; }
+
 template <bool A_K_FAST, bool B_N_FAST, int T, bool PCM, bool PN = false>
-__global__ void __launch_bounds__(256) mvmSimtKernel(MvmProblem p) {
+__global__ void __launch_bounds__(256 * simtGroups(T)) mvmSimtKernel(MvmProblem p) {
   static_assert(!PN || PCM, "separate passes use the line-chain variant");
   constexpr int S = PN ? 2 : 1; // accumulator sets: [negative inputs, positive inputs] or one
   pdlEnter();
   constexpr int BM = 16 * T, BN = 16 * T;
   constexpr int BK = T == 1 ? 64 : (T == 2 ? 32 : 16);
-  __shared__ __align__(16) float As[2][BK][BM + 4];
-  __shared__ __align__(16) float Bs[2][BK][BN + 4];
+  constexpr int G = simtGroups(T);
+  __shared__ __align__(16) float As_all[G][2][BK][BM + 4];
+  __shared__ __align__(16) float Bs_all[G][2][BK][BN + 4];
+  const int grp = G == 1 ? 0 : threadIdx.x >> 8;
+  float(*const As)[BK][BM + 4] = As_all[grp];
+  float(*const Bs)[BK][BN + 4] = Bs_all[grp];
   __shared__ float s_scale[BM];
   const IOEff &io = p.io;
-  const int tid = threadIdx.x;
+  const int tid = threadIdx.x & 255;
   const int tx = tid & 15, ty = tid >> 4;
   const int row0 = blockIdx.y * BM, col0 = blockIdx.x * BN;
   const int K = p.in_size, N = p.out_size;
   const ElemRng g{p.key, p.call, (p.backward ? TAG_BWD_IN : TAG_FWD_IN) + p.noise_id};
 
-  if (tid < BM) {
+  if (threadIdx.x < BM) {
     int r = row0 + tid;
     // (perfect IO has no per-row values: no noise-management pass ran)
     s_scale[tid] = io.is_perfect ? 1.0f : (r < p.m ? p.scale[r] : 0.0f);
   }
-  if (io.is_perfect && blockIdx.x == 0 && blockIdx.y == 0 && tid == 0 && !p.backward && p.bm_stats) {
+  if (io.is_perfect && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0 && !p.backward && p.bm_stats) {
     p.bm_stats[0] = 0;
     p.bm_stats[1] = 0;
   }
@@ -269,13 +278,15 @@ __global__ void __launch_bounds__(256) mvmSimtKernel(MvmProblem p) {
       }
     }
   };
-  load(0);
-  stage(0, 0);
+  // (all groups take the same number of steps; past the end the operands are zeros)
+  load(grp * BK);
+  stage(0, grp * BK);
   __syncthreads();
-  for (int k0 = 0, buf = 0; k0 < K; k0 += BK, buf ^= 1) {
-    const bool more = k0 + BK < K;
+  for (int kb = 0, buf = 0; kb < K; kb += G * BK, buf ^= 1) {
+    const int k0 = kb + grp * BK;
+    const bool more = kb + G * BK < K;
     if (more) {
-      load(k0 + BK);
+      load(k0 + G * BK);
     }
     float an[T], bn[T]; // operands of the next k, on their way from shared memory
     loadRow<T>(&As[buf][0][ty * T], an);
@@ -316,9 +327,34 @@ __global__ void __launch_bounds__(256) mvmSimtKernel(MvmProblem p) {
       }
     }
     if (more) {
-      stage(buf ^ 1, k0 + BK);
+      stage(buf ^ 1, k0 + G * BK);
     }
     __syncthreads();
+  }
+  if (G > 1) {
+    // the second group hands its sums over and is done
+    static_assert(G == 1 || (!PCM && sizeof(As_all) >= sizeof(float) * BM * BN), "room for the sums");
+    float *const sums = &As_all[0][0][0][0];
+    if (grp == 1) {
+#pragma unroll
+      for (int i = 0; i < T; i++) {
+#pragma unroll
+        for (int j = 0; j < T; j++) {
+          sums[(i * T + j) * 256 + tid] = acc[0][i][j];
+        }
+      }
+    }
+    __syncthreads();
+    if (grp == 1) {
+      return;
+    }
+#pragma unroll
+    for (int i = 0; i < T; i++) {
+#pragma unroll
+      for (int j = 0; j < T; j++) {
+        acc[0][i][j] += sums[(i * T + j) * 256 + tid];
+      }
+    }
   }
 
   // noise blocks of four columns, an even number per row (two blocks share one Philox call); a
@@ -726,13 +762,13 @@ void launchMvmSimt(const MvmProblem &p, cudaStream_t stream) {
   {                                                                                                \
     dim3 grid((p.out_size + 16 * TT - 1) / (16 * TT), (p.m + 16 * TT - 1) / (16 * TT));           \
     if (a_k_fast && b_n_fast) {                                                                    \
-      AB200_CUDA(launchChained(mvmSimtKernel<true, true, TT, PCM>, grid, dim3(256), 0, stream, p));                             \
+      AB200_CUDA(launchChained(mvmSimtKernel<true, true, TT, PCM>, grid, dim3(256 * simtGroups(TT)), 0, stream, p));                \
     } else if (a_k_fast) {                                                                         \
-      AB200_CUDA(launchChained(mvmSimtKernel<true, false, TT, PCM>, grid, dim3(256), 0, stream, p));                            \
+      AB200_CUDA(launchChained(mvmSimtKernel<true, false, TT, PCM>, grid, dim3(256 * simtGroups(TT)), 0, stream, p));                            \
     } else if (b_n_fast) {                                                                         \
-      AB200_CUDA(launchChained(mvmSimtKernel<false, true, TT, PCM>, grid, dim3(256), 0, stream, p));                            \
+      AB200_CUDA(launchChained(mvmSimtKernel<false, true, TT, PCM>, grid, dim3(256 * simtGroups(TT)), 0, stream, p));                            \
     } else {                                                                                       \
-      AB200_CUDA(launchChained(mvmSimtKernel<false, false, TT, PCM>, grid, dim3(256), 0, stream, p));                           \
+      AB200_CUDA(launchChained(mvmSimtKernel<false, false, TT, PCM>, grid, dim3(256 * simtGroups(TT)), 0, stream, p));                           \
     }                                                                                              \
   }
   if (pcm && p.io.pos_neg != 0) {

@@ -640,8 +640,6 @@ Tile::~Tile() {
     cudaFree(drift_w0_);
     cudaFree(drift_t_);
     cudaFree(drift_nu_);
-    cudaFree(plane_bl_);
-    cudaFree(plane_nk_);
     cudaFree(plane_ab_);
     cudaFree(chop_in_);
     cudaFree(chop_out_);
@@ -947,8 +945,6 @@ void Tile::ensureScratch(int m) {
   cudaFree(flags_);
   cudaFree(xw_);
   cudaFree(dw_);
-  cudaFree(plane_bl_);
-  cudaFree(plane_nk_);
   cudaFree(plane_ab_);
   plane_bl_ = plane_nk_ = nullptr;
   plane_ab_ = nullptr;
@@ -965,9 +961,9 @@ void Tile::ensureScratch(int m) {
   if (cfg_.device_kind != AB200_DEVICE_IDEAL && up_.pulse_type != AB200_PULSE_NONE) {
     AB200_CUDA(cudaMalloc(&xw_, (size_t)cap * x_size_ * sizeof(uint32_t)));
     AB200_CUDA(cudaMalloc(&dw_, (size_t)cap * d_size_ * sizeof(uint32_t)));
-    AB200_CUDA(cudaMalloc(&plane_bl_, (size_t)cap * sizeof(int)));
-    AB200_CUDA(cudaMalloc(&plane_nk_, (size_t)(cap / 32 + 1) * sizeof(int)));
-    AB200_CUDA(cudaMalloc(&plane_ab_, (size_t)cap * sizeof(float2)));
+    AB200_CUDA(cudaMalloc(&plane_ab_, (size_t)cap * (sizeof(float2) + sizeof(int)) + (size_t)(cap / 32 + 1) * sizeof(int)));
+    plane_bl_ = reinterpret_cast<int *>(plane_ab_ + cap);
+    plane_nk_ = plane_bl_ + cap;
   }
   scratch_m_ = cap;
 }

@@ -713,13 +713,23 @@ void launchCoincidences(const UpdateProblem &p, int32_t *counts_dx, cudaStream_t
 // T x T sums per thread, 16 x 16 threads; the samples come in steps through registers into one of two
 // buffers, so that the loads of a step are in flight while the one before is multiplied. Bound by the fp32
 // units; 64 x 16 sums per CTA with a barrier on each side of an unpipelined load took 194 us for 1024 x 1024 and
-// 512 samples, this takes 48. The sum of an element runs over the samples in order, as before.
+// 512 samples, this takes 41.
+//
+// With 64 x 64 sums per CTA two groups of 256 threads share them, each with every other step, and add up at the
+// end: one group's eight warps do not hide the latency of shared memory.
+__host__ __device__ constexpr int fpUpdateGroups(int T) { return T == 4 ? 2 : 1; }
+
 template <int T>
-__global__ void __launch_bounds__(256) fpUpdateKernel(UpdateProblem p, float lr_signed, int overwrite) {
+__global__ void __launch_bounds__(256 * fpUpdateGroups(T))
+    fpUpdateKernel(UpdateProblem p, float lr_signed, int overwrite) {
   pdlEnter();
   constexpr int BN = 16 * T, BK = 64 / T; // lines and samples per step: four values per thread and operand
-  __shared__ __align__(16) float xs[2][BK][BN + 4], ds[2][BK][BN + 4];
-  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+  constexpr int G = fpUpdateGroups(T);
+  __shared__ __align__(16) float xs_all[G][2][BK][BN + 4], ds_all[G][2][BK][BN + 4];
+  const int grp = G == 1 ? 0 : threadIdx.x >> 8;
+  float(*const xs)[BK][BN + 4] = xs_all[grp];
+  float(*const ds)[BK][BN + 4] = ds_all[grp];
+  const int tid = threadIdx.x & 255, tx = tid & 15, ty = tid >> 4;
   const int i0 = blockIdx.x * BN, j0 = blockIdx.y * BN;
   float rx[4], rd[4], acc[T][T];
 #pragma unroll
@@ -786,13 +796,14 @@ __global__ void __launch_bounds__(256) fpUpdateKernel(UpdateProblem p, float lr_
     stage4(xs[buf], rx, x_line, x_s, x_j);
     stage4(ds[buf], rd, d_line, d_s, d_i);
   };
-  load(0);
+  // (both groups take the same number of steps; past the end the operands are zeros)
+  load(grp * BK);
   stage(0);
   __syncthreads();
-  for (int s0 = 0, buf = 0; s0 < p.m; s0 += BK, buf ^= 1) {
-    const bool more = s0 + BK < p.m;
+  for (int sb = 0, buf = 0; sb < p.m; sb += G * BK, buf ^= 1) {
+    const bool more = sb + G * BK < p.m;
     if (more) {
-      load(s0 + BK);
+      load(sb + (G + grp) * BK);
     }
     float an[T], bn[T]; // operands of the next sample, on their way from shared memory
     loadRow<T>(&xs[buf][0][ty * T], an);
@@ -821,6 +832,30 @@ __global__ void __launch_bounds__(256) fpUpdateKernel(UpdateProblem p, float lr_
       stage(buf ^ 1);
     }
     __syncthreads();
+  }
+  if (G > 1) {
+    static_assert(G == 1 || sizeof(xs_all) >= sizeof(float) * BN * BN, "room for the sums");
+    float *const sums = &xs_all[0][0][0][0];
+    if (grp == 1) {
+#pragma unroll
+      for (int u = 0; u < T; u++) {
+#pragma unroll
+        for (int v = 0; v < T; v++) {
+          sums[(u * T + v) * 256 + tid] = acc[u][v];
+        }
+      }
+    }
+    __syncthreads();
+    if (grp == 1) {
+      return;
+    }
+#pragma unroll
+    for (int u = 0; u < T; u++) {
+#pragma unroll
+      for (int v = 0; v < T; v++) {
+        acc[u][v] += sums[(u * T + v) * 256 + tid];
+      }
+    }
   }
 #pragma unroll
   for (int u = 0; u < T; u++) {
@@ -921,7 +956,7 @@ void launchFPUpdate(const UpdateProblem &p, float lr_signed, cudaStream_t stream
   auto fits = [&](int t) { return (long long)grid(t).x * grid(t).y >= n_sm; };
   const int ow = overwrite ? 1 : 0;
   if (fits(4) || p.x_size > 65535 * 16) {
-    AB200_CUDA(launchChained(fpUpdateKernel<4>, grid(4), dim3(256), 0, stream, p, lr_signed, ow));
+    AB200_CUDA(launchChained(fpUpdateKernel<4>, grid(4), dim3(256 * fpUpdateGroups(4)), 0, stream, p, lr_signed, ow));
   } else if (fits(2)) {
     AB200_CUDA(launchChained(fpUpdateKernel<2>, grid(2), dim3(256), 0, stream, p, lr_signed, ow));
   } else {
