@@ -595,7 +595,7 @@ __global__ void __launch_bounds__(BM_THREADS) bmRerunKernel(MvmProblem p, int n_
           const int k1 = min(K, (sl + 1) * k_slice);
           const float *wp = p.w + (long long)(n < N ? n : 0) * p.wn;
           float a = 0.0f;
-#pragma unroll 16
+#pragma unroll 32
           for (int k = sl * k_slice; k < k1; k++) {
             a = fmaf(v_sh[k], wp[(long long)k * p.wk], a);
           }
@@ -636,7 +636,7 @@ __global__ void __launch_bounds__(BM_THREADS) bmRerunKernel(MvmProblem p, int n_
             acc[0] += part_sh[sl * N + n];
           }
         } else {
-#pragma unroll 8
+#pragma unroll 32
           for (int k = 0; k < K; k++) {
             acc[0] = fmaf(v_sh[k], wp[(long long)k * p.wk], acc[0]);
           }

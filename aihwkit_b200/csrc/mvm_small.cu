@@ -24,9 +24,9 @@ constexpr int SM_WARPS = 16;
 constexpr int SM_K = 512;            // features per step: 32 per warp at most
 constexpr int SM_KW = SM_K / SM_WARPS;
 
-template <int ROWS, bool K_FAST>
-__global__ void __launch_bounds__(32 * SM_WARPS) mvmSmallKernel(MvmProblem p,
-                                                                const __grid_constant__ SmallSplits sp) {
+template <int ROWS, bool K_FAST, typename Splits>
+__global__ void __launch_bounds__(32 * SM_WARPS) mvmSmallKernel(const __grid_constant__ MvmProblem p,
+                                                                const __grid_constant__ Splits sp) {
   // prepared inputs of a step, later the partial sums of the warps
   __shared__ __align__(16) float buf[ROWS * SM_K > SM_WARPS * ROWS * 32 ? ROWS * SM_K : SM_WARPS * ROWS * 32];
   const IOEff &io = p.io;
@@ -320,32 +320,37 @@ bool smallMvmIo(const IOEff &io) {
   return !running && !ioNeedsLineChain(io) && !ioLineSigma(io);
 }
 
-int smallMvmMaxCtas(int in_size) {
-  // Four rounds of one CTA per SM; with more, the 64 x 64 tiles of the general kernel fill the GPU as well and
-  // load less per product. 2048 x 2048, forward, this kernel against the general one: 16 rows (64 CTAs) 28
-  // against 91 us, 64 rows (256) 56 against 179; 4096 x 4096, 32 rows (256) 109 against 367.
-  // Short rows leave most of a CTA's 512 features empty: 64 x 64, 4000 rows (500 CTAs) 22.6 against 17.9 us, but
-  // 128 x 128, 1000 rows (252) 13.3 against 15.4.
+static int smCount() {
   static int n_sm = 0; // SMs of the GPUs of this process (one kind per process)
   if (n_sm == 0) {
     int dev = 0;
     AB200_CUDA(cudaGetDevice(&dev));
     AB200_CUDA(cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev));
   }
-  return (in_size > 128 ? 4 : 2) * n_sm;
+  return n_sm;
 }
 
-template <int ROWS> static void launchRows(const MvmProblem &p, const SmallSplits &sp, bool k_fast, cudaStream_t stream) {
+int smallMvmMaxCtas(int in_size) {
+  // Four rounds of one CTA per SM; with more, the 64 x 64 tiles of the general kernel fill the GPU as well and
+  // load less per product. 2048 x 2048, forward, this kernel against the general one: 16 rows (64 CTAs) 28
+  // against 91 us, 64 rows (256) 56 against 179; 4096 x 4096, 32 rows (256) 109 against 367.
+  // Short rows leave most of a CTA's 512 features empty: 64 x 64, 4000 rows (500 CTAs) 22.6 against 17.9 us, but
+  // 128 x 128, 1000 rows (252) 13.3 against 15.4.
+  return (in_size > 128 ? 4 : 2) * smCount();
+}
+
+template <int ROWS, typename Splits>
+static void launchRows(const MvmProblem &p, const Splits &sp, bool k_fast, cudaStream_t stream) {
   dim3 grid(sp.col_blk[sp.n_out], (p.m + ROWS - 1) / ROWS);
   if (k_fast) {
-    AB200_CUDA(launchChained(mvmSmallKernel<ROWS, true>, grid, dim3(32 * SM_WARPS), 0, stream, p, sp));
+    AB200_CUDA(launchChained(mvmSmallKernel<ROWS, true, Splits>, grid, dim3(32 * SM_WARPS), 0, stream, p, sp));
   } else {
-    AB200_CUDA(launchChained(mvmSmallKernel<ROWS, false>, grid, dim3(32 * SM_WARPS), 0, stream, p, sp));
+    AB200_CUDA(launchChained(mvmSmallKernel<ROWS, false, Splits>, grid, dim3(32 * SM_WARPS), 0, stream, p, sp));
   }
   AB200_LAUNCH_CHECK();
 }
 
-void launchMvmSmall(const MvmProblem &p, SmallSplits &sp, cudaStream_t stream) {
+template <typename Splits> static void launchSplits(const MvmProblem &p, Splits &sp, cudaStream_t stream) {
   const bool k_fast = p.wn != 1;
   sp.vec = 1;
   for (int i = 0; i < sp.n_in; i++) {
@@ -367,6 +372,8 @@ void launchMvmSmall(const MvmProblem &p, SmallSplits &sp, cudaStream_t stream) {
   }
 }
 
+void launchMvmSmall(const MvmProblem &p, SmallSplits &sp, cudaStream_t stream) { launchSplits(p, sp, stream); }
+
 bool smallMvmEligible(const MvmProblem &p) {
   if (p.in_fs != 1 || (p.wk != 1 && p.wn != 1) || p.out_noise_vals != nullptr || p.gather.idx != nullptr ||
       !smallMvmIo(p.io)) {
@@ -375,13 +382,18 @@ bool smallMvmEligible(const MvmProblem &p) {
   return (long long)((p.out_size + 31) / 32) * ((p.m + 15) / 16) <= smallMvmMaxCtas(p.in_size);
 }
 
+bool smallMvmOneRound(const MvmProblem &p) {
+  return smallMvmEligible(p) && p.in_size <= 2 * SM_K &&
+         (long long)((p.out_size + 31) / 32) * ((p.m + 15) / 16) <= smCount();
+}
+
 void launchMvmSmallTile(const MvmProblem &p, cudaStream_t stream) {
-  SmallSplits sp{};
+  SmallSplitsT<1, 1> sp{};
   sp.n_in = sp.n_out = 1;
   sp.in_size[0] = p.in_size;
   sp.out_size[0] = p.out_size;
   sp.tile[0] = SmallTile{p.w, p.wn != 1 ? p.wn : p.wk, p.alpha, p.call, p.noise_id, p.key};
-  launchMvmSmall(p, sp, stream);
+  launchSplits(p, sp, stream);
 }
 
 } // namespace ab200

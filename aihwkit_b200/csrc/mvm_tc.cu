@@ -356,7 +356,6 @@ template <bool BM, bool PAIR, bool CODES = false, bool LINE = false>
 __global__ void __launch_bounds__(TC_THREADS, 1)
     mvmTcKernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_bhi,
                 const __grid_constant__ CUtensorMap tm_blo, const TcKernelParams p) {
-  pdlEnter();
   constexpr int STAGES = PAIR ? TC2_STAGES : TC_STAGES;
   constexpr int STAGE_BYTES = PAIR ? TC2_STAGE_BYTES : TC_STAGE_BYTES;
   constexpr int KCH = PAIR ? TC2_KCH : TC_KCH;
@@ -432,6 +431,9 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
   }
   tcFenceAfter();
   const uint32_t tmem_base = *tmem_slot;
+  // barriers, TMEM and the pair are set up while the kernel before this one ends; up to here nothing has
+  // touched global memory
+  pdlEnter();
 
   if (warp == TC_WARP_TMA) {
     // ------------------------------ TMA producer ------------------------------

@@ -1510,7 +1510,10 @@ bool Tile::tcEligible(const MvmProblem &p) const {
   if (mode >= 2) {
     return true;
   }
-  return p.m >= 128 && (double)p.m * p.in_size * p.out_size >= 16777216.0;
+  // A problem that the small-batch kernel serves with one CTA per SM at the most and in two steps along K takes
+  // it 8 to 18 us; operand split, DAC and tensor-core kernel do not come below 16 to 23 (512 x 512, 128 rows:
+  // 9.5 against 18.1; 1024 x 1024, 64 rows: 16.3 against 21.4).
+  return p.m >= 128 && (double)p.m * p.in_size * p.out_size >= 16777216.0 && !smallMvmOneRound(p);
 }
 
 void Tile::runTc(const MvmProblem &p, cudaStream_t s) {

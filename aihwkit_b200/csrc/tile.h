@@ -149,18 +149,21 @@ struct SmallTile {
   PhiloxKey key;
 };
 constexpr int kSmallSplits = 32, kSmallTiles = 72; // per launch
-struct SmallSplits {
+// N in- / out-splits, NT tiles: a single tile passes a few hundred bytes of parameters, a layer 3 KB
+template <int N, int NT> struct SmallSplitsT {
   int n_in, n_out;
-  int in_off[kSmallSplits], in_size[kSmallSplits];
-  int out_off[kSmallSplits], out_size[kSmallSplits];
-  int col_blk[kSmallSplits + 1]; // first column block of every out-split (set by the launch)
-  int vec;                       // weights may be read in fours along k (set by the launch)
-  const float *bias;             // added once per output column, or null
-  SmallTile tile[kSmallTiles];   // [in-split][out-split]
+  int in_off[N], in_size[N];
+  int out_off[N], out_size[N];
+  int col_blk[N + 1]; // first column block of every out-split (set by the launch)
+  int vec;            // weights may be read in fours along k (set by the launch)
+  const float *bias;  // added once per output column, or null
+  SmallTile tile[NT]; // [in-split][out-split]
 };
+using SmallSplits = SmallSplitsT<kSmallSplits, kSmallTiles>;
 bool smallMvmIo(const IOEff &io); // IO settings these kernels implement
 int smallMvmMaxCtas(int in_size); // column blocks of 32 times row blocks of 16 up to which they are used
 bool smallMvmEligible(const MvmProblem &p);
+bool smallMvmOneRound(const MvmProblem &p); // eligible, one CTA per SM at the most, two steps along K at the most
 void launchMvmSmall(const MvmProblem &p, SmallSplits &sp, cudaStream_t stream);
 void launchMvmSmallTile(const MvmProblem &p, cudaStream_t stream);
 
