@@ -80,8 +80,23 @@ __global__ void __launch_bounds__(256)
   if (e < csr_elems) {
     const float *c = cols + n * per_image;
     const int t1 = csr_off[e + 1];
-    for (int t = csr_off[e]; t < t1; t++) {
-      acc += c[csr_pos[t]];
+    // nine positions name an element of a 3 x 3 convolution: their loads in flight together, the sum in order
+    constexpr int kU = 9;
+    for (int t = csr_off[e]; t < t1; t += kU) {
+      int at[kU];
+      float v[kU];
+#pragma unroll
+      for (int u = 0; u < kU; u++) {
+        at[u] = t + u < t1 ? __ldg(csr_pos + t + u) : -1;
+      }
+#pragma unroll
+      for (int u = 0; u < kU; u++) {
+        v[u] = at[u] >= 0 ? c[at[u]] : 0.0f;
+      }
+#pragma unroll
+      for (int u = 0; u < kU; u++) {
+        acc += v[u];
+      }
     }
   }
   out[n * out_mat + e] = acc;

@@ -979,6 +979,40 @@ __device__ __forceinline__ float dacCode(const DacParams &p, float x, float scal
   }
   return fminf(fmaxf(code, -p.code_bound), p.code_bound);
 }
+// Four codes as bf16 and their squares added to `acc`: rounded by adding 1.5 * 2^23 (the codes of this path
+// are below 2^8; what is larger is clipped), one test for ties and one branch for the four. Instructions
+// bound these kernels: 27 per element with a branch each and rint on the conversion pipe, DACINSTR now.
+__device__ __forceinline__ uint2 dacFour(const DacParams &p, const float4 &x, float scale, float &acc) {
+  const float kMagic = 12582912.0f;
+  const float in[4] = {x.x, x.y, x.z, x.w};
+  float c[4], off = 0.0f;
+#pragma unroll
+  for (int u = 0; u < 4; u++) {
+    const float q = __fmul_rn(__fmul_rn(in[u], scale), p.inv_res_in);
+    c[u] = __fadd_rn(__fadd_rn(q, kMagic), -kMagic);
+    off = fmaxf(off, fabsf(__fsub_rn(q, c[u])));
+    c[u] = fminf(fmaxf(c[u], -p.code_bound), p.code_bound);
+  }
+  if (off > 0.4999f) {
+#pragma unroll 1
+    for (int u = 0; u < 4; u++) {
+      const float e = dacCode(p, u == 0 ? x.x : (u == 1 ? x.y : (u == 2 ? x.z : x.w)), scale);
+      c[0] = u == 0 ? e : c[0];
+      c[1] = u == 1 ? e : c[1];
+      c[2] = u == 2 ? e : c[2];
+      c[3] = u == 3 ? e : c[3];
+    }
+  }
+#pragma unroll
+  for (int u = 0; u < 4; u++) {
+    acc = fmaf(c[u], c[u], acc);
+  }
+  const __nv_bfloat162 lo = __floats2bfloat162_rn(c[0], c[1]), hi = __floats2bfloat162_rn(c[2], c[3]);
+  uint2 pk;
+  pk.x = *reinterpret_cast<const uint32_t *>(&lo);
+  pk.y = *reinterpret_cast<const uint32_t *>(&hi);
+  return pk;
+}
 __device__ __forceinline__ void dacRowScalars(const DacParams &p, int i, int row, float sval, float scale,
                                               float sumsq) {
   const long long si = (long long)i * p.m + row;
@@ -1091,22 +1125,11 @@ __device__ __forceinline__ void dacQuantRows(const DacParams &p, int i0, int row
     for (int j = 0; j < 4; j++) {
       const int k = 4 * (lane + 32 * j);
       if (k < p.kpad) {
-        float c0 = 0.0f, c1 = 0.0f, c2 = 0.0f, c3 = 0.0f;
+        uint2 pk = make_uint2(0u, 0u);
         if (k < is.z && scale[n] != 0.0f) {
-          c0 = dacCode(p, r[n].v[j].x, scale[n]);
-          c1 = dacCode(p, r[n].v[j].y, scale[n]);
-          c2 = dacCode(p, r[n].v[j].z, scale[n]);
-          c3 = dacCode(p, r[n].v[j].w, scale[n]);
+          pk = dacFour(p, r[n].v[j], scale[n], acc[n]);
         }
-        const __nv_bfloat162 lo = __floats2bfloat162_rn(c0, c1), hi = __floats2bfloat162_rn(c2, c3);
-        uint2 pk;
-        pk.x = *reinterpret_cast<const uint32_t *>(&lo);
-        pk.y = *reinterpret_cast<const uint32_t *>(&hi);
         *reinterpret_cast<uint2 *>(c + k) = pk;
-        acc[n] = fmaf(c0, c0, acc[n]);
-        acc[n] = fmaf(c1, c1, acc[n]);
-        acc[n] = fmaf(c2, c2, acc[n]);
-        acc[n] = fmaf(c3, c3, acc[n]);
       }
     }
   }
@@ -1187,23 +1210,11 @@ __global__ void __launch_bounds__(256) dacQuantizeLongRowKernel(DacParams p) {
   const int KP4 = p.kpad >> 2;
 #pragma unroll 2
   for (int k = lane; k < KP4; k += 32) {
-    float c0 = 0.0f, c1 = 0.0f, c2 = 0.0f, c3 = 0.0f;
+    uint2 pk = make_uint2(0u, 0u);
     if (k < K4 && scale != 0.0f) {
-      const float4 v = __ldg(x + k);
-      c0 = dacCode(p, v.x, scale);
-      c1 = dacCode(p, v.y, scale);
-      c2 = dacCode(p, v.z, scale);
-      c3 = dacCode(p, v.w, scale);
+      pk = dacFour(p, __ldg(x + k), scale, acc);
     }
-    const __nv_bfloat162 lo = __floats2bfloat162_rn(c0, c1), hi = __floats2bfloat162_rn(c2, c3);
-    uint2 pk;
-    pk.x = *reinterpret_cast<const uint32_t *>(&lo);
-    pk.y = *reinterpret_cast<const uint32_t *>(&hi);
     *reinterpret_cast<uint2 *>(c + 4 * k) = pk;
-    acc = fmaf(c0, c0, acc);
-    acc = fmaf(c1, c1, acc);
-    acc = fmaf(c2, c2, acc);
-    acc = fmaf(c3, c3, acc);
   }
   for (int o = 16; o > 0; o >>= 1) {
     acc += __shfl_xor_sync(0xffffffffu, acc, o);
@@ -1276,23 +1287,11 @@ __global__ void __launch_bounds__(kGatherWarps * 32) dacQuantizeGatherKernel(Dac
   const float4 *sh4 = reinterpret_cast<const float4 *>(sh);
 #pragma unroll 2
   for (int k = lane; k < KP4; k += 32) {
-    float c0 = 0.0f, c1 = 0.0f, c2 = 0.0f, c3 = 0.0f;
+    uint2 pk = make_uint2(0u, 0u);
     if (scale != 0.0f) {
-      const float4 v = sh4[k]; // zero beyond K: code 0
-      c0 = dacCode(p, v.x, scale);
-      c1 = dacCode(p, v.y, scale);
-      c2 = dacCode(p, v.z, scale);
-      c3 = dacCode(p, v.w, scale);
+      pk = dacFour(p, sh4[k], scale, acc); // zero beyond K: code 0
     }
-    const __nv_bfloat162 lo = __floats2bfloat162_rn(c0, c1), hi = __floats2bfloat162_rn(c2, c3);
-    uint2 pk;
-    pk.x = *reinterpret_cast<const uint32_t *>(&lo);
-    pk.y = *reinterpret_cast<const uint32_t *>(&hi);
     *reinterpret_cast<uint2 *>(c + 4 * k) = pk;
-    acc = fmaf(c0, c0, acc);
-    acc = fmaf(c1, c1, acc);
-    acc = fmaf(c2, c2, acc);
-    acc = fmaf(c3, c3, acc);
   }
   for (int o = 16; o > 0; o >>= 1) {
     acc += __shfl_xor_sync(0xffffffffu, acc, o);
