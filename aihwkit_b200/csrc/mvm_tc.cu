@@ -981,7 +981,8 @@ __device__ __forceinline__ float dacCode(const DacParams &p, float x, float scal
 }
 // Four codes as bf16 and their squares added to `acc`: rounded by adding 1.5 * 2^23 (the codes of this path
 // are below 2^8; what is larger is clipped), one test for ties and one branch for the four. Instructions
-// bound these kernels: 27 per element with a branch each and rint on the conversion pipe, DACINSTR now.
+// bound these kernels: 27 per element with a branch each and rint on the conversion pipe, 12 now. (Loading the next pair of in-splits
+// ahead in dacQuantizeRowKernel, at 95 registers: 41.9 -> 48.8 us.)
 __device__ __forceinline__ uint2 dacFour(const DacParams &p, const float4 &x, float scale, float &acc) {
   const float kMagic = 12582912.0f;
   const float in[4] = {x.x, x.y, x.z, x.w};

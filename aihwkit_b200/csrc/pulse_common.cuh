@@ -264,12 +264,15 @@ template <int KIND> struct PulseStep {
   static constexpr bool kOnePlus =
       KIND == AB200_DEVICE_CONSTANT_STEP || KIND == AB200_DEVICE_LINEAR_STEP;
   __device__ __forceinline__ float apply(const UpdateProblem &p, float w, bool down, float xi) const {
+    return apply(p, w, down, xi, p.mult_noise != 0);
+  }
+  __device__ __forceinline__ float apply(const UpdateProblem &p, float w, bool down, float xi, bool mult) const {
     if (KIND == AB200_DEVICE_CONSTANT_STEP) {
       w = __fadd_rn(w, __fmul_rn(xi, down ? scale_dn : q.x));
       return fmaxf(fminf(w, q.z), q.w);
     } else if (KIND == AB200_DEVICE_LINEAR_STEP) {
       const float sc = down ? scale_dn : q.x, sl = __fmul_rn(down ? slope_dn : e.x, w);
-      const float dw = p.mult_noise ? __fmul_rn(__fadd_rn(sl, sc), xi) : __fadd_rn(sl, __fmul_rn(sc, xi));
+      const float dw = mult ? __fmul_rn(__fadd_rn(sl, sc), xi) : __fadd_rn(sl, __fmul_rn(sc, xi));
       return fminf(fmaxf(__fadd_rn(w, dw), q.w), q.z);
     } else if (KIND == AB200_DEVICE_SOFT_BOUNDS_REFERENCE && by_reciprocal) {
       const float bound = down ? q.w : q.z, y = down ? slope_dn : e.y, sc = down ? scale_dn : q.x;
@@ -278,8 +281,7 @@ template <int KIND> struct PulseStep {
       a = __fmaf_rn(__fmaf_rn(-bound, a, w), y, a);
       a = __fmaf_rn(__fmaf_rn(-bound, a, w), y, a);
       const float rest = __fsub_rn(1.0f, a);
-      const float dw = p.mult_noise ? __fmul_rn(__fmul_rn(sc, rest), __fadd_rn(1.0f, xi))
-                                    : __fmul_rn(sc, __fadd_rn(rest, xi));
+      const float dw = mult ? __fmul_rn(__fmul_rn(sc, rest), __fadd_rn(1.0f, xi)) : __fmul_rn(sc, __fadd_rn(rest, xi));
       w = fminf(fmaxf(__fadd_rn(w, dw), q.w), q.z);
       return __fsub_rn(w, e.x);
     } else {

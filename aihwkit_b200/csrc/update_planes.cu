@@ -281,7 +281,7 @@ __device__ __noinline__ void refillPool(PhiloxKey key, uint64_t pair, uint32_t c
 // refill; the busiest lane sets the number of rounds, 0.66 of the lanes have an event in one. A list of
 // {coincidences, directions} words in shared memory instead of the queue of bits took 7 % fewer instructions
 // and the same time (24 instead of 32 warps per SM).
-template <int KIND, bool NOISY>
+template <int KIND, bool NOISY, bool MULT>
 __global__ void __launch_bounds__(32 * UP_WARPS, 8) pulsedUpdatePlanesKernel(UpdateProblem p) {
   pdlEnter();
   __shared__ UpdatePlanesSmem sm;
@@ -323,7 +323,9 @@ __global__ void __launch_bounds__(32 * UP_WARPS, 8) pulsedUpdatePlanesKernel(Upd
   uint8_t *const counts = &sm.counts[warp][0][lane];
   int cnt = 0;        // events in the queue
   uint32_t queue = 0; // their directions, the newest in bit 0
-  uint32_t multi = 0; // events (by ordinal) of more than one pulse
+  uint32_t multi = 0; // events (by ordinal) of more than one pulse,
+  uint32_t triple = 0; // and of three (where trains are longer, the counts are in shared memory)
+  const bool deep = *p.plane_max > 3; // some train has more slots than the first four planes hold
   int pool_pos = UP_POOL; // empty
   uint32_t refills = 0;
   const uint32_t lt_mask = (1u << lane) - 1u;
@@ -346,7 +348,7 @@ __global__ void __launch_bounds__(32 * UP_WARPS, 8) pulsedUpdatePlanesKernel(Upd
       xi = pool[pool_pos + __popc(takers & lt_mask)];
       pool_pos += n_take;
     }
-    const float w_new = step.apply(p, w, down, xi);
+    const float w_new = step.apply(p, w, down, xi, MULT);
     w = act ? w_new : w;
   };
 
@@ -359,7 +361,10 @@ __global__ void __launch_bounds__(32 * UP_WARPS, 8) pulsedUpdatePlanesKernel(Upd
       queue <<= 1;
       pulse(r < cnt, down);
       if ((multi_any & 1u) != 0u) {
-        const int n = ((multi >> r) & 1u) != 0u ? counts[r * 32] : 0;
+        int n = 0;
+        if (((multi >> r) & 1u) != 0u) {
+          n = deep ? counts[r * 32] : 2 + (int)((triple >> r) & 1u);
+        }
         for (int k = 1; __any_sync(0xffffffffu, k < n); k++) {
           pulse(k < n, down);
         }
@@ -368,14 +373,13 @@ __global__ void __launch_bounds__(32 * UP_WARPS, 8) pulsedUpdatePlanesKernel(Upd
     }
     cnt = 0;
     queue = 0u;
-    multi = 0u;
+    multi = triple = 0u;
   };
 
   const int b_first = p.s_begin >> 5, b_last = (p.s_end - 1) >> 5;
   const uint4 *xb = reinterpret_cast<const uint4 *>(p.xw) + (long long)b_first * 8 * p.x_size + j;
   const uint4 *db = reinterpret_cast<const uint4 *>(p.dw) + (long long)b_first * 8 * p.d_size + (i_ok ? i : 0);
   const long long x_step = 8LL * p.x_size, d_step = 8LL * p.d_size;
-  const bool deep = *p.plane_max > 3; // some train has more slots than the first four planes hold
   // rows of the first / last block outside of [s_begin, s_end)
   const uint32_t rows_first = 0xffffffffu << (p.s_begin & 31);
   const uint32_t rows_last = 0xffffffffu >> (31 - ((p.s_end - 1) & 31));
@@ -398,8 +402,18 @@ __global__ void __launch_bounds__(32 * UP_WARPS, 8) pulsedUpdatePlanesKernel(Upd
       ev = rest;
     }
   };
-  auto pushCounts = [&](uint32_t more, uint32_t ev, int before, uint32_t c0, uint32_t c1, uint32_t c2,
-                        uint32_t c3, uint32_t c4) {
+  // the events of more than one pulse among `ev`, which start at ordinal `before`; c0..c4 the bits of the counts
+  auto pushCounts = [&](uint32_t more, uint32_t ev, int before, uint32_t c0) {
+    while (more != 0u) {
+      const uint32_t bit = more & (0u - more);
+      more ^= bit;
+      const uint32_t at = 1u << (before + __popc(ev & (bit - 1u)));
+      multi |= at;
+      triple |= (c0 & bit) != 0u ? at : 0u;
+    }
+  };
+  auto pushDeepCounts = [&](uint32_t more, uint32_t ev, int before, uint32_t c0, uint32_t c1, uint32_t c2,
+                            uint32_t c3, uint32_t c4) {
     while (more != 0u) {
       const uint32_t bit = more & (0u - more);
       more ^= bit;
@@ -426,8 +440,8 @@ __global__ void __launch_bounds__(32 * UP_WARPS, 8) pulsedUpdatePlanesKernel(Upd
       push(any1, x1.x ^ d1.x ^ flip);
       const uint32_t m0 = (p0 & p1) | (p0 & p2) | (p1 & p2), m1 = (q0 & q1) | (q0 & q2) | (q1 & q2);
       if (((m0 | m1) & lane_on) != 0u) {
-        pushCounts(m0 & lane_on, any0, cnt, p0 ^ p1 ^ p2, m0, 0u, 0u, 0u);
-        pushCounts(m1 & lane_on, any1, cnt + n0, q0 ^ q1 ^ q2, m1, 0u, 0u, 0u);
+        pushCounts(m0 & lane_on, any0, cnt, p0 ^ p1 ^ p2);
+        pushCounts(m1 & lane_on, any1, cnt + n0, q0 ^ q1 ^ q2);
       }
       cnt += n0 + n1;
       rank0 += (uint32_t)(__popc(x0.y | x0.z | x0.w) + __popc(x1.y | x1.z | x1.w));
@@ -505,7 +519,11 @@ __global__ void __launch_bounds__(32 * UP_WARPS, 8) pulsedUpdatePlanesKernel(Upd
       }
       if (ev != 0u) {
         push(ev, dir);
-        pushCounts(ev & (c1 | c2 | c3 | c4), ev, cnt, c0, c1, c2, c3, c4);
+        if (deep) {
+          pushDeepCounts(ev & (c1 | c2 | c3 | c4), ev, cnt, c0, c1, c2, c3, c4);
+        } else {
+          pushCounts(ev & c1, ev, cnt, c0);
+        }
         cnt += __popc(ev);
       }
       if (!full && !end) {
@@ -530,19 +548,28 @@ __global__ void __launch_bounds__(32 * UP_WARPS, 8) pulsedUpdatePlanesKernel(Upd
   }
 }
 
-template <int KIND, bool NOISY>
+template <int KIND, bool NOISY, bool MULT>
 static void launchPlanesInstance(const UpdateProblem &p, cudaStream_t stream) {
   const long long blocks =
       (long long)((p.d_size + 31) / 32) * ((p.x_size + UP_WARPS - 1) / UP_WARPS);
-  AB200_CUDA(launchChained(pulsedUpdatePlanesKernel<KIND, NOISY>, dim3((unsigned)blocks), dim3(32 * UP_WARPS),
+  AB200_CUDA(launchChained(pulsedUpdatePlanesKernel<KIND, NOISY, MULT>, dim3((unsigned)blocks), dim3(32 * UP_WARPS),
                            0, stream, p));
 }
 
 template <int KIND> static void launchPlanesKind(const UpdateProblem &p, cudaStream_t stream) {
+  // (the two rules that have it multiply the noise with the step or add it)
+  constexpr bool can_mult = KIND == AB200_DEVICE_LINEAR_STEP || KIND == AB200_DEVICE_SOFT_BOUNDS_REFERENCE;
+  const bool mult = can_mult && p.mult_noise != 0;
   if (p.dw_min_std > 0.0f) {
-    launchPlanesInstance<KIND, true>(p, stream);
+    if (mult) {
+      launchPlanesInstance<KIND, true, can_mult>(p, stream);
+    } else {
+      launchPlanesInstance<KIND, true, false>(p, stream);
+    }
+  } else if (mult) {
+    launchPlanesInstance<KIND, false, can_mult>(p, stream);
   } else {
-    launchPlanesInstance<KIND, false>(p, stream);
+    launchPlanesInstance<KIND, false, false>(p, stream);
   }
 }
 
