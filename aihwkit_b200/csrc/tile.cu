@@ -1755,13 +1755,13 @@ void Tile::update(const float *x, const float *d, bool bias, int m, bool x_trans
 }
 
 // used by the mapped array: update from sub-blocks of wider activation / gradient matrices
-void Tile::updateStrided(const float *x, long long x_ss, const float *d, long long d_ss, int m,
-                         cudaStream_t s) {
-  updateCore(x, x_ss, 1, x_size_, d, d_ss, 1, m, s);
+void Tile::updateStrided(const float *x, long long x_ss, const float *d, long long d_ss, int m, cudaStream_t s,
+                         std::vector<UpdateProblem> *collect) {
+  updateCore(x, x_ss, 1, x_size_, d, d_ss, 1, m, s, collect);
 }
 
-void Tile::updateCore(const float *x, long long x_ss, long long x_fs, int x_in, const float *d,
-                      long long d_ss, long long d_fs, int m, cudaStream_t s) {
+void Tile::updateCore(const float *x, long long x_ss, long long x_fs, int x_in, const float *d, long long d_ss,
+                      long long d_fs, int m, cudaStream_t s, std::vector<UpdateProblem> *collect) {
   requireDevice("update");
   if (m <= 0 || lr_ == 0.0f) {
     return; // "if (!learning_rate) return" (rpu_weight_updater.cpp:206-208)
@@ -1849,6 +1849,11 @@ void Tile::updateCore(const float *x, long long x_ss, long long x_fs, int x_in, 
   u.plane_nk = plane_nk_ ? plane_nk_ + 1 : nullptr; // the first word holds the longest of all
   u.plane_max = plane_nk_;
   const bool planes = streamUpdateEligible(u);
+  if (collect && planes && !pulses_up_ && cfg_.device_kind != AB200_DEVICE_TRANSFER) {
+    u.w = w_;
+    collect->push_back(u);
+    return;
+  }
   if (!planes || pulses_up_) {
     launchPulsePrepare(u, s);
   }

@@ -250,6 +250,10 @@ bool streamUpdateEligible(const UpdateProblem &p);
 void setUpdatePath(int mode);
 void launchPulsePlanes(const UpdateProblem &p, cudaStream_t stream);
 void launchPulsedUpdatePlanes(const UpdateProblem &p, cudaStream_t stream);
+// the whole update of the tiles of a mapped layer (one batch size, one kind of device), up to
+// kUpdateBatch of them per launch
+constexpr int kUpdateBatch = 8;
+void launchPulsedUpdateTiles(const UpdateProblem *p, int n, cudaStream_t stream);
 void launchPulsedUpdate(const UpdateProblem &p, cudaStream_t stream);
 void launchCoincidences(const UpdateProblem &p, int32_t *counts_dx, cudaStream_t stream);
 // pulses of the samples [s_begin, s_end) of a prepared batch, added per weight to `up` (the weight
@@ -396,8 +400,9 @@ public:
 
   void backwardStrided(const float *d, long long d_ss, float *x, long long x_ss, int m,
                        bool accumulate, uint32_t noise_id, float out_scale, cudaStream_t s);
-  void updateStrided(const float *x, long long x_ss, const float *d, long long d_ss, int m,
-                     cudaStream_t s);
+  // (`collect`: an update that several tiles can share a launch for is appended there instead of being run)
+  void updateStrided(const float *x, long long x_ss, const float *d, long long d_ss, int m, cudaStream_t s,
+                     std::vector<UpdateProblem> *collect = nullptr);
 
   const IOEff &fio() const { return f_io_; }
   float *weightsXD() { return w_; }
@@ -421,8 +426,8 @@ private:
   void backwardCore(const float *d, long long d_ss, long long d_fs, float *x, long long x_ss,
                     long long x_fs, int x_store, int m, bool accumulate, uint32_t noise_id,
                     float out_scale, cudaStream_t s, int out_t_rows = 0);
-  void updateCore(const float *x, long long x_ss, long long x_fs, int x_in, const float *d,
-                  long long d_ss, long long d_fs, int m, cudaStream_t s);
+  void updateCore(const float *x, long long x_ss, long long x_fs, int x_in, const float *d, long long d_ss,
+                  long long d_fs, int m, cudaStream_t s, std::vector<UpdateProblem> *collect = nullptr);
   void requireSingleDevice(const char *what);
   void ensurePar3(DeviceStore &ds);
   int opTargets(float *w[2], DeviceStore *ds[2]);

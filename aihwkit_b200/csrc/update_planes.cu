@@ -19,7 +19,16 @@
 // with 256 rows 407 -> 257 us.
 #include "pulse_common.cuh"
 
+#include <algorithm>
+
 namespace ab200 {
+
+// The problems of one launch: a tile, or tiles of a mapped layer along the last grid dimension. Grids are those
+// of the largest tile.
+template <int N> struct UpdateBatch {
+  UpdateProblem tile[N];
+};
+#define AB200_BATCH_TILE(z) batch.tile[N == 1 ? 0 : (z)]
 
 // ---------------------------------------------------------------------------------------------
 // update management per sample
@@ -36,7 +45,9 @@ __device__ __forceinline__ void storeSampleParams(const UpdateProblem &p, int s,
 }
 
 // plain rows (any strides) and rows gathered through a row-major index array: one CTA per sample
-__global__ void __launch_bounds__(128) pulseStatsKernel(UpdateProblem p) {
+template <int N>
+__global__ void __launch_bounds__(128) pulseStatsKernel(const __grid_constant__ UpdateBatch<N> batch) {
+  const UpdateProblem &p = AB200_BATCH_TILE(blockIdx.y);
   pdlEnter();
   __shared__ float sh[4];
   const int s = blockIdx.x;
@@ -122,14 +133,20 @@ constexpr int PP_LINES = 64; // lines per CTA, eight per warp
 // Lane = row: a ballot then yields one plane word of one line. The values are staged through shared
 // memory where the rows are contiguous along the lines, and read directly where they are contiguous
 // along the rows (transposed inputs, index arrays [x_size][m_batch]).
-__global__ void __launch_bounds__(256) pulsePlanesKernel(UpdateProblem p, int n_xchunk) {
+template <int N>
+__global__ void __launch_bounds__(256) pulsePlanesKernel(const __grid_constant__ UpdateBatch<N> batch) {
+  const UpdateProblem &p = AB200_BATCH_TILE(blockIdx.y);
   pdlEnter();
   __shared__ float tile[PP_LINES][33];
   __shared__ uint32_t planes[32][PP_LINES + 1];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int nseg = p.nseg > 0 ? p.nseg : 1;
+  const int n_xchunk = (p.x_size + PP_LINES - 1) / PP_LINES;
   const int n_chunk = n_xchunk + (p.d_size + PP_LINES - 1) / PP_LINES;
-  const int blk = blockIdx.x / n_chunk, chunk = blockIdx.x - blk * n_chunk;
+  const int blk = (int)(blockIdx.x / (unsigned)n_chunk), chunk = (int)(blockIdx.x - (unsigned)blk * n_chunk);
+  if (N > 1 && blk * 32 >= p.m * nseg) {
+    return;
+  }
   const bool is_x = chunk < n_xchunk;
   const int line0 = (is_x ? chunk : chunk - n_xchunk) * PP_LINES;
   const int n_lines = is_x ? p.x_size : p.d_size;
@@ -281,8 +298,10 @@ __device__ __noinline__ void refillPool(PhiloxKey key, uint64_t pair, uint32_t c
 // refill; the busiest lane sets the number of rounds, 0.66 of the lanes have an event in one. A list of
 // {coincidences, directions} words in shared memory instead of the queue of bits took 7 % fewer instructions
 // and the same time (24 instead of 32 warps per SM).
-template <int KIND, bool NOISY, bool MULT>
-__global__ void __launch_bounds__(32 * UP_WARPS, 8) pulsedUpdatePlanesKernel(UpdateProblem p) {
+template <int KIND, bool NOISY, bool MULT, int N>
+__global__ void __launch_bounds__(32 * UP_WARPS, 8)
+    pulsedUpdatePlanesKernel(const __grid_constant__ UpdateBatch<N> batch) {
+  const UpdateProblem &p = AB200_BATCH_TILE(blockIdx.y);
   pdlEnter();
   __shared__ UpdatePlanesSmem sm;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -426,8 +445,9 @@ __global__ void __launch_bounds__(32 * UP_WARPS, 8) pulsedUpdatePlanesKernel(Upd
 
   int b = b_first;
   while (true) {
-    // Two inner blocks at a time as long as no lane fills up in them and no train is longer than three slots.
-    while (!deep && b > b_first && b + 1 < b_last) {
+    // Two inner blocks at a time as long as no lane fills up in them and no train of theirs is longer than
+    // three slots.
+    while (b > b_first && b + 1 < b_last && (!deep || (p.plane_nk[b] <= 3 && p.plane_nk[b + 1] <= 3))) {
       const uint4 x0 = xb[0], x1 = xb[x_step], d0 = db[0], d1 = db[d_step];
       const uint32_t p0 = x0.y & d0.y, p1 = x0.z & d0.z, p2 = x0.w & d0.w;
       const uint32_t q0 = x1.y & d1.y, q1 = x1.z & d1.z, q2 = x1.w & d1.w;
@@ -440,8 +460,13 @@ __global__ void __launch_bounds__(32 * UP_WARPS, 8) pulsedUpdatePlanesKernel(Upd
       push(any1, x1.x ^ d1.x ^ flip);
       const uint32_t m0 = (p0 & p1) | (p0 & p2) | (p1 & p2), m1 = (q0 & q1) | (q0 & q2) | (q1 & q2);
       if (((m0 | m1) & lane_on) != 0u) {
-        pushCounts(m0 & lane_on, any0, cnt, p0 ^ p1 ^ p2);
-        pushCounts(m1 & lane_on, any1, cnt + n0, q0 ^ q1 ^ q2);
+        if (deep) {
+          pushDeepCounts(m0 & lane_on, any0, cnt, p0 ^ p1 ^ p2, m0, 0u, 0u, 0u);
+          pushDeepCounts(m1 & lane_on, any1, cnt + n0, q0 ^ q1 ^ q2, m1, 0u, 0u, 0u);
+        } else {
+          pushCounts(m0 & lane_on, any0, cnt, p0 ^ p1 ^ p2);
+          pushCounts(m1 & lane_on, any1, cnt + n0, q0 ^ q1 ^ q2);
+        }
       }
       cnt += n0 + n1;
       rank0 += (uint32_t)(__popc(x0.y | x0.z | x0.w) + __popc(x1.y | x1.z | x1.w));
@@ -548,74 +573,107 @@ __global__ void __launch_bounds__(32 * UP_WARPS, 8) pulsedUpdatePlanesKernel(Upd
   }
 }
 
-template <int KIND, bool NOISY, bool MULT>
-static void launchPlanesInstance(const UpdateProblem &p, cudaStream_t stream) {
-  const long long blocks =
-      (long long)((p.d_size + 31) / 32) * ((p.x_size + UP_WARPS - 1) / UP_WARPS);
-  AB200_CUDA(launchChained(pulsedUpdatePlanesKernel<KIND, NOISY, MULT>, dim3((unsigned)blocks), dim3(32 * UP_WARPS),
-                           0, stream, p));
+template <int KIND, bool NOISY, bool MULT, int N>
+static void launchPlanesInstance(const UpdateBatch<N> &batch, int n, cudaStream_t stream) {
+  long long blocks = 0;
+  for (int k = 0; k < n; k++) {
+    const UpdateProblem &p = batch.tile[k];
+    blocks = std::max(blocks, (long long)((p.d_size + 31) / 32) * ((p.x_size + UP_WARPS - 1) / UP_WARPS));
+  }
+  AB200_CUDA(launchChained(pulsedUpdatePlanesKernel<KIND, NOISY, MULT, N>, dim3((unsigned)blocks, n),
+                           dim3(32 * UP_WARPS), 0, stream, batch));
 }
 
-template <int KIND> static void launchPlanesKind(const UpdateProblem &p, cudaStream_t stream) {
+template <int KIND, int N> static void launchPlanesKind(const UpdateBatch<N> &batch, int n, cudaStream_t stream) {
+  const UpdateProblem &p = batch.tile[0];
   // (the two rules that have it multiply the noise with the step or add it)
   constexpr bool can_mult = KIND == AB200_DEVICE_LINEAR_STEP || KIND == AB200_DEVICE_SOFT_BOUNDS_REFERENCE;
   const bool mult = can_mult && p.mult_noise != 0;
   if (p.dw_min_std > 0.0f) {
     if (mult) {
-      launchPlanesInstance<KIND, true, can_mult>(p, stream);
+      launchPlanesInstance<KIND, true, can_mult>(batch, n, stream);
     } else {
-      launchPlanesInstance<KIND, true, false>(p, stream);
+      launchPlanesInstance<KIND, true, false>(batch, n, stream);
     }
   } else if (mult) {
-    launchPlanesInstance<KIND, false, can_mult>(p, stream);
+    launchPlanesInstance<KIND, false, can_mult>(batch, n, stream);
   } else {
-    launchPlanesInstance<KIND, false, false>(p, stream);
+    launchPlanesInstance<KIND, false, false>(batch, n, stream);
   }
 }
 
-void launchPulsePlanes(const UpdateProblem &p, cudaStream_t stream) {
-  if (p.gather.idx != nullptr && p.gather.idx_t != nullptr) {
-    AB200_CUDA(launchChained(pulseStatsGatherKernel, dim3((p.m + 31) / 32), dim3(1024), 0, stream, p));
+template <int N> static void launchPlanesOf(const UpdateBatch<N> &batch, int n, cudaStream_t stream) {
+  const UpdateProblem &p0 = batch.tile[0];
+  if (p0.gather.idx != nullptr && p0.gather.idx_t != nullptr) {
+    AB200_CUDA(launchChained(pulseStatsGatherKernel, dim3((p0.m + 31) / 32), dim3(1024), 0, stream, p0));
   } else {
-    AB200_CUDA(launchChained(pulseStatsKernel, dim3(p.m), dim3(128), 0, stream, p));
+    AB200_CUDA(launchChained(pulseStatsKernel<N>, dim3(p0.m, n), dim3(128), 0, stream, batch));
   }
   AB200_LAUNCH_CHECK();
-  const int n_blk = (p.m * (p.nseg > 0 ? p.nseg : 1) + 31) / 32;
-  const int n_x = (p.x_size + PP_LINES - 1) / PP_LINES, n_d = (p.d_size + PP_LINES - 1) / PP_LINES;
-  AB200_CUDA(launchChained(pulsePlanesKernel, dim3((unsigned)((long long)n_blk * (n_x + n_d))), dim3(256), 0,
-                           stream, p, n_x));
+  long long blocks = 0;
+  for (int k = 0; k < n; k++) {
+    const UpdateProblem &p = batch.tile[k];
+    const long long n_blk = (p.m * (p.nseg > 0 ? p.nseg : 1) + 31) / 32;
+    blocks = std::max(blocks, n_blk * ((p.x_size + PP_LINES - 1) / PP_LINES + (p.d_size + PP_LINES - 1) / PP_LINES));
+  }
+  AB200_CUDA(launchChained(pulsePlanesKernel<N>, dim3((unsigned)blocks, n), dim3(256), 0, stream, batch));
   AB200_LAUNCH_CHECK();
 }
 
-void launchPulsedUpdatePlanes(const UpdateProblem &p0, cudaStream_t stream) {
-  const UpdateProblem p = inRows(p0);
-  if (p.s_end <= p.s_begin) {
-    return;
+template <int N> static void launchUpdateOf(const UpdateBatch<N> &batch0, int n, cudaStream_t stream) {
+  UpdateBatch<N> batch = batch0;
+  for (int k = 0; k < n; k++) {
+    batch.tile[k] = inRows(batch0.tile[k]);
   }
-  switch (p.kind) {
+  switch (batch.tile[0].kind) {
   case AB200_DEVICE_CONSTANT_STEP:
-    launchPlanesKind<AB200_DEVICE_CONSTANT_STEP>(p, stream);
+    launchPlanesKind<AB200_DEVICE_CONSTANT_STEP>(batch, n, stream);
     break;
   case AB200_DEVICE_LINEAR_STEP:
   case AB200_DEVICE_SOFT_BOUNDS:
-    launchPlanesKind<AB200_DEVICE_LINEAR_STEP>(p, stream);
+    launchPlanesKind<AB200_DEVICE_LINEAR_STEP>(batch, n, stream);
     break;
   case AB200_DEVICE_SOFT_BOUNDS_REFERENCE:
-    launchPlanesKind<AB200_DEVICE_SOFT_BOUNDS_REFERENCE>(p, stream);
+    launchPlanesKind<AB200_DEVICE_SOFT_BOUNDS_REFERENCE>(batch, n, stream);
     break;
   case AB200_DEVICE_POW_STEP:
-    launchPlanesKind<AB200_DEVICE_POW_STEP>(p, stream);
+    launchPlanesKind<AB200_DEVICE_POW_STEP>(batch, n, stream);
     break;
   case AB200_DEVICE_EXP_STEP:
-    launchPlanesKind<AB200_DEVICE_EXP_STEP>(p, stream);
+    launchPlanesKind<AB200_DEVICE_EXP_STEP>(batch, n, stream);
     break;
   case AB200_DEVICE_PIECEWISE_STEP:
-    launchPlanesKind<AB200_DEVICE_PIECEWISE_STEP>(p, stream);
+    launchPlanesKind<AB200_DEVICE_PIECEWISE_STEP>(batch, n, stream);
     break;
   default:
     AB200_FATAL("pulsed update: device kind not implemented");
   }
   AB200_LAUNCH_CHECK();
+}
+
+void launchPulsePlanes(const UpdateProblem &p, cudaStream_t stream) {
+  launchPlanesOf(UpdateBatch<1>{{p}}, 1, stream);
+}
+
+void launchPulsedUpdatePlanes(const UpdateProblem &p, cudaStream_t stream) {
+  if (p.s_end > p.s_begin) {
+    launchUpdateOf(UpdateBatch<1>{{p}}, 1, stream);
+  }
+}
+
+void launchPulsedUpdateTiles(const UpdateProblem *p, int n, cudaStream_t stream) {
+  if (n == 1) {
+    launchPulsePlanes(p[0], stream);
+    launchPulsedUpdatePlanes(p[0], stream);
+    return;
+  }
+  if (n < 1 || n > kUpdateBatch) {
+    AB200_FATAL("pulsed update: invalid number of tiles in a launch");
+  }
+  UpdateBatch<kUpdateBatch> batch{};
+  std::copy(p, p + n, batch.tile);
+  launchPlanesOf(batch, n, stream);
+  launchUpdateOf(batch, n, stream);
 }
 
 } // namespace ab200

@@ -23,10 +23,21 @@ def _philox7(c, key):
     return c
 
 
-def _trains(v, strength, bl, key, tag):
+def _managed(x, d, lr, dw_min, desired):
+    """Train length and the factors of d and x per sample, update management on."""
+    f = np.float32
+    xm, dm = np.abs(x).max(1), np.abs(d).max(1)
+    k = ((f(lr) * xm).astype(f) * dm).astype(f) / f(dw_min)
+    bl = np.minimum(np.ceil(k), desired).astype(int)
+    unit = np.sqrt(f(lr) / (f(dw_min) * bl.astype(f)).astype(f)).astype(f)
+    dm = np.where(k > desired, (dm * (f(desired) / k)).astype(f), dm)
+    return bl, (unit * np.sqrt(xm / dm).astype(f)).astype(f), (unit * np.sqrt(dm / xm).astype(f)).astype(f)
+
+
+def _trains(v, strength, lengths, bl, key, tag):
     """Pulses ``[sample, line, slot]`` of a batch ``[sample, line]``."""
     m, n = v.shape
-    p = (np.abs(v) * np.float32(strength)).astype(np.float32)
+    p = (np.abs(v) * strength[:, None]).astype(np.float32)
     thr = np.ceil((p * np.float32(65536) - np.float32(0.5)).astype(np.float32))
     out = np.zeros((m, n, bl), bool)
     line, smp = np.arange(n)[None, :], np.arange(m)[:, None]
@@ -34,7 +45,7 @@ def _trains(v, strength, bl, key, tag):
         seg, slot = divmod(k, 31)
         r = _philox7((line, smp, 0, tag + seg * 4 + slot // 8), key)[(slot % 8) >> 1]
         out[:, :, k] = ((r >> np.uint64(16 * (slot & 1))) & np.uint64(0xFFFF)).astype(np.float64) < thr
-    return out
+    return out & (np.arange(bl) < lengths[:, None])[:, None, :]
 
 
 def _pool(task, refill, key):
@@ -94,6 +105,7 @@ def _apply_task(w, hi, lo, up, down, counts, dirs, rows, std, task, key):
     (4, 40, 70, 4, 0.8, "rows"),     # the first train of more than three slots
     (3, 32, 45, 31, 0.7, "trans"),   # longest train of one segment, many pulses per event
     (2, 35, 40, 40, 0.5, "rows"),    # two segments per sample
+    (3, 33, 300, 20, 0.5, "managed"),  # lengths per sample: blocks with and without more than three slots
 ])
 def test_pulses_and_noise_event_by_event(x_size, d_size, m, bl, scale, layout):
     from aihwkit_b200.rpu_base import devices as D
@@ -102,7 +114,7 @@ def test_pulses_and_noise_event_by_event(x_size, d_size, m, bl, scale, layout):
     rng = np.random.default_rng(x_size * 1000 + m)
     p = D.AnalogTileParameter()
     p.update.pulse_type, p.update.desired_bl = D.PulseType.StochasticCompressed, bl
-    p.update.update_management = p.update.update_bl_management = False
+    p.update.update_management = p.update.update_bl_management = layout == "managed"
     p.update.fixed_bl = True
     dp = D.ConstantStepResistiveDeviceParameter()
     dp.dw_min, dp.dw_min_std, dp.construction_seed, dp.enforce_consistency = 0.002, 0.3, 11, True
@@ -110,12 +122,17 @@ def test_pulses_and_noise_event_by_event(x_size, d_size, m, bl, scale, layout):
     seed = (5 << 32) | 1234567
     t.set_seed(seed)
     key = (seed & 0xFFFFFFFF, (seed >> 32) ^ 0x5BD1E995)
-    lr = 0.002 * bl  # strength sqrt(lr / (dw_min * bl)) = 1
+    lr = 0.01 if layout == "managed" else 0.002 * bl  # else: strength sqrt(lr / (dw_min * bl)) = 1
     t.set_learning_rate(lr)
-    strength = np.sqrt(np.float32(lr) / (np.float32(0.002) * np.float32(bl))).astype(np.float32)
     x = (rng.uniform(0.2, 1, (m, x_size)) * rng.choice([-1, 1], (m, x_size)) * scale).astype(np.float32)
     d = (rng.uniform(0.2, 1, (m, d_size)) * rng.choice([-1, 1], (m, d_size)) * scale).astype(np.float32)
     x[rng.random((m, x_size)) < 0.2] = 0.0
+    lengths = np.full(m, bl)
+    a = b = np.full(m, np.sqrt(np.float32(lr) / (np.float32(0.002) * np.float32(bl))), np.float32)
+    if layout == "managed":
+        x[:, 0], x[40:50] = np.where(x[:, 0] == 0, 0.5, x[:, 0]), x[40:50] * 4  # (no sample without a pulse)
+        lengths, a, b = _managed(x, d, lr, 0.002, bl)
+        assert (lengths <= 3).sum() > 200 and (lengths > 3).any()
     names = t.get_hidden_parameter_names()
     hp = t.get_hidden_parameters().numpy()
     hi, lo, up, down = (hp[names.index(k)] for k in ("max_bound", "min_bound", "dwmin_up", "dwmin_down"))
@@ -130,7 +147,7 @@ def test_pulses_and_noise_event_by_event(x_size, d_size, m, bl, scale, layout):
 
     # rows: samples, or the segments of at most 31 slots of each
     n_seg = (bl + 30) // 31
-    px, pd = _trains(x, strength, bl, key, TAG_X), _trains(d, strength, bl, key, TAG_D)
+    px, pd = _trains(x, b, lengths, bl, key, TAG_X), _trains(d, a, lengths, bl, key, TAG_D)
     busiest = 0
     for j in range(x_size):
         cut = [slice(31 * g, min(bl, 31 * g + 31)) for g in range(n_seg)]
@@ -148,3 +165,38 @@ def test_pulses_and_noise_event_by_event(x_size, d_size, m, bl, scale, layout):
     # cosine are approximations); a Gaussian given to another pulse moves a weight by about 6e-4
     assert np.abs(got - w).max() <= busiest * 2.0 ** -24
     assert busiest > 3
+
+
+@pytest.mark.parametrize("out_size,in_size,max_tile,m,omega", [
+    (70, 33, 64, 32, 0.0),     # two ragged tiles in one launch
+    (200, 130, 64, 65, 0.6),   # twelve tiles: a full launch and a rest, scaled gradients
+    (96, 300, 100, 40, 0.0),   # three tiles along the inputs
+])
+def test_tiles_of_a_layer_share_launches(out_size, in_size, max_tile, m, omega):
+    """Device noise off: the shared launches against the staged kernel tile by tile, bit for bit."""
+    from aihwkit_b200 import _cabi
+    from aihwkit_b200.rpu_base import tiles as T
+    from tests import helpers as H
+
+    g = torch.Generator().manual_seed(out_size + m)
+    p = H.training_params(noise=False, pulse_det=False)
+    cfg = p._config(max_tile, max_tile, H.device("sb", False, dw_min=0.002, dw_min_dtod=0.3), seed=5)
+    w = torch.rand(out_size, in_size, generator=g) - 0.5
+    x = (torch.rand(m, in_size, generator=g) * 2 - 1).cuda()
+    d = (torch.randn(m, out_size, generator=g) * 0.2).cuda()
+    out = []
+    lib = _cabi.lib()
+    try:
+        for path in (0, 1):
+            _cabi.check(lib.ab200_set_update_path(path))
+            layer = T.TileArray(cfg, out_size, in_size, max_tile, max_tile, cuda_device=0)
+            layer.set_seed(9)
+            layer.set_weights(w, weight_scaling_omega=omega)
+            layer.set_learning_rate(0.05)
+            for _ in range(2):
+                layer.update(x, d)
+            out.append(layer.get_weights())
+    finally:
+        _cabi.check(lib.ab200_set_update_path(0))
+    assert torch.equal(out[0], out[1])
+    assert (out[0] - w).abs().max() > 1e-3
