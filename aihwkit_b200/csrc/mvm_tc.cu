@@ -308,10 +308,11 @@ __device__ __forceinline__ uint64_t smemDesc(uint32_t saddr) {
   return d;
 }
 
-// kind::f16 instruction descriptor: D = F32, A = B = BF16, both K-major, M = 128, N = 256 (the
-// stacked hi and lo rows of the weight tile).
-constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) |
-                            ((uint32_t)(TC_ACC_COLS >> 3) << 17) | ((uint32_t)(TC_M >> 4) << 24);
+// kind::f16 instruction descriptor: D = F32, A = B = BF16, both K-major, M = 128, N = the stacked hi and lo rows
+// of the weight tile (256, fewer for a part of a chunk).
+__host__ __device__ constexpr uint32_t idesc(int n) {
+  return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(TC_M >> 4) << 24);
+}
 // the same for a CTA pair: M = 256, 128 rows in each CTA
 constexpr uint32_t kIdescPair = (1u << 4) | (1u << 7) | (1u << 10) |
                                 ((uint32_t)(TC_ACC_COLS >> 3) << 17) |
@@ -352,14 +353,21 @@ __device__ __forceinline__ void ownerOf(const TcKernelParams &p, int grow0, int 
 //               the accumulator rows of its own 128 rows in its own TMEM and runs its own epilogue.
 // LINE: the std-dev of the output noise is read per output line from a table (out_noise_std > 0,
 // single tile) and combined per element with the weight-noise term of the row.
-template <bool BM, bool PAIR, bool CODES = false, bool LINE = false>
+// CN (single CTAs): columns per work item, 128 or a part of a chunk. A product that fills a fraction of the
+// GPU is as long as one item, two thirds of it the epilogue's 32 columns per thread: with parts of 32 columns
+// the epilogue has eight.
+template <bool BM, bool PAIR, bool CODES = false, bool LINE = false, int CN = TC_N>
 __global__ void __launch_bounds__(TC_THREADS, 1)
     mvmTcKernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_bhi,
                 const __grid_constant__ CUtensorMap tm_blo, const TcKernelParams p) {
+  static_assert(CN == TC_N || (!PAIR && !CODES && !LINE), "parts of a chunk are for single CTAs");
+  constexpr int SUB = TC_N / CN; // parts of a chunk
+  constexpr int STAGE_B = CN * TC_K * 2;
+  constexpr int EPI_COLS = CN / (TC_EPI_WARPS / 4), ACC_COLS = 2 * CN;
   constexpr int STAGES = PAIR ? TC2_STAGES : TC_STAGES;
-  constexpr int STAGE_BYTES = PAIR ? TC2_STAGE_BYTES : TC_STAGE_BYTES;
   constexpr int KCH = PAIR ? TC2_KCH : TC_KCH;
-  constexpr int CHUNK_BYTES = PAIR ? TC2_CHUNK_BYTES : TC_CHUNK_BYTES;
+  constexpr int CHUNK_BYTES = PAIR ? TC2_CHUNK_BYTES : TC_STAGE_A + 2 * STAGE_B;
+  constexpr int STAGE_BYTES = KCH * CHUNK_BYTES;
   extern __shared__ uint8_t smem_raw[];
   // 1024-byte alignment for the swizzled tiles
   uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -380,10 +388,11 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
   // per group.
   constexpr int ROWS = PAIR ? 2 * TC_M : TC_M; // rows per work item
   const int n_rb = (p.m + ROWS - 1) / ROWS;
-  const int n_items = p.n_chunks * n_rb;
+  const int n_items = p.n_chunks * n_rb * SUB;
   const int worker = PAIR ? (int)blockIdx.x / 2 : (int)blockIdx.x;
   const int n_workers = PAIR ? (int)gridDim.x / 2 : (int)gridDim.x;
   auto item = [&](int w, int &chunk_idx, int &rb) {
+    w /= SUB; // (the part is w % SUB)
     const int per_group = p.group * n_rb;
     const int g = w / per_group, rem = w - g * per_group;
     const int gsize = min(p.group, p.n_chunks - g * p.group); // last group may be smaller
@@ -449,7 +458,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
       const int r0 = rb * ROWS + rank * TC_M;
       for (int i = 0; i < p.I && ok; i++) {
         const int4 is = p.insplit[i];
-        const int brow = i * p.nrows_pad + chunk_idx * TC_N;
+        const int brow = i * p.nrows_pad + chunk_idx * TC_N + (w % SUB) * CN;
         for (int kc0 = 0; kc0 < is.y; kc0 += KCH, it++) {
           const int nch = min(KCH, is.y - kc0); // chunks in this stage
           if (!TC_TIMED_WAIT(w_empty, mbarWait(&empty[ps], pph ^ 1u, abort_flag))) {
@@ -483,7 +492,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
                 const int kc = kc0 + c;
                 tmaLoad2d(st, &tm_a, &full[ps], is.x + kc * TC_K, r0);
                 tmaLoad2d(st + TC_STAGE_A, &tm_bhi, &full[ps], kc * TC_K, brow);
-                tmaLoad2d(st + TC_STAGE_A + TC_STAGE_B, &tm_blo, &full[ps], kc * TC_K, brow);
+                tmaLoad2d(st + TC_STAGE_A + STAGE_B, &tm_blo, &full[ps], kc * TC_K, brow);
               }
             }
           }
@@ -533,7 +542,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
           break;
         }
         tcFenceAfter();
-        const uint32_t d_tmem = tmem_base + (uint32_t)(b * TC_ACC_COLS);
+        const uint32_t d_tmem = tmem_base + (uint32_t)(b * ACC_COLS);
         for (int kc0 = 0; kc0 < nk; kc0 += KCH) {
           if (!TC_TIMED_WAIT(w_full, mbarWait(&full[ms], mph, abort_flag))) {
             atomicCAS(p.status, 0, TC_ERR_FULL);
@@ -559,7 +568,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
                 if (PAIR) {
                   tcMmaPair(d_tmem, da + 2 * k, db + 2 * k, kIdescPair, accum);
                 } else {
-                  tcMma(d_tmem, da + 2 * k, db + 2 * k, kIdesc, accum);
+                  tcMma(d_tmem, da + 2 * k, db + 2 * k, idesc(ACC_COLS), accum);
                 }
               }
             }
@@ -598,7 +607,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
   } else {
     // ------------------------------ epilogue warps ------------------------------
     const int q = warp & 3;                      // TMEM lane quarter this warp may access
-    const int cbase = (warp >> 2) * TC_EPI_COLS; // first of this warp's columns
+    const int cbase = (warp >> 2) * EPI_COLS; // first of this warp's columns
     const IOEff &io = p.io;
     const uint32_t tag = p.backward ? TAG_BWD_OUT : TAG_FWD_OUT;
     const bool adc = io.res_out > 0.0f;
@@ -613,7 +622,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
     auto loadAcc8 = [](uint32_t ta, float (&acc)[8]) {
       uint32_t vh[8], vl[8];
       tcLd8(ta, vh);
-      tcLd8(ta + (uint32_t)TC_N, vl);
+      tcLd8(ta + (uint32_t)CN, vl);
       tcWaitLd();
 #pragma unroll
       for (int j = 0; j < 8; j++) {
@@ -627,7 +636,13 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
     for (int w = worker; w < n_items && ok; w += n_workers) {
     int chunk_idx, rb;
     item(w, chunk_idx, rb);
-    const int4 ch = p.chunk[chunk_idx];
+    int4 ch = p.chunk[chunk_idx];
+    if (SUB > 1) {
+      const int first = (w % SUB) * CN; // of this part's columns
+      ch.y += first;
+      ch.z += first;
+      ch.w = min(ch.w - first, CN); // (not positive: nothing to store)
+    }
     const int row = rb * ROWS + rank * TC_M + q * 32 + lane;
     const bool row_ok = row < p.m;
     const uint32_t n4h = (uint32_t)((p.outn[ch.x] + 7) >> 3); // noise block pairs per row
@@ -635,9 +650,9 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
     // multiples of 8 columns)
     const uint64_t ctr0 = (uint64_t)((ch.y + cbase) >> 3);
     bool exceeded = false;
-    float sum[TC_EPI_COLS]; // running sums over the in-splits
+    float sum[EPI_COLS]; // running sums over the in-splits
 #pragma unroll
-    for (int c = 0; c < TC_EPI_COLS; c++) {
+    for (int c = 0; c < EPI_COLS; c++) {
       sum[c] = 0.0f;
     }
     // per-row scalars of the next in-split are fetched one iteration ahead
@@ -684,7 +699,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
       }
       tcFenceAfter();
       const uint32_t taddr =
-          tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(b * TC_ACC_COLS + cbase);
+          tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(b * ACC_COLS + cbase);
       const bool live = row_ok && sc != 0.0f;
       if (fast) {
         // Noisy regime with an ADC (the inference setting): the Gaussian decides the ADC code, so
@@ -697,10 +712,10 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
         if (CODES) {
           // The rounded, clipped code stays in the low mantissa bits of (value + 1.5 * 2^23):
           // its low byte is the two's-complement code. Four codes per word, eight words per row.
-          uint32_t cw[TC_EPI_COLS / 4];
+          uint32_t cw[EPI_COLS / 4];
           const float lo_m = kMagic - bound_codes, hi_m = kMagic + bound_codes;
 #pragma unroll
-          for (int c0 = 0; c0 < TC_EPI_COLS; c0 += 8) {
+          for (int c0 = 0; c0 < EPI_COLS; c0 += 8) {
             float acc[8];
             loadAcc8(taddr + (uint32_t)c0, acc);
             float z[8];
@@ -732,7 +747,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
             for (int h = 0; h < 2; h++) {
               uint32_t v[4];
 #pragma unroll
-              for (int j = 0; j < TC_EPI_COLS / 4; j++) {
+              for (int j = 0; j < EPI_COLS / 4; j++) {
                 const uint32_t t = __shfl_sync(0xffffffffu, cw[j], (lane >> 1) + 16 * h);
                 if ((j >> 2) == (lane & 1)) {
                   v[j & 3] = t;
@@ -746,7 +761,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
           }
         } else {
 #pragma unroll
-        for (int c0 = 0; c0 < TC_EPI_COLS; c0 += 8) {
+        for (int c0 = 0; c0 < EPI_COLS; c0 += 8) {
           float acc[8];
           loadAcc8(taddr + (uint32_t)c0, acc);
           float z[8];
@@ -766,7 +781,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
         }
       } else {
 #pragma unroll
-        for (int c0 = 0; c0 < TC_EPI_COLS; c0 += 8) {
+        for (int c0 = 0; c0 < EPI_COLS; c0 += 8) {
           float acc[8];
           loadAcc8(taddr + (uint32_t)c0, acc);
           if (live) {
@@ -813,7 +828,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
     }
     if (CODES) {
       // everything went out in-split by in-split
-    } else if (ok && (p.out_table || p.row_stores)) {
+    } else if (EPI_COLS == 32 && ok && (p.out_table || p.row_stores)) {
       // Scatter to the row-block owners, possibly peer memory: transpose the warp's 32 x 32
       // block in registers (five exchange steps) so that every store instruction writes 128
       // contiguous bytes of one row - over NVLink the 16-byte pieces of the row-per-lane layout
@@ -821,7 +836,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
 #pragma unroll
       for (int st = 16; st >= 1; st >>= 1) {
 #pragma unroll
-        for (int c = 0; c < TC_EPI_COLS; c++) {
+        for (int c = 0; c < EPI_COLS; c++) {
           if ((c & st) == 0) {
             const bool upper = (lane & st) != 0;
             const float send = upper ? sum[c] : sum[c | st];
@@ -859,7 +874,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
       const int blk = grow / p.out_t_rows, l = grow - blk * p.out_t_rows;
       float *o = p.out + ((long long)blk * p.out_ss + ch.z + cbase) * p.out_t_rows + l;
 #pragma unroll
-      for (int c = 0; c < TC_EPI_COLS; c++) {
+      for (int c = 0; c < EPI_COLS; c++) {
         if (cbase + c < ch.w) {
           o[(long long)c * p.out_t_rows] = sum[c] + (p.bias ? p.bias[ch.z + cbase + c] : 0.0f);
         }
@@ -870,14 +885,14 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
       float *orow = p.out + (long long)row * p.out_ss + ch.z + cbase;
       if (p.bias) {
 #pragma unroll
-        for (int c = 0; c < TC_EPI_COLS; c++) {
+        for (int c = 0; c < EPI_COLS; c++) {
           if (cbase + c < ch.w) {
             sum[c] += p.bias[ch.z + cbase + c];
           }
         }
       }
 #pragma unroll
-      for (int c = 0; c < TC_EPI_COLS; c += 4) {
+      for (int c = 0; c < EPI_COLS; c += 4) {
         const int cl = cbase + c;
         if (vec && cl + 3 < ch.w) {
           *reinterpret_cast<float4 *>(orow + c) =
@@ -1362,11 +1377,11 @@ static EncodeTiledFn encodeTiled() {
 
 // 2-D bf16 tensor [rows][cols] with row pitch `ld` elements; box = 64 columns x 128 rows,
 // 128-byte swizzle, out-of-range elements read as zero.
-static CUtensorMap makeMap(void *base, uint64_t rows, uint64_t cols, uint64_t ld) {
+static CUtensorMap makeMap(void *base, uint64_t rows, uint64_t cols, uint64_t ld, int box_rows = TC_M) {
   CUtensorMap map;
   cuuint64_t dims[2] = {cols, rows};
   cuuint64_t strides[1] = {ld * 2};
-  cuuint32_t box[2] = {(cuuint32_t)TC_K, (cuuint32_t)TC_M};
+  cuuint32_t box[2] = {(cuuint32_t)TC_K, (cuuint32_t)box_rows};
   cuuint32_t estr[2] = {1, 1};
   if (((uintptr_t)base & 15) != 0 || (strides[0] & 15) != 0) {
     AB200_FATAL("tensor map: base and row pitch must be 16-byte aligned");
@@ -1712,8 +1727,17 @@ void TcEngine::launchMma(const Run &r0, int row0, int rows, cudaStream_t s) {
   } d{ps.scale, ps.factor, ps.vnorm, ps.flags};
 
   CUtensorMap tm_a = makeMap(codes_part, (uint64_t)r.m, (uint64_t)I * kpad_, (uint64_t)I * kpad_);
-  CUtensorMap tm_bhi = makeMap(op_hi_, (uint64_t)I * nrows_pad_, (uint64_t)kpad_, (uint64_t)kpad_);
-  CUtensorMap tm_blo = makeMap(op_lo_, (uint64_t)I * nrows_pad_, (uint64_t)kpad_, (uint64_t)kpad_);
+  if (n_sm_ == 0) {
+    AB200_CUDA(cudaDeviceGetAttribute(&n_sm_, cudaDevAttrMultiProcessorCount, device_));
+  }
+  // Parts of a chunk where whole chunks leave most SMs idle: 32 columns while four times the items still are one
+  // per SM, else 64 (1024 x 1024, 256 rows: 16 items of 128 x 128 in 15.2 us, 64 of 128 x 32
+  // in 9.6; 512 x 512: 12.8 against 7.2)
+  const long long whole_items = (long long)n_chunks_ * ((r.m + TC_M - 1) / TC_M);
+  const bool may_part = mvmPath() != 3 && r.code_table == nullptr && r.onv == nullptr && r.out_table == nullptr;
+  const int part = !may_part ? TC_N : (4 * whole_items <= n_sm_ ? 32 : (2 * whole_items <= n_sm_ ? 64 : TC_N));
+  CUtensorMap tm_bhi = makeMap(op_hi_, (uint64_t)I * nrows_pad_, (uint64_t)kpad_, (uint64_t)kpad_, part);
+  CUtensorMap tm_blo = makeMap(op_lo_, (uint64_t)I * nrows_pad_, (uint64_t)kpad_, (uint64_t)kpad_, part);
 
   TcKernelParams p{};
   p.m = r.m;
@@ -1806,9 +1830,6 @@ void TcEngine::launchMma(const Run &r0, int row0, int rows, cudaStream_t s) {
   }
   p.prof = prof_dev;
   int grid_x = 0;
-  if (n_sm_ == 0) {
-    AB200_CUDA(cudaDeviceGetAttribute(&n_sm_, cudaDevAttrMultiProcessorCount, device_));
-  }
   const int n_sm = n_sm_;
   // the dynamic shared memory limit of a kernel variant is raised once per device
   auto raiseSmem = [&](auto kernel, int variant, int bytes) {
@@ -1819,7 +1840,7 @@ void TcEngine::launchMma(const Run &r0, int row0, int rows, cudaStream_t s) {
   };
   // chained with the kernels around it (see launchChained); not when the kernel signals peers
   const bool chained = pdlEnabled() && p.flag_table == nullptr;
-  const bool pair = usePairs(r.m);
+  const bool pair = part == TC_N && usePairs(r.m);
   const bool bm = r.io.bm != AB200_BM_NONE;
   const bool line = r.onv != nullptr;
   if (line && (codes || in_sizes_.size() != 1 || out_sizes_.size() != 1)) {
@@ -1850,12 +1871,20 @@ void TcEngine::launchMma(const Run &r0, int row0, int rows, cudaStream_t s) {
     AB200_CUDA(cudaLaunchKernelEx(&cfg, kernel, tm_a, tm_bhi, tm_blo, p));
     grid_x = 2 * n_pairs;
   } else {
-    const int n_items = n_chunks_ * ((r.m + TC_M - 1) / TC_M);
+    const int n_items = (int)whole_items * (TC_N / part);
     dim3 grid(n_items < n_sm ? n_items : n_sm); // one persistent CTA per SM
     auto kernel = codes ? mvmTcKernel<false, false, true>
                         : line ? (bm ? mvmTcKernel<true, false, false, true> : mvmTcKernel<false, false, false, true>)
                                : (bm ? mvmTcKernel<true, false> : mvmTcKernel<false, false>);
-    raiseSmem(kernel, codes ? 3 : (bm ? 4 : 5) + (line ? 6 : 0), TC_SMEM_BYTES);
+    int variant = codes ? 3 : (bm ? 4 : 5) + (line ? 6 : 0);
+    if (part == 64) {
+      kernel = bm ? mvmTcKernel<true, false, false, false, 64> : mvmTcKernel<false, false, false, false, 64>;
+      variant = bm ? 12 : 13;
+    } else if (part == 32) {
+      kernel = bm ? mvmTcKernel<true, false, false, false, 32> : mvmTcKernel<false, false, false, false, 32>;
+      variant = bm ? 14 : 15;
+    }
+    raiseSmem(kernel, variant, TC_SMEM_BYTES); // (parts of a chunk use less of it)
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = grid;
     cfg.blockDim = dim3(TC_THREADS);
