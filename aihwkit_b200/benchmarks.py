@@ -264,7 +264,7 @@ def main(argv=None, on_line=None):
     ap.add_argument("--batch", type=int, default=0, help="override the batch size")
     ap.add_argument("--indexed", action="store_true", help="config 3 through the indexed interface")
     ap.add_argument("--update-path", type=int, default=0, choices=[0, 1, 2],
-                    help="kernel of the pulsed update: 0 automatic, 1 staged, 2 streaming")
+                    help="kernel of the pulsed update: 0 automatic, 1 staged, 2 bit planes")
     args = ap.parse_args(argv)
     print(json.dumps(run(args.config, args.steps, args.warmup, args.batch, args.indexed, on_line,
                          args.update_path)))
