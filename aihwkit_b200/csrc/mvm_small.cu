@@ -383,7 +383,7 @@ bool smallMvmEligible(const MvmProblem &p) {
 }
 
 bool smallMvmOneRound(const MvmProblem &p) {
-  return smallMvmEligible(p) && p.in_size <= 2 * SM_K &&
+  return smallMvmEligible(p) && p.in_size <= SM_K &&
          (long long)((p.out_size + 31) / 32) * ((p.m + 15) / 16) <= smCount();
 }
 

@@ -1510,9 +1510,10 @@ bool Tile::tcEligible(const MvmProblem &p) const {
   if (mode >= 2) {
     return true;
   }
-  // A problem that the small-batch kernel serves with one CTA per SM at the most and in two steps along K takes
-  // it 8 to 18 us; operand split, DAC and tensor-core kernel do not come below 16 to 23 (512 x 512, 128 rows:
-  // 9.5 against 18.1; 1024 x 1024, 64 rows: 16.3 against 21.4).
+  // A problem that the small-batch kernel serves with one CTA per SM at the most and one step along K takes it
+  // 8 to 10 us; DAC and tensor-core kernel take 8 to 12 and the operand split another 3 once the weights have
+  // changed (512 x 512, 128 rows, forward 9.4 against 12.4 + 3, backward 10.2 against 9.4 + 3). With a second step
+  // or a second round it is the longer way (1024 x 512, 128 rows, backward: 18.7 against 9.4).
   return p.m >= 128 && (double)p.m * p.in_size * p.out_size >= 16777216.0 && !smallMvmOneRound(p);
 }
 

@@ -163,7 +163,7 @@ using SmallSplits = SmallSplitsT<kSmallSplits, kSmallTiles>;
 bool smallMvmIo(const IOEff &io); // IO settings these kernels implement
 int smallMvmMaxCtas(int in_size); // column blocks of 32 times row blocks of 16 up to which they are used
 bool smallMvmEligible(const MvmProblem &p);
-bool smallMvmOneRound(const MvmProblem &p); // eligible, one CTA per SM at the most, two steps along K at the most
+bool smallMvmOneRound(const MvmProblem &p); // eligible, one CTA per SM at the most, one step along K
 void launchMvmSmall(const MvmProblem &p, SmallSplits &sp, cudaStream_t stream);
 void launchMvmSmallTile(const MvmProblem &p, cudaStream_t stream);
 
