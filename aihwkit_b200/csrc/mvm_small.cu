@@ -169,7 +169,8 @@ __global__ void __launch_bounds__(32 * SM_WARPS) mvmSmallKernel(const __grid_con
           v = io.res_in > 0.0f ? __fmul_rn(code, io.res_in) : v;
           v = v > io.inp_bound ? io.inp_bound : v;
           v = v < -io.inp_bound ? -io.inp_bound : v;
-          v = scale != 0.0f ? v : 0.0f;
+          // (features past the end: zero whatever the scale, which is infinite for a row of very small numbers)
+          v = scale != 0.0f && q * 32 + lane < kn ? v : 0.0f;
           xr[q] = v;
           v_row[q * 32 + lane] = v;
         }
