@@ -5,6 +5,11 @@
 #include "mvm_common.cuh"
 #include "tile.h"
 
+#include <algorithm>
+#include <climits>
+#include <cmath>
+#include <cstring>
+
 namespace ab200 {
 
 __device__ __forceinline__ float blockMax(float v, float *sh) {
@@ -72,6 +77,35 @@ blAB(const UpEff &up, float lr, float dw_min, float xm, float dm, int &BL, float
       B = __fmul_rn(B, __fsqrt_rn(__fdiv_rn(d_val, x_val)));
     }
   }
+}
+
+// The longest train that blAB returns for any sample of an update with these settings: without a fixed length
+// and without update BL management a train has ceil(lr / dw_min) slots where that is more than desired_bl.
+static inline int longestTrain(const UpEff &up, float lr, float dw_min) {
+  if (up.fixed_bl || up.update_bl_management || !(dw_min * (float)up.desired_bl < lr)) {
+    return up.desired_bl;
+  }
+  const float bl = std::ceil(lr / dw_min);
+  return bl < 2147483648.0f ? std::max((int)bl, 1) : INT_MAX;
+}
+
+// Pulses of an implicit pair of lines with c = d * BL * x: |c| to the nearest integer, ties to even; none for
+// NaN. Up to kShortTrain slots (|c| <= BL) by adding 2^23, whose neighbours are 1 apart, which keeps the
+// count off the conversion pipe.
+constexpr int kShortTrain = 1 << 20;
+__host__ __device__ inline int implicitPulses(float c, bool short_train) {
+  const float a = fmaxf(fabsf(c), 0.0f);
+#ifdef __CUDA_ARCH__
+  return short_train ? __float_as_int(__fadd_rn(a, 8388608.0f)) - 0x4B000000 : __float2int_rn(a);
+#else
+  if (short_train) {
+    const float v = a + 8388608.0f;
+    int bits;
+    std::memcpy(&bits, &v, sizeof(bits));
+    return bits - 0x4B000000;
+  }
+  return a < 2147483648.0f ? (int)std::nearbyint(a) : INT_MAX;
+#endif
 }
 
 // A draw u of 16 bits gives a pulse when u + 0.5 < 65536 pp; as a comparison u < threshold of integers,

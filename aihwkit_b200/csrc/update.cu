@@ -460,7 +460,8 @@ constexpr int UD_I = 64;    // d-lines per CTA
 constexpr int UD_S = 64;    // samples staged at a time
 constexpr int UD_T = 4;     // groups of 64 threads, EJ x-lines each
 
-template <int KIND, int EJ> __global__ void __launch_bounds__(UD_I *UD_T) pulsedUpdateDenseKernel(UpdateProblem p) {
+template <int KIND, int EJ>
+__global__ void __launch_bounds__(UD_I *UD_T) pulsedUpdateDenseKernel(UpdateProblem p, bool short_train) {
   pdlEnter();
   constexpr int UJ = UD_T * EJ;
   __shared__ float sd[UD_S][UD_I];
@@ -468,7 +469,6 @@ template <int KIND, int EJ> __global__ void __launch_bounds__(UD_I *UD_T) pulsed
   const int ti = threadIdx.x % UD_I, tj = threadIdx.x / UD_I;
   const int i = blockIdx.x * UD_I + ti, j0 = blockIdx.y * UJ;
   const bool i_ok = i < p.d_size;
-  const bool small = p.up.desired_bl < (1 << 20); // |d BL x| <= BL: rounded by adding 1.5 * 2^23
   float w[EJ], w_in[EJ];
   PulseStep<KIND> step[EJ];
   bool flip[EJ];
@@ -510,14 +510,16 @@ template <int KIND, int EJ> __global__ void __launch_bounds__(UD_I *UD_T) pulsed
     __syncthreads();
     for (int r = 0; r < n_s; r++) {
       const float dv = sd[r][ti];
-      float c[EJ], n[EJ], most = 0.0f;
+      float c[EJ];
+      int n[EJ], most = 0;
 #pragma unroll
       for (int t = 0; t < EJ; t++) {
         c[t] = __fmul_rn(dv, sx[r][tj * EJ + t]);
-        n[t] = fabsf(small ? __fadd_rn(__fadd_rn(c[t], 12582912.0f), -12582912.0f) : rintf(c[t]));
-        most = fmaxf(most, n[t]);
+        n[t] = implicitPulses(c[t], short_train);
+        most = max(most, n[t]);
       }
-      for (float k = 0.5f; __any_sync(0xffffffffu, most > k); k += 1.0f) {
+      // (counted in whole numbers: the end is reached whatever the length of the train)
+      for (int k = 0; __any_sync(0xffffffffu, most > k); k++) {
 #pragma unroll
         for (int t = 0; t < EJ; t++) {
           // positive = decrease
@@ -546,10 +548,11 @@ template <int KIND> static void launchUpdateDense(const UpdateProblem &p, cudaSt
   }
   // four weights per thread where that still gives every SM a CTA, else one
   const int gx = (p.d_size + UD_I - 1) / UD_I, gy4 = (p.x_size + 15) / 16, gy1 = (p.x_size + 3) / 4;
+  const bool st = longestTrain(p.up, p.lr, p.dw_min) <= kShortTrain;
   if ((long long)gx * gy4 >= n_sm) {
-    AB200_CUDA(launchChained(pulsedUpdateDenseKernel<KIND, 4>, dim3(gx, gy4), dim3(UD_I * UD_T), 0, stream, p));
+    AB200_CUDA(launchChained(pulsedUpdateDenseKernel<KIND, 4>, dim3(gx, gy4), dim3(UD_I * UD_T), 0, stream, p, st));
   } else {
-    AB200_CUDA(launchChained(pulsedUpdateDenseKernel<KIND, 1>, dim3(gx, gy1), dim3(UD_I * UD_T), 0, stream, p));
+    AB200_CUDA(launchChained(pulsedUpdateDenseKernel<KIND, 1>, dim3(gx, gy1), dim3(UD_I * UD_T), 0, stream, p, st));
   }
 }
 

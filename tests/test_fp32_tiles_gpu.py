@@ -77,3 +77,29 @@ def test_implicit_pulses_without_noise(kind, x_size, d_size, m):
     t.update(torch.from_numpy(x).cuda(), torch.from_numpy(d).cuda())
     assert np.abs(t.get_weights().numpy() - w).max() <= 1e-6
     assert m * x_size < 5 or np.abs(w - before).max() > 0
+
+
+def test_implicit_pulses_of_long_trains():
+    """A train of ceil(lr / dw_min) = 2 million slots, past the length up to which the counts are rounded by adding
+    2^23, with few pulses per pair."""
+    from aihwkit_b200.rpu_base import tiles as T
+
+    rng = np.random.default_rng(3)
+    p = H.training_params(noise=False, pulse_det=True)
+    p.update.fixed_bl = p.update.update_management = p.update.update_bl_management = False
+    dp = H.device("sb", False, dw_min=5e-5, dw_min_dtod=0.3)
+    x_size, d_size, m = 40, 70, 33
+    cfg = p._config(x_size, d_size, dp, seed=5)
+    t = T.AnalogTile(cfg, cuda_device=0)
+    names, hp = t.get_hidden_parameter_names(), t.get_hidden_parameters().numpy()
+    t.set_weights(torch.from_numpy(rng.uniform(-0.3, 0.3, (d_size, x_size)).astype(np.float32)))
+    w = t.get_weights().numpy().copy()
+    t.set_learning_rate(100.0)
+    x = rng.uniform(-3e-3, 3e-3, (m, x_size)).astype(np.float32)
+    d = rng.uniform(-3e-3, 3e-3, (m, d_size)).astype(np.float32)
+    dev = O.DeviceArrays.from_hidden(O.DEV_SOFT_BOUNDS, names, hp, 0.0, getattr(dp, "mult_noise", True))
+    before = w.copy()
+    O.update(w, x, d, 100.0, dp.dw_min, O.Up.from_c(cfg.update), dev, None)
+    t.update(torch.from_numpy(x).cuda(), torch.from_numpy(d).cuda())
+    assert np.abs(t.get_weights().numpy() - w).max() <= 1e-6
+    assert np.abs(w - before).max() > 1e-3
