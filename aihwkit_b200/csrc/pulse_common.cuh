@@ -108,6 +108,19 @@ __host__ __device__ inline int implicitPulses(float c, bool short_train) {
 #endif
 }
 
+// Place in a warp's pool of `kNoisePool` Gaussians from which lane `lane` takes, or would take, its next one:
+// `pos` are gone, `takers` take one each and fit. All lanes look, those past the last taker just behind it: one
+// place behind the end when the pool is used up, which a row of the pool has.
+constexpr int kNoisePool = 256, kNoisePoolRow = kNoisePool + 1;
+__host__ __device__ inline int noisePoolSlot(int pos, uint32_t takers, int lane) {
+  const uint32_t before = takers & ((1u << lane) - 1u);
+#ifdef __CUDA_ARCH__
+  return pos + __popc(before);
+#else
+  return pos + __builtin_popcount(before);
+#endif
+}
+
 // A draw u of 16 bits gives a pulse when u + 0.5 < 65536 pp; as a comparison u < threshold of integers,
 // which keeps the draws off the conversion pipe.
 __device__ __forceinline__ int pulseThreshold(float pp) {

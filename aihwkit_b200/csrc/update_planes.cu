@@ -265,12 +265,12 @@ __global__ void __launch_bounds__(256) pulsePlanesKernel(const __grid_constant__
 // the update
 // ---------------------------------------------------------------------------------------------
 constexpr int UP_WARPS = 4;   // x-lines per CTA (neighbours share the sectors of the x planes)
-constexpr int UP_POOL = 256;  // Gaussians per warp pool (eight per lane and refill)
+constexpr int UP_POOL = kNoisePool; // Gaussians per warp pool (eight per lane and refill)
 constexpr int UP_DRAIN = 20;  // a lane with more events than this has the warp apply all events
 constexpr int UP_EVENTS = 24; // most events of a lane between two drains
 
 struct UpdatePlanesSmem {
-  float pool[UP_WARPS][UP_POOL]; // (lanes without an event read up to 31 values past the end)
+  float pool[UP_WARPS][kNoisePoolRow];
   uint8_t counts[UP_WARPS][UP_EVENTS][32]; // pulses of the events that have more than one
 };
 
@@ -364,7 +364,7 @@ __global__ void __launch_bounds__(32 * UP_WARPS, 8)
         refills++;
         pool_pos = 0;
       }
-      xi = pool[pool_pos + __popc(takers & lt_mask)];
+      xi = pool[noisePoolSlot(pool_pos, takers, lane)];
       pool_pos += n_take;
     }
     const float w_new = step.apply(p, w, down, xi, MULT);

@@ -1,5 +1,5 @@
 """Host-side rules of the pulsed update and arithmetic that its kernels share with the host, compiled and run on the
-CPU: the longest train of an update, the count of an implicit pair of lines."""
+CPU: the longest train of an update, the count of an implicit pair of lines, places in the pool of Gaussians."""
 
 import os
 import shutil
@@ -27,6 +27,19 @@ int main(int argc, char **argv) {
     for (int i = 3; i < argc; i++) {
       printf("%d\n", implicitPulses(strtof(argv[i], nullptr), argv[2][0] == '1'));
     }
+  } else { // the largest place that any lane looks at in a pool's row, and the length of the row
+    int largest = 0;
+    uint32_t takers = 1u;
+    for (int turn = 0; turn < 2000; turn++) {
+      takers = turn == 0 ? 0u : (turn == 1 ? 0xffffffffu : takers * 1664525u + 1013904223u);
+      const int n = __builtin_popcount(takers);
+      for (int pos = 0; pos + n <= kNoisePool; pos++) {
+        for (int lane = 0; lane < 32; lane++) {
+          largest = std::max(largest, noisePoolSlot(pos, takers, lane));
+        }
+      }
+    }
+    printf("%d %d\n", largest, kNoisePoolRow);
   }
   return 0;
 }
@@ -75,3 +88,8 @@ def test_counts_of_implicit_pulses(rules):
             assert got == [int(v) for v in np.rint(values)]
         assert rules("c", short, "nan") == [0]
     assert rules("c", "0", "1e12", "-inf") == [2 ** 31 - 1] * 2
+
+
+def test_no_lane_looks_past_its_pool(rules):
+    largest, row = rules("p")
+    assert largest < row
