@@ -120,7 +120,7 @@ enum : uint32_t {
   TAG_BWD_OUT = 0x20000000u,
   TAG_PULSE_X = 0x30000000u,
   TAG_PULSE_D = 0x40000000u,
-  TAG_DEVICE = 0x50000000u,    // + refill ordinal
+  TAG_DEVICE = 0x50000000u,    // + first row of the range of a batch that a launch applies
   TAG_TRANSFER_READ = 0x60000000u,
   TAG_FWD_IN = 0x70000000u,    // input noise / stochastic DAC rounding; + bound-management round
   TAG_BWD_IN = 0x80000000u,

@@ -108,6 +108,12 @@ __host__ __device__ inline int implicitPulses(float c, bool short_train) {
 #endif
 }
 
+// Stream of the device noise of a launch. A batch in which transfers fall is applied in ranges of its rows, a launch
+// each, under one call counter: the first row keeps their draws apart (a whole batch starts at row 0).
+__device__ __forceinline__ uint32_t deviceNoiseTag(const UpdateProblem &p) {
+  return TAG_DEVICE + (uint32_t)p.s_begin;
+}
+
 // Place in a warp's pool of `kNoisePool` Gaussians from which lane `lane` takes, or would take, its next one:
 // `pos` are gone, `takers` take one each and fit. All lanes look, those past the last taker just behind it: one
 // place behind the end when the pool is used up, which a row of the pool has.

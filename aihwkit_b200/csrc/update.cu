@@ -169,9 +169,9 @@ template <int NT, int UTJ> struct UpdateSmem {
 // rare, and inlining it into each of the four per-weight loop bodies makes the kernel spill out of
 // the instruction cache.
 __device__ __noinline__ void refillReservoir(PhiloxKey key, uint32_t gid, uint32_t refills,
-                                             uint32_t call, float *column, int stride) {
+                                             uint32_t call, uint32_t tag, float *column, int stride) {
   float z[8];
-  gauss8(key, (uint64_t)gid | ((uint64_t)refills << 32), call, TAG_DEVICE, z);
+  gauss8(key, (uint64_t)gid | ((uint64_t)refills << 32), call, tag, z);
 #pragma unroll
   for (int r = 0; r < URES; r++) {
     column[r * stride] = z[r];
@@ -360,13 +360,13 @@ __global__ void __launch_bounds__(UT_I *UTJ / EJ, (UT_I * UTJ / EJ) >= 1024 ? 1 
           // cannot serve its event (leftovers are discarded), so the refill is never divergent;
           // only an event with more pulses than the reservoir holds refills on its own.
           if (__any_sync(0xffffffffu, n > rc)) {
-            refillReservoir(p.key, gid, refills, p.call, &sm.sz[0][threadIdx.x], UNT);
+            refillReservoir(p.key, gid, refills, p.call, deviceNoiseTag(p), &sm.sz[0][threadIdx.x], UNT);
             rc = URES;
             refills++;
           }
           for (int k = 0; k < n; k++) {
             if (rc == 0) {
-              refillReservoir(p.key, gid, refills, p.call, &sm.sz[0][threadIdx.x], UNT);
+              refillReservoir(p.key, gid, refills, p.call, deviceNoiseTag(p), &sm.sz[0][threadIdx.x], UNT);
               rc = URES;
               refills++;
             }

@@ -276,10 +276,10 @@ struct UpdatePlanesSmem {
 
 // Eight fresh Gaussians per lane for a warp's pool, as offset + std * z. Out of line: rare against the pulses
 // that take from the pool at two places, and the largest piece of code among them.
-__device__ __noinline__ void refillPool(PhiloxKey key, uint64_t pair, uint32_t call, float std, float offset,
-                                        float *column) {
+__device__ __noinline__ void refillPool(PhiloxKey key, uint64_t pair, uint32_t call, uint32_t tag, float std,
+                                        float offset, float *column) {
   float z[8];
-  gauss8(key, pair, call, TAG_DEVICE, z);
+  gauss8(key, pair, call, tag, z);
 #pragma unroll
   for (int rr = 0; rr < 8; rr++) {
     column[rr * 32] = __fadd_rn(offset, __fmul_rn(std, z[rr]));
@@ -358,7 +358,7 @@ __global__ void __launch_bounds__(32 * UP_WARPS, 8)
       if (pool_pos + n_take > UP_POOL) {
         // all lanes refill together; what is left of the old pool is dropped
         __syncwarp();
-        refillPool(p.key, (uint64_t)(task * 32 + lane) | ((uint64_t)refills << 40), p.call, std,
+        refillPool(p.key, (uint64_t)(task * 32 + lane) | ((uint64_t)refills << 40), p.call, deviceNoiseTag(p), std,
                    PulseStep<KIND>::kOnePlus ? 1.0f : 0.0f, pool + lane);
         __syncwarp();
         refills++;

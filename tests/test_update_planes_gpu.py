@@ -200,3 +200,43 @@ def test_tiles_of_a_layer_share_launches(out_size, in_size, max_tile, m, omega):
         _cabi.check(lib.ab200_set_update_path(0))
     assert torch.equal(out[0], out[1])
     assert (out[0] - w).abs().max() > 1e-3
+
+
+@pytest.mark.parametrize("path,m", [(1, 24), (2, 24), (0, 64), (1, 64)])
+@pytest.mark.parametrize("every", [1, 5])
+def test_noise_of_the_ranges_between_transfers(path, m, every):
+    """A transfer compound whose transfers fall inside the batch applies it in ranges; a pulse on every weight for
+    every row, so the spread of the weights tells whether the ranges draw their noise independently."""
+    from aihwkit_b200 import _cabi
+    from aihwkit_b200.rpu_base import devices as D
+    from aihwkit_b200.rpu_base import tiles as T
+    from tests import helpers as H
+
+    x_size, d_size, dw_min, std = 40, 70, 1e-3, 0.3
+    dp = D.TransferResistiveDeviceParameter()
+    for _ in range(2):
+        dp.append_parameter(H.device("cs", True, dw_min=dw_min, dw_min_std=std, dw_min_dtod=0.0, up_down_dtod=0.0,
+                                     w_max=1.0, w_min=-1.0))
+    dp.construction_seed, dp.gamma, dp.transfer_every, dp.units_in_mbatch = 21, 0.0, float(every), False
+    dp.transfer_lr, dp.fast_lr = 0.0, 0.0  # the pulses take the learning rate; transfers cut the batch and write nothing
+    p = H.training_params(noise=False, pulse_det=False)
+    p.update.desired_bl, p.update.fixed_bl = 1, True
+    p.update.update_management = p.update.update_bl_management = False
+    lib = _cabi.lib()
+    try:
+        _cabi.check(lib.ab200_set_update_path(path))
+        t = T.AnalogTile(p._config(x_size, d_size, dp, seed=3), cuda_device=0)
+        t.set_learning_rate(dw_min)
+        t.set_weights(torch.zeros(d_size, x_size))
+        names = t.get_hidden_parameter_names()
+        fast = next(i for i, n in enumerate(names) if n.startswith("hidden_weights"))
+        before = t.get_hidden_parameters()[fast].double()
+        t.update(torch.ones(m, x_size, device="cuda"), -torch.ones(m, d_size, device="cuda"))
+        change = (t.get_hidden_parameters()[fast].double() - before) / dw_min
+    finally:
+        _cabi.check(lib.ab200_set_update_path(0))
+    n = change.numel()
+    # sums of m independent steps 1 + std * z over n weights: the mean of all, and their spread, each within five
+    # standard errors (the same draws in every range of r rows spread the sums sqrt(m / r) times as far)
+    assert abs(float(change.mean()) - m) <= 5 * std * (m / n) ** 0.5
+    assert abs(float(change.std()) / (std * m ** 0.5) - 1) <= 5 * (0.5 / n) ** 0.5
