@@ -18,17 +18,23 @@
 #include "mvm_common.cuh"
 #include "tile.h"
 
+#include <type_traits>
+
 namespace ab200 {
 
 constexpr int SM_WARPS = 16;
 constexpr int SM_K = 512;            // features per step: 32 per warp at most
 constexpr int SM_KW = SM_K / SM_WARPS;
 
-template <int ROWS, bool K_FAST, typename Splits>
+// STRIDED (single tiles): the features of a row are not neighbours in memory (transposed inputs, [features][rows]).
+// Neighbouring threads then load neighbouring rows, and the step goes through shared memory to the warps of the
+// rows.
+template <int ROWS, bool K_FAST, bool STRIDED, typename Splits>
 __global__ void __launch_bounds__(32 * SM_WARPS) mvmSmallKernel(const __grid_constant__ MvmProblem p,
                                                                 const __grid_constant__ Splits sp) {
   // prepared inputs of a step, later the partial sums of the warps
-  __shared__ __align__(16) float buf[ROWS * SM_K > SM_WARPS * ROWS * 32 ? ROWS * SM_K : SM_WARPS * ROWS * 32];
+  constexpr int LD = STRIDED ? SM_K + 4 : SM_K; // (the rows of a feature in other banks)
+  __shared__ __align__(16) float buf[ROWS * LD > SM_WARPS * ROWS * 32 ? ROWS * LD : SM_WARPS * ROWS * 32];
   const IOEff &io = p.io;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   int o = 0;
@@ -61,7 +67,22 @@ __global__ void __launch_bounds__(32 * SM_WARPS) mvmSmallKernel(const __grid_con
     kn = min(K - k0, SM_K);
     kw = ((kn + SM_WARPS - 1) / SM_WARPS + 3) & ~3; // features per warp, in fours
     kb = warp * kw;                                 // this warp's first, within the step
-    if (warp < ROWS) { // the inputs first: all that follows waits for them
+    if (STRIDED) { // element q: row threadIdx.x % ROWS, feature threadIdx.x / ROWS + q * (threads / ROWS)
+      const int r = blockIdx.y * ROWS + threadIdx.x % ROWS, f = threadIdx.x / ROWS;
+      const float *x = p.in + (long long)r * p.in_ss + (long long)(k0 + f) * p.in_fs;
+#pragma unroll
+      for (int q = 0; q < ROWS; q++) {
+        const int k = f + q * (32 * SM_WARPS / ROWS);
+        xr[q] = 0.0f;
+        if (r < p.m && k < kn) {
+          xr[q] = 1.0f; // the bias line
+          if (k0 + k < p.in_real) {
+            xr[q] = *x;
+          }
+        }
+        x += (32 * SM_WARPS / ROWS) * p.in_fs;
+      }
+    } else if (warp < ROWS) { // the inputs first: all that follows waits for them
       const int real = sp.n_in == 1 ? p.in_real - k0 : kn;
       const float *x = x_row + sp.in_off[ii] + k0 + lane;
 #pragma unroll
@@ -119,10 +140,24 @@ __global__ void __launch_bounds__(32 * SM_WARPS) mvmSmallKernel(const __grid_con
     acc[r] = 0.0f;
   }
   float total = 0.0f, scale = 0.0f, sval = 0.0f, vn = 0.0f;
+  const long long fs = STRIDED ? p.in_fs : 1;
   while (true) {
+    if (STRIDED) {
+#pragma unroll
+      for (int q = 0; q < ROWS; q++) {
+        buf[threadIdx.x % ROWS * LD + threadIdx.x / ROWS + q * (32 * SM_WARPS / ROWS)] = xr[q];
+      }
+      __syncthreads();
+      if (warp < ROWS) {
+#pragma unroll
+        for (int q = 0; q < SM_K / 32; q++) {
+          xr[q] = buf[warp * LD + q * 32 + lane];
+        }
+      }
+    }
     if (warp < ROWS) {
       const SmallTile &t = sp.tile[ii * sp.n_out + o];
-      float *const v_row = buf + warp * SM_K;
+      float *const v_row = buf + warp * LD;
       if (k0 == 0) {
         NmStats st;
         if (nmNeedsStats(io)) {
@@ -143,7 +178,7 @@ __global__ void __launch_bounds__(32 * SM_WARPS) mvmSmallKernel(const __grid_con
             const int real = sp.n_in == 1 ? p.in_real : K;
 #pragma unroll 4
             for (int k = SM_K + lane; k < K; k += 32) {
-              st.add(k < real ? x_row[sp.in_off[ii] + k] : 1.0f);
+              st.add(k < real ? x_row[sp.in_off[ii] + k * fs] : 1.0f);
             }
           }
           if (io.nm == AB200_NM_ABS_MAX) {
@@ -181,7 +216,7 @@ __global__ void __launch_bounds__(32 * SM_WARPS) mvmSmallKernel(const __grid_con
           for (int q = 0; q < SM_K / 32; q++) {
             const int k = k0 + q * 32 + lane;
             if (((ties >> q) & 1u) != 0u && q * 32 + lane < kn) {
-              xr[q] = dacPlain(io, inv_res, k < real ? x[k] : 1.0f, scale);
+              xr[q] = dacPlain(io, inv_res, k < real ? x[k * fs] : 1.0f, scale);
               v_row[q * 32 + lane] = xr[q];
             }
           }
@@ -218,7 +253,7 @@ __global__ void __launch_bounds__(32 * SM_WARPS) mvmSmallKernel(const __grid_con
       if (q < kw) {
 #pragma unroll
         for (int r = 0; r < ROWS; r++) {
-          const float4 a = *reinterpret_cast<const float4 *>(buf + r * SM_K + kb + q);
+          const float4 a = *reinterpret_cast<const float4 *>(buf + r * LD + kb + q);
           acc[r] = fmaf(a.x, w[q], acc[r]);
           acc[r] = fmaf(a.y, w[q + 1], acc[r]);
           acc[r] = fmaf(a.z, w[q + 2], acc[r]);
@@ -269,7 +304,10 @@ __global__ void __launch_bounds__(32 * SM_WARPS) mvmSmallKernel(const __grid_con
         } else if (io.is_perfect) {
           y *= fac;
         } else {
-          const float sigma = outputSigma(io, vn);
+          // (out_noise_std > 0: a standard deviation for every line)
+          const float sigma = p.out_noise_vals != nullptr
+                                  ? outputSigmaLine(io, vn, p.out_noise_vals, c_ok ? c : 0, 0.0f)
+                                  : outputSigma(io, vn);
           const uint64_t blk = (uint64_t)row * n4 + (uint64_t)(c >> 2);
           const int q = lane & 3; // column blocks start at multiples of 32
           float z = 0.0f, uq = 0.5f;
@@ -315,11 +353,12 @@ __global__ void __launch_bounds__(32 * SM_WARPS) mvmSmallKernel(const __grid_con
   }
 }
 
-bool smallMvmIo(const IOEff &io) {
+static bool smallMvmTileIo(const IOEff &io) {
   const bool running = !io.is_perfect && (io.nm == AB200_NM_AVERAGE_ABS_MAX ||
                                           io.nm == AB200_NM_AVERAGE_ABS_MAX_SINGLE_VALUE);
-  return !running && !ioNeedsLineChain(io) && !ioLineSigma(io);
+  return !running && !ioNeedsLineChain(io);
 }
+bool smallMvmIo(const IOEff &io) { return smallMvmTileIo(io) && !ioLineSigma(io); }
 
 static int smCount() {
   static int n_sm = 0; // SMs of the GPUs of this process (one kind per process)
@@ -343,10 +382,22 @@ int smallMvmMaxCtas(int in_size) {
 template <int ROWS, typename Splits>
 static void launchRows(const MvmProblem &p, const Splits &sp, bool k_fast, cudaStream_t stream) {
   dim3 grid(sp.col_blk[sp.n_out], (p.m + ROWS - 1) / ROWS);
+  const dim3 threads(32 * SM_WARPS);
+  if constexpr (std::is_same<Splits, SmallSplitsT<1, 1>>::value) {
+    if (p.in_fs != 1) {
+      if (k_fast) {
+        AB200_CUDA(launchChained(mvmSmallKernel<ROWS, true, true, Splits>, grid, threads, 0, stream, p, sp));
+      } else {
+        AB200_CUDA(launchChained(mvmSmallKernel<ROWS, false, true, Splits>, grid, threads, 0, stream, p, sp));
+      }
+      AB200_LAUNCH_CHECK();
+      return;
+    }
+  }
   if (k_fast) {
-    AB200_CUDA(launchChained(mvmSmallKernel<ROWS, true, Splits>, grid, dim3(32 * SM_WARPS), 0, stream, p, sp));
+    AB200_CUDA(launchChained(mvmSmallKernel<ROWS, true, false, Splits>, grid, threads, 0, stream, p, sp));
   } else {
-    AB200_CUDA(launchChained(mvmSmallKernel<ROWS, false, Splits>, grid, dim3(32 * SM_WARPS), 0, stream, p, sp));
+    AB200_CUDA(launchChained(mvmSmallKernel<ROWS, false, false, Splits>, grid, threads, 0, stream, p, sp));
   }
   AB200_LAUNCH_CHECK();
 }
@@ -376,15 +427,14 @@ template <typename Splits> static void launchSplits(const MvmProblem &p, Splits 
 void launchMvmSmall(const MvmProblem &p, SmallSplits &sp, cudaStream_t stream) { launchSplits(p, sp, stream); }
 
 bool smallMvmEligible(const MvmProblem &p) {
-  if (p.in_fs != 1 || (p.wk != 1 && p.wn != 1) || p.out_noise_vals != nullptr || p.gather.idx != nullptr ||
-      !smallMvmIo(p.io)) {
+  if ((p.wk != 1 && p.wn != 1) || p.gather.idx != nullptr || !smallMvmTileIo(p.io)) {
     return false;
   }
   return (long long)((p.out_size + 31) / 32) * ((p.m + 15) / 16) <= smallMvmMaxCtas(p.in_size);
 }
 
 bool smallMvmOneRound(const MvmProblem &p) {
-  return smallMvmEligible(p) && p.in_size <= SM_K &&
+  return smallMvmEligible(p) && p.out_noise_vals == nullptr && p.in_size <= SM_K &&
          (long long)((p.out_size + 31) / 32) * ((p.m + 15) / 16) <= smCount();
 }
 

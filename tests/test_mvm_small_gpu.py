@@ -101,3 +101,72 @@ def test_rows_of_very_small_numbers(size, w_noise, bm):
         assert (diff <= 16.01 * 24.0 / 510.0 * amax).all()
         assert (diff > 1e-3 * 24.0 / 510.0 * amax).double().mean() <= 0.005
     assert out[0][1][1].abs().max() > 0
+
+
+@pytest.mark.parametrize("m", [2, 4, 7, 16, 50])
+@pytest.mark.parametrize("x_size,d_size", [(2, 33), (40, 3), (130, 785), (512, 64), (513, 31), (1030, 40)])
+@pytest.mark.parametrize("bias", [False, True])
+def test_transposed_inputs_bit_for_bit(m, x_size, d_size, bias):
+    """[features][rows] inputs and outputs against the same rows the other way round, noise, bound management and
+    weight noise on."""
+    from aihwkit_b200.rpu_base import tiles as T
+
+    rng = np.random.default_rng(m * 1000 + x_size)
+    p = H.training_params(noise=True, pulse_det=False, out_bound=2.0)
+    for io in (p.forward_io, p.backward_io):
+        io.w_noise, io.w_noise_type = 0.02, H.D.WeightNoiseType.AdditiveConstant
+    cfg = p._config(x_size, d_size, H.device("cs", False), seed=3)
+    w = torch.from_numpy(rng.uniform(-0.5, 0.5, (d_size, x_size)).astype(np.float32))
+    x = torch.from_numpy(rng.uniform(-1, 1, (m, x_size - int(bias))).astype(np.float32)).cuda()
+    d = torch.from_numpy(rng.uniform(-1, 1, (m, d_size)).astype(np.float32)).cuda()
+    out = []
+    for trans in (False, True):
+        t = T.AnalogTile(cfg, cuda_device=0)
+        t.set_weights(w)
+        if trans:
+            y = t.forward(x.t().contiguous(), bias, True, True).t()
+            out.append((y, t.backward(d.t().contiguous(), bias, True, True).t()))
+        else:
+            out.append((t.forward(x, bias), t.backward(d, bias)))
+    assert torch.equal(out[0][0], out[1][0])
+    assert torch.equal(out[0][1], out[1][1])
+
+
+@pytest.mark.parametrize("x_size,d_size", [(40, 70), (600, 130)])
+@pytest.mark.parametrize("trans", [False, True])
+def test_noise_of_every_line(x_size, d_size, trans):
+    """out_noise_std > 0: a standard deviation per output line. Against the general kernel on a batch with the same
+    rows at its head."""
+    from aihwkit_b200 import _cabi
+    from aihwkit_b200.rpu_base import tiles as T
+
+    rng = np.random.default_rng(x_size)
+    p = H.training_params(noise=True, pulse_det=False)
+    for io in (p.forward_io, p.backward_io):
+        io.out_noise_std = 0.5
+    p.forward_io.bound_management = H.D.BoundManagementType.None_
+    cfg = p._config(x_size, d_size, H.device("cs", False), seed=3)
+    w = torch.from_numpy(rng.uniform(-0.1, 0.1, (d_size, x_size)).astype(np.float32))
+    x = rng.uniform(-1, 1, (8192, x_size)).astype(np.float32)
+    d = rng.uniform(-1, 1, (8192, d_size)).astype(np.float32)
+    out = []
+    lib = _cabi.lib()
+    try:
+        _cabi.check(lib.ab200_set_mvm_path(1))
+        for m in (9, 8192):
+            t = T.AnalogTile(cfg, cuda_device=0)
+            t.set_weights(w)
+            xm, dm = torch.from_numpy(x[:m]).cuda(), torch.from_numpy(d[:m]).cuda()
+            if trans:
+                y = t.forward(xm.t().contiguous(), False, True, True).t()
+                g = t.backward(dm.t().contiguous(), False, True, True).t()
+            else:
+                y, g = t.forward(xm), t.backward(dm)
+            out.append((y[:9].cpu().double(), g[:9].cpu().double()))
+    finally:
+        _cabi.check(lib.ab200_set_mvm_path(0))
+    for got, want, rows in zip(out[0], out[1], (x, d)):
+        # sums in another order: a code differs by one where the sum is next to a rounding tie
+        step = 24.0 / 510.0 * torch.from_numpy(np.abs(rows[:9]).max(1)).double()[:, None]
+        diff = (got - want).abs()
+        assert (diff <= 1.01 * step).all() and (diff > 1e-3 * step).double().mean() <= 0.005
