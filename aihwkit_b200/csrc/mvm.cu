@@ -478,7 +478,36 @@ __global__ void __launch_bounds__(256 * simtGroups(T)) mvmSimtKernel(MvmProblem 
 // ---------------------------------------------------------------------------------------------
 constexpr int BM_THREADS = 1024;
 
-__global__ void __launch_bounds__(BM_THREADS) bmRerunKernel(MvmProblem p, int n_slices, int k_slice) {
+// sum of v[k] w[k wk], k from k0 to k1 in order, with up to 32 loads in flight
+__device__ __forceinline__ float dotAhead(const float *v, const float *w, long long wk, int k0, int k1) {
+  float a = 0.0f;
+  int k = k0;
+  w += k0 * wk;
+  for (; k + 32 <= k1; k += 32) {
+#pragma unroll
+    for (int u = 0; u < 32; u++, w += wk) {
+      a = fmaf(v[k + u], *w, a);
+    }
+  }
+  for (; k + 8 <= k1; k += 8) {
+#pragma unroll
+    for (int u = 0; u < 8; u++, w += wk) {
+      a = fmaf(v[k + u], *w, a);
+    }
+  }
+  for (; k < k1; k++, w += wk) {
+    a = fmaf(v[k], *w, a);
+  }
+  return a;
+}
+
+// CHAIN: the IO settings need the line chain (three more sums per output; kept apart for the registers).
+// Products do not depend on the threads of the CTA: the K slices are those of the launch.
+// Flags of as many rows of a CTA as it has threads are read together: in the usual case, no row clipped, a walk over
+// them one after the other is all the kernel would spend its time on (131072 rows: 113 us of dependent loads
+// against 25).
+template <bool CHAIN>
+__global__ void __launch_bounds__(BM_THREADS, 1) bmRerunKernel(MvmProblem p, int n_slices, int k_slice) {
   pdlEnter();
   extern __shared__ float v_sh[]; // K prepared inputs, then the partial sums of the K slices
   const IOEff &io = p.io;
@@ -486,230 +515,206 @@ __global__ void __launch_bounds__(BM_THREADS) bmRerunKernel(MvmProblem p, int n_
   const uint64_t n4 = (uint64_t)(((N + 7) >> 3) << 1);
   float *const part_sh = v_sh + K;
   const int n_cb = (N + 31) / 32, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  // The flags of up to blockDim.x of this CTA's rows are read together: in the usual case, no row
-  // clipped, a walk over them one after the other is all the kernel would spend its time on (131072 rows:
-  // 113 us of dependent loads against 25).
   __shared__ int todo[BM_THREADS], n_todo;
-  for (long long base = blockIdx.x; base < p.m; base += (long long)gridDim.x * BM_THREADS) {
   if (threadIdx.x == 0) {
     n_todo = 0;
   }
-  __syncthreads();
-  {
+  for (long long base = blockIdx.x; base < p.m; base += (long long)gridDim.x * blockDim.x) {
     const long long mine = base + (long long)threadIdx.x * gridDim.x;
-    if (mine < p.m && p.flags[mine] != 0) {
+    const bool clipped = mine < p.m && p.flags[mine] != 0;
+    if (__syncthreads_or(clipped) == 0) {
+      continue;
+    }
+    if (clipped) {
       todo[atomicAdd(&n_todo, 1)] = (int)mine;
     }
-  }
-  __syncthreads();
-  const int n_rows = n_todo;
-  for (int at = 0; at < n_rows; at++) {
-    const int r = todo[at];
-    float sval = p.sval[r];
-    const float *row = p.in + (long long)r * p.in_ss;
-    const bool gathered = p.gather.idx != nullptr; // rows read through an index array
-    float reduction = 1.0f;
-    float scale = 1.0f;
-    int round = 0;
-    bool done = false;
-    while (!done) {
-      reduction *= 2.0f;
-      round++;
-      if (round == 1 && io.bm == AB200_BM_ITERATIVE_WORST_CASE && io.nm != AB200_NM_ABS_MAX_NP_SUM) {
-        // IterativeWorstCase: the first re-run switches to the AbsMaxNPSum scale and starts the
-        // halving again from there (rpu_forward_backward_pass.cpp:945-950)
-        NmStats st;
+    __syncthreads();
+    const int n_rows = n_todo;
+    for (int at = 0; at < n_rows; at++) {
+      const int r = todo[at];
+      float sval = p.sval[r];
+      const float *row = p.in + (long long)r * p.in_ss;
+      const bool gathered = p.gather.idx != nullptr; // rows read through an index array
+      float reduction = 1.0f;
+      float scale = 1.0f;
+      int round = 0;
+      bool done = false;
+      while (!done) {
+        reduction *= 2.0f;
+        round++;
+        if (round == 1 && io.bm == AB200_BM_ITERATIVE_WORST_CASE && io.nm != AB200_NM_ABS_MAX_NP_SUM) {
+          // IterativeWorstCase: the first re-run switches to the AbsMaxNPSum scale and starts the
+          // halving again from there (rpu_forward_backward_pass.cpp:945-950)
+          NmStats st;
+          for (int k = threadIdx.x; k < K; k += blockDim.x) {
+            st.add(gathered ? gatherRowElement(p.gather, p.in, r, k)
+                            : (k < p.in_real ? row[(long long)k * p.in_fs] : 1.0f));
+          }
+          st.warpReduce();
+          __shared__ float st_sh[BM_THREADS / 32][3];
+          if ((threadIdx.x & 31) == 0) {
+            st_sh[threadIdx.x >> 5][0] = st.amax;
+            st_sh[threadIdx.x >> 5][1] = st.psum;
+            st_sh[threadIdx.x >> 5][2] = st.nsum;
+          }
+          __syncthreads();
+          NmStats all;
+          for (int i = 0; i < (int)(blockDim.x >> 5); i++) {
+            all.amax = fmaxf(all.amax, st_sh[i][0]);
+            all.psum += st_sh[i][1];
+            all.nsum += st_sh[i][2];
+          }
+          __syncthreads();
+          sval = nmValueNPSum(io, all);
+          reduction = 1.0f;
+        }
+        scale = inputScale(io, sval, reduction, true);
+        const ElemRng g{p.key, p.call, TAG_FWD_IN + p.noise_id + (uint32_t)round * 0x10000u};
+        // squared norm of the prepared input, negative and positive half apart (the separate
+        // passes of pos_neg each see their own half)
+        float nacc_n = 0.0f, nacc_p = 0.0f;
         for (int k = threadIdx.x; k < K; k += blockDim.x) {
-          st.add(gathered ? gatherRowElement(p.gather, p.in, r, k)
-                          : (k < p.in_real ? row[(long long)k * p.in_fs] : 1.0f));
+          const float xin = gathered ? gatherRowElement(p.gather, p.in, r, k)
+                                     : (k < p.in_real ? row[(long long)k * p.in_fs] : 1.0f);
+          float v = prepareInput(io, xin, scale, g, (uint32_t)r, (uint32_t)k);
+          v_sh[k] = v;
+          if (v < 0.0f) {
+            nacc_n = fmaf(v, v, nacc_n);
+          } else {
+            nacc_p = fmaf(v, v, nacc_p);
+          }
         }
-        st.warpReduce();
-        __shared__ float st_sh[BM_THREADS / 32][3];
-        if ((threadIdx.x & 31) == 0) {
-          st_sh[threadIdx.x >> 5][0] = st.amax;
-          st_sh[threadIdx.x >> 5][1] = st.psum;
-          st_sh[threadIdx.x >> 5][2] = st.nsum;
+        float vn = 0.0f, vn_n = 0.0f, vn_p = 0.0f;
+        if (io.w_noise_type == AB200_WNOISE_ADDITIVE_CONSTANT && io.w_noise > 0.0f) {
+          for (int o = 16; o > 0; o >>= 1) {
+            nacc_n += __shfl_xor_sync(0xffffffffu, nacc_n, o);
+            nacc_p += __shfl_xor_sync(0xffffffffu, nacc_p, o);
+          }
+          __shared__ float red2_sh[BM_THREADS / 32][2];
+          if ((threadIdx.x & 31) == 0) {
+            red2_sh[threadIdx.x >> 5][0] = nacc_n;
+            red2_sh[threadIdx.x >> 5][1] = nacc_p;
+          }
+          __syncthreads();
+          float tn = 0.0f, tp = 0.0f;
+          for (int i = 0; i < (int)(blockDim.x >> 5); i++) {
+            tn += red2_sh[i][0];
+            tp += red2_sh[i][1];
+          }
+          vn = sqrtf(tn + tp);
+          vn_n = sqrtf(tn);
+          vn_p = sqrtf(tp);
         }
         __syncthreads();
-        NmStats all;
-        for (int i = 0; i < (int)(blockDim.x >> 5); i++) {
-          all.amax = fmaxf(all.amax, st_sh[i][0]);
-          all.psum += st_sh[i][1];
-          all.nsum += st_sh[i][2];
+        constexpr bool pcm = CHAIN;
+        const int pos_neg = CHAIN ? io.pos_neg : 0;
+        float sigma = pcm ? io.out_noise : outputSigma(io, vn);
+        const bool line_sigma = p.out_noise_vals != nullptr;
+        const LineChain lc{p.v_offset, p.out_nl, p.nl_factor, __fdiv_rn((float)K, io.ir_g_ratio)};
+        const uint32_t round_tag = TAG_FWD_OUT + p.noise_id + (uint32_t)round * 0x10000u;
+        const uint32_t round_tag_u = TAG_FWD_OUT_U + p.noise_id + (uint32_t)round * 0x10000u;
+        const bool w_draw = io.w_noise > 0.0f && io.w_noise_type != AB200_WNOISE_NONE;
+        int fail = 0;
+        if (n_slices > 1) {
+          // fewer blocks of 32 columns than warps: the warps share slices of K
+          for (int t = warp; t < n_cb * n_slices; t += (int)blockDim.x / 32) {
+            const int cb = t % n_cb, sl = t / n_cb, n = cb * 32 + lane;
+            const int k1 = min(K, (sl + 1) * k_slice);
+            const float *wp = p.w + (long long)(n < N ? n : 0) * p.wn;
+            const float a = dotAhead(v_sh, wp, p.wk, sl * k_slice, k1);
+            if (n < N) {
+              part_sh[sl * N + n] = a;
+            }
+          }
+          __syncthreads();
         }
-        __syncthreads();
-        sval = nmValueNPSum(io, all);
-        reduction = 1.0f;
+        for (int n = threadIdx.x; n < N; n += blockDim.x) {
+          // accumulator sets: [0] the only pass, or the pass over the positive inputs; [1] the
+          // pass over the negative inputs
+          float acc[2] = {0.0f, 0.0f}, acc2[2] = {0.0f, 0.0f}, acc_c[2] = {0.0f, 0.0f}, acc_i[2] = {0.0f, 0.0f};
+          const float *wp = p.w + (long long)n * p.wn;
+          if (pos_neg != 0) {
+            for (int k = 0; k < K; k++) {
+              const float wv = wp[(long long)k * p.wk], v = v_sh[k];
+              const float vp = fmaxf(v, 0.0f), vm = fminf(v, 0.0f), pw = irPosWeight(k, K), aw = fabsf(wv);
+              acc[0] = fmaf(vp, wv, acc[0]);
+              acc2[0] = fmaf(vp * vp, aw, acc2[0]);
+              acc_c[0] = fmaf(vp, aw, acc_c[0]);
+              acc_i[0] = fmaf(vp * pw, wv, acc_i[0]);
+              acc[1] = fmaf(vm, wv, acc[1]);
+              acc2[1] = fmaf(vm * vm, aw, acc2[1]);
+              acc_c[1] = fmaf(-vm, aw, acc_c[1]);
+              acc_i[1] = fmaf(vm * pw, wv, acc_i[1]);
+            }
+          } else if (pcm) {
+            for (int k = 0; k < K; k++) {
+              const float wv = wp[(long long)k * p.wk], v = v_sh[k];
+              acc[0] = fmaf(v, wv, acc[0]);
+              acc2[0] = fmaf(v * v, fabsf(wv), acc2[0]);
+              acc_c[0] = fmaf(fabsf(v), fabsf(wv), acc_c[0]);
+              acc_i[0] = fmaf(v * irPosWeight(k, K), wv, acc_i[0]);
+            }
+          } else if (n_slices > 1) {
+            for (int sl = 0; sl < n_slices; sl++) {
+              acc[0] += part_sh[sl * N + n];
+            }
+          } else {
+            acc[0] = dotAhead(v_sh, wp, p.wk, 0, K);
+          }
+          if (line_sigma) {
+            sigma = pcm ? p.out_noise_vals[n] : outputSigmaLine(io, vn, p.out_noise_vals, n, 0.0f);
+          }
+          const uint64_t blk = (uint64_t)r * n4 + (uint64_t)(n >> 2);
+          if (pcm) {
+            const float zw = w_draw ? gaussOf4(p.key, blk, p.call, round_tag ^ 0x04000000u, n & 3) : 0.0f;
+            acc[0] = lineChain(io, lc, acc[0], n, acc_c[0], acc_i[0], acc2[0], pos_neg != 0 ? vn_p : vn, zw,
+                               /*with_nl=*/pos_neg == 0);
+            if (pos_neg != 0) {
+              const float zwn = w_draw ? gaussOf4(p.key, blk, p.call, round_tag ^ 0x0c000000u, n & 3) : 0.0f;
+              acc[1] = lineChain(io, lc, acc[1], n, acc_c[1], acc_i[1], acc2[1], vn_n, zwn, /*with_nl=*/false);
+              if (pos_neg == 2) {
+                acc[0] = lineNonLinearity(lc, acc[0], n);
+                acc[1] = lineNonLinearity(lc, acc[1], n);
+              } else {
+                acc[0] = lineNonLinearity(lc, __fadd_rn(acc[0], acc[1]), n); // analog sum, then the output stage
+              }
+            }
+          }
+          const float z = sigma > 0.0f ? gaussOf4(p.key, blk, p.call, round_tag, n & 3) : 0.0f;
+          const float u = io.out_sto_round ? uniformOf4(p.key, blk, p.call, round_tag_u, n & 3) : 0.5f;
+          bool ex = false;
+          float y;
+          if (pos_neg == 2) {
+            const float zn = sigma > 0.0f ? gaussOf4(p.key, blk, p.call, round_tag ^ 0x08000000u, n & 3) : 0.0f;
+            const float un = io.out_sto_round ? uniformOf4(p.key, blk, p.call, round_tag_u ^ 0x08000000u, n & 3) : 0.5f;
+            const float yn = finalizeOutput(io, acc[1], sigma, zn, ex, un);
+            y = __fadd_rn(finalizeOutput(io, acc[0], sigma, z, ex, u), yn);
+          } else {
+            y = finalizeOutput(io, acc[0], sigma, z, ex, u);
+          }
+          fail |= ex ? 1 : 0;
+          if (n < p.out_store) {
+            *mvmOutPtr(p, r, n) = y;
+          }
+        }
+        int any_fail = __syncthreads_or(fail);
+        done = !any_fail || ((int)reduction > io.max_bm_factor) ||
+               (io.res_in > 0.0f && reduction > __fdiv_rn(io.max_bm_res, io.res_in));
       }
-      scale = inputScale(io, sval, reduction, true);
-      const ElemRng g{p.key, p.call, TAG_FWD_IN + p.noise_id + (uint32_t)round * 0x10000u};
-      // squared norm of the prepared input, negative and positive half apart (the separate
-      // passes of pos_neg each see their own half)
-      float nacc_n = 0.0f, nacc_p = 0.0f;
-      for (int k = threadIdx.x; k < K; k += blockDim.x) {
-        const float xin = gathered ? gatherRowElement(p.gather, p.in, r, k)
-                                   : (k < p.in_real ? row[(long long)k * p.in_fs] : 1.0f);
-        float v = prepareInput(io, xin, scale, g, (uint32_t)r, (uint32_t)k);
-        v_sh[k] = v;
-        if (v < 0.0f) {
-          nacc_n = fmaf(v, v, nacc_n);
-        } else {
-          nacc_p = fmaf(v, v, nacc_p);
-        }
+      float fac = outputFactor(io, p.alpha, sval, scale, false);
+      for (int n = threadIdx.x; n < N && n < p.out_store; n += blockDim.x) {
+        *mvmOutPtr(p, r, n) *= fac;
       }
-      float vn = 0.0f, vn_n = 0.0f, vn_p = 0.0f;
-      if (io.w_noise_type == AB200_WNOISE_ADDITIVE_CONSTANT && io.w_noise > 0.0f) {
-        for (int o = 16; o > 0; o >>= 1) {
-          nacc_n += __shfl_xor_sync(0xffffffffu, nacc_n, o);
-          nacc_p += __shfl_xor_sync(0xffffffffu, nacc_p, o);
-        }
-        __shared__ float red2_sh[BM_THREADS / 32][2];
-        if ((threadIdx.x & 31) == 0) {
-          red2_sh[threadIdx.x >> 5][0] = nacc_n;
-          red2_sh[threadIdx.x >> 5][1] = nacc_p;
-        }
-        __syncthreads();
-        float tn = 0.0f, tp = 0.0f;
-        for (int i = 0; i < (int)(blockDim.x >> 5); i++) {
-          tn += red2_sh[i][0];
-          tp += red2_sh[i][1];
-        }
-        vn = sqrtf(tn + tp);
-        vn_n = sqrtf(tn);
-        vn_p = sqrtf(tp);
+      if (threadIdx.x == 0) {
+        atomicAdd(&p.bm_stats[0], 1);
+        atomicMax(&p.bm_stats[1], __float_as_int(reduction));
+        p.flags[r] = 0; // served: the flags are zero again when the next pass starts
       }
       __syncthreads();
-      const bool pcm = ioNeedsLineChain(io);
-      const int pos_neg = io.pos_neg;
-      float sigma = pcm ? io.out_noise : outputSigma(io, vn);
-      const bool line_sigma = p.out_noise_vals != nullptr;
-      const LineChain lc{p.v_offset, p.out_nl, p.nl_factor, __fdiv_rn((float)K, io.ir_g_ratio)};
-      const uint32_t round_tag = TAG_FWD_OUT + p.noise_id + (uint32_t)round * 0x10000u;
-      const uint32_t round_tag_u = TAG_FWD_OUT_U + p.noise_id + (uint32_t)round * 0x10000u;
-      const bool w_draw = io.w_noise > 0.0f && io.w_noise_type != AB200_WNOISE_NONE;
-      int fail = 0;
-      if (n_slices > 1) {
-        // fewer blocks of 32 columns than warps: the warps share slices of K
-        for (int t = warp; t < n_cb * n_slices; t += BM_THREADS / 32) {
-          const int cb = t % n_cb, sl = t / n_cb, n = cb * 32 + lane;
-          const int k1 = min(K, (sl + 1) * k_slice);
-          const float *wp = p.w + (long long)(n < N ? n : 0) * p.wn;
-          float a = 0.0f;
-#pragma unroll 32
-          for (int k = sl * k_slice; k < k1; k++) {
-            a = fmaf(v_sh[k], wp[(long long)k * p.wk], a);
-          }
-          if (n < N) {
-            part_sh[sl * N + n] = a;
-          }
-        }
-        __syncthreads();
-      }
-      for (int n = threadIdx.x; n < N; n += blockDim.x) {
-        // accumulator sets: [0] the only pass, or the pass over the positive inputs; [1] the
-        // pass over the negative inputs
-        float acc[2] = {0.0f, 0.0f}, acc2[2] = {0.0f, 0.0f}, acc_c[2] = {0.0f, 0.0f}, acc_i[2] = {0.0f, 0.0f};
-        const float *wp = p.w + (long long)n * p.wn;
-        if (pos_neg != 0) {
-          for (int k = 0; k < K; k++) {
-            const float wv = wp[(long long)k * p.wk], v = v_sh[k];
-            const float vp = fmaxf(v, 0.0f), vm = fminf(v, 0.0f), pw = irPosWeight(k, K), aw = fabsf(wv);
-            acc[0] = fmaf(vp, wv, acc[0]);
-            acc2[0] = fmaf(vp * vp, aw, acc2[0]);
-            acc_c[0] = fmaf(vp, aw, acc_c[0]);
-            acc_i[0] = fmaf(vp * pw, wv, acc_i[0]);
-            acc[1] = fmaf(vm, wv, acc[1]);
-            acc2[1] = fmaf(vm * vm, aw, acc2[1]);
-            acc_c[1] = fmaf(-vm, aw, acc_c[1]);
-            acc_i[1] = fmaf(vm * pw, wv, acc_i[1]);
-          }
-        } else if (pcm) {
-          for (int k = 0; k < K; k++) {
-            const float wv = wp[(long long)k * p.wk], v = v_sh[k];
-            acc[0] = fmaf(v, wv, acc[0]);
-            acc2[0] = fmaf(v * v, fabsf(wv), acc2[0]);
-            acc_c[0] = fmaf(fabsf(v), fabsf(wv), acc_c[0]);
-            acc_i[0] = fmaf(v * irPosWeight(k, K), wv, acc_i[0]);
-          }
-        } else if (n_slices > 1) {
-          for (int sl = 0; sl < n_slices; sl++) {
-            acc[0] += part_sh[sl * N + n];
-          }
-        } else {
-#pragma unroll 32
-          for (int k = 0; k < K; k++) {
-            acc[0] = fmaf(v_sh[k], wp[(long long)k * p.wk], acc[0]);
-          }
-        }
-        if (line_sigma) {
-          sigma = pcm ? p.out_noise_vals[n] : outputSigmaLine(io, vn, p.out_noise_vals, n, 0.0f);
-        }
-        const uint64_t blk = (uint64_t)r * n4 + (uint64_t)(n >> 2);
-        if (pcm) {
-          float zw[4] = {0.f, 0.f, 0.f, 0.f};
-          if (w_draw) {
-            gauss4(p.key, blk, p.call, round_tag ^ 0x04000000u, zw);
-          }
-          acc[0] = lineChain(io, lc, acc[0], n, acc_c[0], acc_i[0], acc2[0], pos_neg != 0 ? vn_p : vn, zw[n & 3],
-                             /*with_nl=*/pos_neg == 0);
-          if (pos_neg != 0) {
-            float zwn[4] = {0.f, 0.f, 0.f, 0.f};
-            if (w_draw) {
-              gauss4(p.key, blk, p.call, round_tag ^ 0x0c000000u, zwn);
-            }
-            acc[1] = lineChain(io, lc, acc[1], n, acc_c[1], acc_i[1], acc2[1], vn_n, zwn[n & 3], /*with_nl=*/false);
-            if (pos_neg == 2) {
-              acc[0] = lineNonLinearity(lc, acc[0], n);
-              acc[1] = lineNonLinearity(lc, acc[1], n);
-            } else {
-              acc[0] = lineNonLinearity(lc, __fadd_rn(acc[0], acc[1]), n); // analog sum, then the output stage
-            }
-          }
-        }
-        float z[4] = {0.f, 0.f, 0.f, 0.f};
-        if (sigma > 0.0f) {
-          gauss4(p.key, blk, p.call, round_tag, z);
-        }
-        float u[4] = {0.5f, 0.5f, 0.5f, 0.5f};
-        if (io.out_sto_round) {
-          uniform4(p.key, blk, p.call, round_tag_u, u);
-        }
-        bool ex = false;
-        float y;
-        if (pos_neg == 2) {
-          float zn[4] = {0.f, 0.f, 0.f, 0.f}, un[4] = {0.5f, 0.5f, 0.5f, 0.5f};
-          if (sigma > 0.0f) {
-            gauss4(p.key, blk, p.call, round_tag ^ 0x08000000u, zn);
-          }
-          if (io.out_sto_round) {
-            uniform4(p.key, blk, p.call, round_tag_u ^ 0x08000000u, un);
-          }
-          const float yn = finalizeOutput(io, acc[1], sigma, zn[n & 3], ex, un[n & 3]);
-          y = __fadd_rn(finalizeOutput(io, acc[0], sigma, z[n & 3], ex, u[n & 3]), yn);
-        } else {
-          y = finalizeOutput(io, acc[0], sigma, z[n & 3], ex, u[n & 3]);
-        }
-        fail |= ex ? 1 : 0;
-        if (n < p.out_store) {
-          *mvmOutPtr(p, r, n) = y;
-        }
-      }
-      int any_fail = __syncthreads_or(fail);
-      done = !any_fail || ((int)reduction > io.max_bm_factor) ||
-             (io.res_in > 0.0f && reduction > __fdiv_rn(io.max_bm_res, io.res_in));
-    }
-    float fac = outputFactor(io, p.alpha, sval, scale, false);
-    for (int n = threadIdx.x; n < N && n < p.out_store; n += blockDim.x) {
-      *mvmOutPtr(p, r, n) *= fac;
     }
     if (threadIdx.x == 0) {
-      atomicAdd(&p.bm_stats[0], 1);
-      atomicMax(&p.bm_stats[1], __float_as_int(reduction));
-      p.flags[r] = 0; // served: the flags are zero again when the next pass starts
+      n_todo = 0; // (read by all before the row loop, whose end is behind a barrier; next used behind another)
     }
-    __syncthreads();
-  }
-  __syncthreads();
   }
 }
 
@@ -810,19 +815,37 @@ void launchBmRerun(const MvmProblem &p, cudaStream_t stream) {
   if ((size_t)p.in_size * sizeof(float) > 200 * 1024) {
     AB200_FATAL("bound management: x_size too large for the re-run kernel");
   }
-  // K slices: as many as there are more warps than column blocks, 64 features each at the least (785 x 130,
-  // 10 rows of which some clip: 59 -> 23 us)
+  static int n_sm = 0; // SMs of the GPUs of this process (one kind per process)
+  if (n_sm == 0) {
+    int dev = 0;
+    AB200_CUDA(cudaGetDevice(&dev));
+    AB200_CUDA(cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev));
+  }
+  const bool chain = ioNeedsLineChain(p.io);
   const int n_cb = (p.out_size + 31) / 32;
-  const int n_slices =
-      ioNeedsLineChain(p.io) ? 1 : std::max(1, std::min(BM_THREADS / 32 / n_cb, p.in_size / 64));
+  const int max_slices = chain ? 1 : std::max(1, p.in_size / 64);
+  // Threads per row. Where a CTA has a row of its own: 1024, the shortest way for that row. With more rows than
+  // that: as many as columns, 256 at least (128 where K slices of 64 features do not fill more), so that two to
+  // eight rows share an SM and the barriers and output stages of one pass beside the loads of another. Half of the
+  // rows re-run, one row per SM against this, us: 256 x 256, 4096 rows 393 / 201; 512 x 512, 2048 rows 847 / 459; 785 x
+  // 130, 1000 rows with the line chain 3190 / 682. (592 CTAs of 256 threads for all: 193, 528, 1236.)
+  int threads = BM_THREADS;
+  if (p.m > 2 * n_sm && p.out_size <= 512) {
+    threads = p.out_size > 256 ? 512 : ((long long)n_cb * max_slices <= 4 ? 128 : 256);
+  }
+  // (two CTAs in turn for every place on an SM even out how many of their rows clip; one where the rows are small)
+  const int blocks = std::min(p.m, (threads > 128 ? 2 : 1) * n_sm * (BM_THREADS / threads));
+  // K slices: as many as 1024 threads have more warps than column blocks, 64 features each at the least (785 x 130,
+  // 10 rows of which some clip: 59 -> 23 us)
+  const int n_slices = std::max(1, std::min(BM_THREADS / 32 / n_cb, max_slices));
   const int k_slice = (p.in_size + n_slices - 1) / n_slices;
   const size_t smem =
       ((size_t)p.in_size + (n_slices > 1 ? (size_t)n_slices * p.out_size : 0)) * sizeof(float);
+  auto kernel = chain ? bmRerunKernel<true> : bmRerunKernel<false>;
   if (smem > 40 * 1024) {
-    AB200_CUDA(cudaFuncSetAttribute(bmRerunKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 204 * 1024));
+    AB200_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 204 * 1024));
   }
-  const int blocks = p.m < 296 ? p.m : 296; // two per SM at the most
-  AB200_CUDA(launchChained(bmRerunKernel, dim3(blocks), dim3(BM_THREADS), smem, stream, p, n_slices, k_slice));
+  AB200_CUDA(launchChained(kernel, dim3(blocks), dim3(threads), smem, stream, p, n_slices, k_slice));
   AB200_LAUNCH_CHECK();
 }
 

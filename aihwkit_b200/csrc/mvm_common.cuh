@@ -290,6 +290,13 @@ uniform4(PhiloxKey key, uint64_t blk, uint32_t call, uint32_t tag, float u[4]) {
   }
 }
 
+// uniform q (0..3) of that block
+__device__ __forceinline__ float uniformOf4(PhiloxKey key, uint64_t blk, uint32_t call, uint32_t tag, int q) {
+  uint32_t r[4];
+  philox4x32<7>((uint32_t)blk, (uint32_t)(blk >> 32), call, tag, key, r);
+  return u01(q == 0 ? r[0] : (q == 1 ? r[1] : (q == 2 ? r[2] : r[3])));
+}
+
 // finalizeOutputImplStage5 (rpu_forward_backward_pass.cpp:673-719): asymmetry of negative values,
 // noise, ADC (rounding to nearest, or stochastic with the uniform `u`), clip / bound test.
 __device__ __forceinline__ float

@@ -170,3 +170,39 @@ def test_noise_of_every_line(x_size, d_size, trans):
         step = 24.0 / 510.0 * torch.from_numpy(np.abs(rows[:9]).max(1)).double()[:, None]
         diff = (got - want).abs()
         assert (diff <= 1.01 * step).all() and (diff > 1e-3 * step).double().mean() <= 0.005
+
+
+@pytest.mark.parametrize("kind", ["plain", "weight noise", "line noise", "line chain", "worst case"])
+@pytest.mark.parametrize("x_size,d_size", [(40, 33), (300, 70), (75, 300), (130, 520)])
+def test_rerun_of_a_row_does_not_depend_on_the_other_rows(kind, x_size, d_size):
+    """Bound management with 256, 512 and 1024 threads per row and up to five rows per CTA: a row has the same bits
+    whether it is the only one of its CTA that clips or one of all."""
+    from aihwkit_b200.rpu_base import tiles as T
+
+    rng = np.random.default_rng(x_size)
+    p = H.training_params(noise=True, pulse_det=False, out_bound=0.05 * x_size)
+    io = p.forward_io
+    if kind == "weight noise":
+        io.w_noise, io.w_noise_type = 0.05, H.D.WeightNoiseType.AdditiveConstant
+    elif kind == "line noise":
+        io.out_noise_std = 0.3
+    elif kind == "line chain":
+        io.w_noise, io.w_noise_type = 0.02, H.D.WeightNoiseType.PCMRead
+    elif kind == "worst case":
+        io.bound_management = H.D.BoundManagementType.IterativeWorstCase
+    cfg = p._config(x_size, d_size, H.device("cs", False), seed=3)
+    w = rng.uniform(-0.5, 0.5, (d_size, x_size)).astype(np.float32)
+    m = 1300  # up to five rows per CTA
+    few = np.sort(rng.choice(m, 40, replace=False))
+    x = (np.sign(w[rng.integers(0, d_size, m)]) * rng.uniform(0.8, 1, (m, x_size))).astype(np.float32)
+    rest = 0.02 * rng.uniform(-1, 1, (m, x_size)).astype(np.float32)
+    rest[:, 0] = 1.0
+    rest[few] = x[few]
+    out, served = [], []
+    for rows in (x, rest):
+        t = T.AnalogTile(cfg, cuda_device=0)
+        t.set_weights(torch.from_numpy(w))
+        out.append(t.forward(torch.from_numpy(rows).cuda())[torch.from_numpy(few).cuda()])
+        served.append(t.last_bm_stats()[0])
+    assert served[0] == m and 40 <= served[1] <= 60
+    assert torch.equal(out[0], out[1])
