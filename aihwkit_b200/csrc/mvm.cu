@@ -148,6 +148,8 @@ __global__ void __launch_bounds__(256 * simtGroups(T)) mvmSimtKernel(MvmProblem 
   float(*const As)[BK][BM + 4] = As_all[grp];
   float(*const Bs)[BK][BN + 4] = Bs_all[grp];
   __shared__ float s_scale[BM];
+  // position weights of a step: a division per feature and thread otherwise (785 x 130, 1000 rows: 192 -> 111 us)
+  __shared__ float Ps[2][PCM ? BK : 1];
   const IOEff &io = p.io;
   const int tid = threadIdx.x & 255;
   const int tx = tid & 15, ty = tid >> 4;
@@ -248,6 +250,9 @@ __global__ void __launch_bounds__(256 * simtGroups(T)) mvmSimtKernel(MvmProblem 
     }
   };
   auto stage = [&](int buf, int k0) {
+    if (PCM && tid < BK) {
+      Ps[buf][PCM ? tid : 0] = irPosWeight(k0 + tid, K);
+    }
 #pragma unroll
     for (int u = 0; u < NE; u++) {
       const int r = a_r + (A_K_FAST ? 0 : u), kk = a_k + (A_K_FAST ? u : 0);
@@ -294,7 +299,7 @@ __global__ void __launch_bounds__(256 * simtGroups(T)) mvmSimtKernel(MvmProblem 
 #pragma unroll
     for (int kk = 0; kk < BK; kk++) {
       float a[T], b[T];
-      const float posw = PCM ? irPosWeight(k0 + kk, K) : 0.0f;
+      const float posw = PCM ? Ps[buf][PCM ? kk : 0] : 0.0f;
 #pragma unroll
       for (int i = 0; i < T; i++) {
         a[i] = an[i];
