@@ -108,8 +108,9 @@ __host__ __device__ inline int implicitPulses(float c, bool short_train) {
 #endif
 }
 
-// Stream of the device noise of a launch. A batch in which transfers fall is applied in ranges of its rows, a launch
-// each, under one call counter: the first row keeps their draws apart (a whole batch starts at row 0).
+// Stream of the device noise of a launch of the staged kernel. A batch in which transfers fall is applied in ranges of
+// its rows, a launch each, under one call counter: the first row keeps their draws apart (a whole batch starts at
+// row 0).
 __device__ __forceinline__ uint32_t deviceNoiseTag(const UpdateProblem &p) {
   return TAG_DEVICE + (uint32_t)p.s_begin;
 }

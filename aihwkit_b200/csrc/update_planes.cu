@@ -266,6 +266,9 @@ __global__ void __launch_bounds__(256) pulsePlanesKernel(const __grid_constant__
 // ---------------------------------------------------------------------------------------------
 constexpr int UP_WARPS = 4;   // x-lines per CTA (neighbours share the sectors of the x planes)
 constexpr int UP_POOL = kNoisePool; // Gaussians per warp pool (eight per lane and refill)
+// most refills per row: 31 pulses of 32 weights, and up to 31 values of a pool are left when it is refilled
+constexpr uint32_t UP_ROW_REFILLS = 5;
+static_assert(kPulseSegSlots * 32 <= (int)UP_ROW_REFILLS * (UP_POOL - 31), "room for the refills of a row");
 constexpr int UP_DRAIN = 20;  // a lane with more events than this has the warp apply all events
 constexpr int UP_EVENTS = 24; // most events of a lane between two drains
 
@@ -276,10 +279,10 @@ struct UpdatePlanesSmem {
 
 // Eight fresh Gaussians per lane for a warp's pool, as offset + std * z. Out of line: rare against the pulses
 // that take from the pool at two places, and the largest piece of code among them.
-__device__ __noinline__ void refillPool(PhiloxKey key, uint64_t pair, uint32_t call, uint32_t tag, float std,
-                                        float offset, float *column) {
+__device__ __noinline__ void refillPool(PhiloxKey key, uint64_t pair, uint32_t call, float std, float offset,
+                                        float *column) {
   float z[8];
-  gauss8(key, pair, call, tag, z);
+  gauss8(key, pair, call, TAG_DEVICE, z);
 #pragma unroll
   for (int rr = 0; rr < 8; rr++) {
     column[rr * 32] = __fadd_rn(offset, __fmul_rn(std, z[rr]));
@@ -346,7 +349,9 @@ __global__ void __launch_bounds__(32 * UP_WARPS, 8)
   uint32_t triple = 0; // and of three (where trains are longer, the counts are in shared memory)
   const bool deep = *p.plane_max > 3; // some train has more slots than the first four planes hold
   int pool_pos = UP_POOL; // empty
-  uint32_t refills = 0;
+  // Refills are numbered over the whole batch: a batch in which transfers fall is applied in ranges of its rows, a
+  // launch each, and a row takes no more than UP_ROW_REFILLS.
+  uint32_t refills = UP_ROW_REFILLS * (uint32_t)p.s_begin;
   const uint32_t lt_mask = (1u << lane) - 1u;
 
   // one pulse for the lanes in `act`
@@ -358,7 +363,7 @@ __global__ void __launch_bounds__(32 * UP_WARPS, 8)
       if (pool_pos + n_take > UP_POOL) {
         // all lanes refill together; what is left of the old pool is dropped
         __syncwarp();
-        refillPool(p.key, (uint64_t)(task * 32 + lane) | ((uint64_t)refills << 40), p.call, deviceNoiseTag(p), std,
+        refillPool(p.key, (uint64_t)(task * 32 + lane) | ((uint64_t)refills << 40), p.call, std,
                    PulseStep<KIND>::kOnePlus ? 1.0f : 0.0f, pool + lane);
         __syncwarp();
         refills++;
