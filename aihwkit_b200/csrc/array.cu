@@ -261,7 +261,14 @@ __global__ void __launch_bounds__(256)
   }
 }
 
-void TileArray::ensureGradientScratch(size_t need, cudaStream_t s) {
+const float *TileArray::scaledGradient(const float *d, int oi, int m, float factor, long long &ld,
+                                       cudaStream_t s, bool divide) {
+  if (factor == 1.0f) {
+    ld = out_size_;
+    return d + out_off_[oi];
+  }
+  const int cols = out_sizes_[oi];
+  const size_t need = (size_t)m * cols;
   if (need > d_scratch_floats_) {
     AB200_CUDA(cudaStreamSynchronize(s));
     cudaFree(d_scratch_);
@@ -270,23 +277,11 @@ void TileArray::ensureGradientScratch(size_t need, cudaStream_t s) {
     AB200_CUDA(cudaMalloc(&d_scratch_, need * sizeof(float)));
     d_scratch_floats_ = need;
   }
-}
-
-const float *TileArray::scaledGradient(const float *d, int oi, int m, float factor, long long &ld,
-                                       cudaStream_t s, bool divide, size_t offset) {
-  if (factor == 1.0f) {
-    ld = out_size_;
-    return d + out_off_[oi];
-  }
-  const int cols = out_sizes_[oi];
-  const size_t need = (size_t)m * cols;
-  ensureGradientScratch(offset + need, s);
-  float *const dst = d_scratch_ + offset;
-  scaleBlockKernel<<<(unsigned)((need + 255) / 256), 256, 0, s>>>(d + out_off_[oi], out_size_, dst, cols,
+  scaleBlockKernel<<<(unsigned)((need + 255) / 256), 256, 0, s>>>(d + out_off_[oi], out_size_, d_scratch_, cols,
                                                                (long long)need, factor, divide ? 1 : 0);
   AB200_LAUNCH_CHECK();
   ld = cols;
-  return dst;
+  return d_scratch_;
 }
 
 void TileArray::forwardScatter(const float *x_local, int m, float *const *out_table_dev,
@@ -397,30 +392,29 @@ void TileArray::backward(const float *d, float *x_grad, int m, cudaStream_t s) {
 }
 
 // The tiles are independent, and one alone does not fill the GPU to the end: the launches of the bit-plane update
-// are shared by up to eight tiles (1024 x 1024 on four tiles, 256 rows: 12 launches -> 3, 424 -> 322 us).
+// are shared by up to eight tiles (1024 x 1024 on four tiles, 256 rows: 12 launches -> 3, 424 -> 322 us). They divide
+// the gradient by the mapping scales themselves; tiles that go one by one get a scaled copy.
 void TileArray::update(const float *x, const float *d, int m, cudaStream_t s) {
   if (m <= 0) {
     return;
   }
   AB200_CUDA(cudaSetDevice(device_));
   const int n_ol = nOutLocal();
-  size_t slot = 0; // of the scaled gradients, which stay until their launch
-  for (int size : out_sizes_) {
-    slot = std::max(slot, (size_t)m * size);
-  }
-  slot = (slot + 3) & ~(size_t)3; // 16-byte aligned
-  if (scaled_) {
-    ensureGradientScratch(slot * std::min((size_t)kUpdateBatch, tiles_.size()), s);
-  }
   std::vector<UpdateProblem> batch;
   for (int ii = in_begin_; ii < in_end_; ii++) {
     for (int oi = out_begin_; oi < out_end_; oi++) {
       const float alpha =
           scaled_ ? tile_scale_host_[(size_t)(ii - in_begin_) * n_ol + (oi - out_begin_)] : 1.0f;
-      long long ld = 0;
       // pre_update: the gradient is divided by the tile's mapping scale
-      const float *dt = scaledGradient(d, oi, m, alpha, ld, s, /*divide=*/true, slot * batch.size());
-      tile(ii - in_begin_, oi - out_begin_).updateStrided(x + in_off_[ii], in_size_, dt, ld, m, s, &batch);
+      Tile &t = tile(ii - in_begin_, oi - out_begin_);
+      if (t.sharesUpdate(m) && alpha != 0.0f) {
+        t.updateStrided(x + in_off_[ii], in_size_, d + out_off_[oi], out_size_, m, s, &batch,
+                        alpha != 1.0f ? alpha : 0.0f);
+      } else {
+        long long ld = 0;
+        const float *dt = scaledGradient(d, oi, m, alpha, ld, s, /*divide=*/true);
+        t.updateStrided(x + in_off_[ii], in_size_, dt, ld, m, s);
+      }
       if ((int)batch.size() == kUpdateBatch) {
         launchPulsedUpdateTiles(batch.data(), (int)batch.size(), s);
         batch.clear();

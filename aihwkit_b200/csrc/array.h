@@ -81,11 +81,10 @@ private:
   bool scaled_ = false;
   float *bias_dev_ = nullptr;
   const ab200_scatter_plan *plan_ = nullptr; // set only while a scatter forward runs
-  float *d_scratch_ = nullptr; // [tiles of a launch][m][out-split]: gradients times / over the tile scale
+  float *d_scratch_ = nullptr; // [m][largest out-split]: gradients times / over the tile scale
   size_t d_scratch_floats_ = 0;
-  void ensureGradientScratch(size_t need, cudaStream_t s);
   const float *scaledGradient(const float *d, int oi, int m, float factor, long long &ld,
-                              cudaStream_t s, bool divide = false, size_t offset = 0);
+                              cudaStream_t s, bool divide = false);
   std::unique_ptr<TcEngine> tc_;
   std::vector<uint64_t> tc_versions_;
   bool tcEligible(int m);

@@ -1757,12 +1757,22 @@ void Tile::update(const float *x, const float *d, bool bias, int m, bool x_trans
 
 // used by the mapped array: update from sub-blocks of wider activation / gradient matrices
 void Tile::updateStrided(const float *x, long long x_ss, const float *d, long long d_ss, int m, cudaStream_t s,
-                         std::vector<UpdateProblem> *collect) {
-  updateCore(x, x_ss, 1, x_size_, d, d_ss, 1, m, s, collect);
+                         std::vector<UpdateProblem> *collect, float d_div) {
+  updateCore(x, x_ss, 1, x_size_, d, d_ss, 1, m, s, collect, d_div);
+}
+
+// updates on bit planes of single devices, the counting pass aside
+bool Tile::sharesUpdate(int m) const {
+  UpdateProblem u{};
+  u.up = up_;
+  u.nseg = pulseSegments(up_);
+  u.m = m;
+  return !cfg_.mixed.enabled && cfg_.device_kind != AB200_DEVICE_IDEAL &&
+         cfg_.device_kind != AB200_DEVICE_TRANSFER && !pulses_up_ && streamUpdateEligible(u);
 }
 
 void Tile::updateCore(const float *x, long long x_ss, long long x_fs, int x_in, const float *d, long long d_ss,
-                      long long d_fs, int m, cudaStream_t s, std::vector<UpdateProblem> *collect) {
+                      long long d_fs, int m, cudaStream_t s, std::vector<UpdateProblem> *collect, float d_div) {
   requireDevice("update");
   if (m <= 0 || lr_ == 0.0f) {
     return; // "if (!learning_rate) return" (rpu_weight_updater.cpp:206-208)
@@ -1850,8 +1860,9 @@ void Tile::updateCore(const float *x, long long x_ss, long long x_fs, int x_in, 
   u.plane_nk = plane_nk_ ? plane_nk_ + 1 : nullptr; // the first word holds the longest of all
   u.plane_max = plane_nk_;
   const bool planes = streamUpdateEligible(u);
-  if (collect && planes && !pulses_up_ && cfg_.device_kind != AB200_DEVICE_TRANSFER) {
+  if (collect && sharesUpdate(m)) {
     u.w = w_;
+    u.d_div = d_div;
     collect->push_back(u);
     return;
   }

@@ -198,6 +198,7 @@ struct UpdateProblem {
   const float *x;
   long long x_ss, x_fs;
   int x_real; // features >= x_real read as 1.0 (bias)
+  float d_div; // bit planes only: the d values are divided by it (mapping scale of a tile), 0 = taken as they are
   const float *d;
   long long d_ss, d_fs;
   int x_size, d_size, m;
@@ -400,9 +401,11 @@ public:
 
   void backwardStrided(const float *d, long long d_ss, float *x, long long x_ss, int m,
                        bool accumulate, uint32_t noise_id, float out_scale, cudaStream_t s);
-  // (`collect`: an update that several tiles can share a launch for is appended there instead of being run)
+  // (`collect`: an update that several tiles can share a launch for - see sharesUpdate - is appended there instead of
+  // being run, with the gradient to be divided by `d_div`)
   void updateStrided(const float *x, long long x_ss, const float *d, long long d_ss, int m, cudaStream_t s,
-                     std::vector<UpdateProblem> *collect = nullptr);
+                     std::vector<UpdateProblem> *collect = nullptr, float d_div = 0.0f);
+  bool sharesUpdate(int m) const;
 
   const IOEff &fio() const { return f_io_; }
   float *weightsXD() { return w_; }
@@ -427,7 +430,8 @@ private:
                     long long x_fs, int x_store, int m, bool accumulate, uint32_t noise_id,
                     float out_scale, cudaStream_t s, int out_t_rows = 0);
   void updateCore(const float *x, long long x_ss, long long x_fs, int x_in, const float *d, long long d_ss,
-                  long long d_fs, int m, cudaStream_t s, std::vector<UpdateProblem> *collect = nullptr);
+                  long long d_fs, int m, cudaStream_t s, std::vector<UpdateProblem> *collect = nullptr,
+                  float d_div = 0.0f);
   void requireSingleDevice(const char *what);
   void ensurePar3(DeviceStore &ds);
   int opTargets(float *w[2], DeviceStore *ds[2]);

@@ -72,6 +72,8 @@ __global__ void __launch_bounds__(128) pulseStatsKernel(const __grid_constant__ 
     for (int i = threadIdx.x; i < p.d_size; i += 128) {
       dm = fmaxf(dm, fabsf(dr[(long long)i * p.d_fs]));
     }
+    // (rounding keeps the order, so the largest quotient is that of the largest value)
+    dm = N > 1 && p.d_div != 0.0f ? fabsf(__fdiv_rn(dm, p.d_div)) : dm;
     xm = blockMax(xm, sh);
     dm = blockMax(dm, sh);
   }
@@ -154,6 +156,7 @@ __global__ void __launch_bounds__(256) pulsePlanesKernel(const __grid_constant__
   const float *src = is_x ? p.x : p.d;
   const long long ss = is_x ? p.x_ss : p.d_ss, fs = is_x ? p.x_fs : p.d_fs;
   const bool gathered = is_x && p.gather.idx != nullptr;
+  const bool divide = N > 1 && !is_x && p.d_div != 0.0f; // (only tiles of a layer have scales)
   const bool gather_t = gathered && p.gather.idx_t != nullptr;
   const bool direct = gather_t || (!gathered && ss == 1 && fs != 1);
 
@@ -190,6 +193,7 @@ __global__ void __launch_bounds__(256) pulsePlanesKernel(const __grid_constant__
             v = gatherRowElement(p.gather, p.x, rs, line);
           } else {
             v = line < real ? src[(long long)rs * ss + (long long)line * fs] : 1.0f;
+            v = divide ? __fdiv_rn(v, p.d_div) : v;
           }
         }
         tile[h + lane][rr] = v;
@@ -215,6 +219,7 @@ __global__ void __launch_bounds__(256) pulsePlanesKernel(const __grid_constant__
         v[q] = e <= 1 ? (float)e : __ldg(p.x + (long long)img_n * p.gather.image_size + (e - 2));
       } else {
         v[q] = line < real ? src[s + (long long)line * fs] : 1.0f;
+        v[q] = divide ? __fdiv_rn(v[q], p.d_div) : v[q];
       }
     }
   }
@@ -667,7 +672,7 @@ void launchPulsedUpdatePlanes(const UpdateProblem &p, cudaStream_t stream) {
 }
 
 void launchPulsedUpdateTiles(const UpdateProblem *p, int n, cudaStream_t stream) {
-  if (n == 1) {
+  if (n == 1 && p[0].d_div == 0.0f) { // (the kernels of single tiles divide nothing)
     launchPulsePlanes(p[0], stream);
     launchPulsedUpdatePlanes(p[0], stream);
     return;

@@ -240,3 +240,25 @@ def test_noise_of_the_ranges_between_transfers(path, m, every):
     # standard errors (the same draws in every range of r rows spread the sums sqrt(m / r) times as far)
     assert abs(float(change.mean()) - m) <= 5 * std * (m / n) ** 0.5
     assert abs(float(change.std()) / (std * m ** 0.5) - 1) <= 5 * (0.5 / n) ** 0.5
+
+
+def test_scaled_gradients_take_no_memory_of_their_own():
+    """The shared launches divide by the mapping scales themselves: an update of a scaled layer holds no copy of the
+    gradient per tile."""
+    from aihwkit_b200.rpu_base import tiles as T
+    from tests import helpers as H
+
+    size, tile, m = 1024, 256, 4096  # sixteen tiles; a block of the gradient is 4 MB
+    p = H.training_params(noise=False, pulse_det=False)
+    layer = T.TileArray(p._config(tile, tile, H.device("sb", False), seed=5), size, size, tile, tile, cuda_device=0)
+    layer.set_weights(torch.rand(size, size) - 0.5, weight_scaling_omega=0.6)
+    layer.set_learning_rate(0.01)
+    x, d = torch.rand(m, size, device="cuda"), 0.01 * torch.randn(m, size, device="cuda")
+    layer.update(x[:64], d[:64])  # loads the kernels
+    layer.forward(x)
+    layer.backward(d)
+    torch.cuda.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    layer.update(x, d)
+    torch.cuda.synchronize()
+    assert before - torch.cuda.mem_get_info()[0] < m * tile * 4
