@@ -103,3 +103,21 @@ def test_implicit_pulses_of_long_trains():
     t.update(torch.from_numpy(x).cuda(), torch.from_numpy(d).cuda())
     assert np.abs(t.get_weights().numpy() - w).max() <= 1e-6
     assert np.abs(w - before).max() > 1e-3
+
+
+@pytest.mark.parametrize("x_size,d_size", [(1024, 1024), (1023, 1025), (1500, 902)])
+@pytest.mark.parametrize("m", [1, 15, 16, 17])
+def test_floating_point_update_of_few_samples(x_size, d_size, m):
+    """One step of samples on the 64-wide tiles, weights in fours and one by one; 17 samples take two steps."""
+    from aihwkit_b200.rpu_base import tiles as T
+
+    g = torch.Generator().manual_seed(x_size + m)
+    t = T.FloatingPointTile(x_size, d_size, cuda_device=0)
+    w = torch.rand(d_size, x_size, generator=g) - 0.5
+    x, d = torch.rand(m, x_size, generator=g) - 0.5, torch.rand(m, d_size, generator=g) - 0.5
+    t.set_weights(w)
+    t.set_learning_rate(0.25)
+    t.update(x.cuda(), d.cuda())
+    want = w.double() - 0.25 * (d.double().t() @ x.double())
+    # m products of at most 1/4, each sum rounded once, and the step on the weight
+    assert (t.get_weights().double() - want).abs().max() <= (0.25 * m * m * 0.25 + 1.0) * 2.0 ** -24
