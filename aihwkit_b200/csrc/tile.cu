@@ -1768,7 +1768,7 @@ bool Tile::sharesUpdate(int m) const {
   u.nseg = pulseSegments(up_);
   u.m = m;
   return !cfg_.mixed.enabled && cfg_.device_kind != AB200_DEVICE_IDEAL &&
-         cfg_.device_kind != AB200_DEVICE_TRANSFER && !pulses_up_ && streamUpdateEligible(u);
+         cfg_.device_kind != AB200_DEVICE_TRANSFER && !pulses_up_ && planeUpdateEligible(u);
 }
 
 void Tile::updateCore(const float *x, long long x_ss, long long x_fs, int x_in, const float *d, long long d_ss,
@@ -1859,7 +1859,7 @@ void Tile::updateCore(const float *x, long long x_ss, long long x_fs, int x_in, 
   u.plane_ab = plane_ab_;
   u.plane_nk = plane_nk_ ? plane_nk_ + 1 : nullptr; // the first word holds the longest of all
   u.plane_max = plane_nk_;
-  const bool planes = streamUpdateEligible(u);
+  const bool planes = planeUpdateEligible(u);
   if (collect && sharesUpdate(m)) {
     u.w = w_;
     u.d_div = d_div;

@@ -244,8 +244,8 @@ struct UpdateProblem {
 void launchPulsePrepare(const UpdateProblem &p, cudaStream_t stream);
 // Stochastic pulse trains: the update works on bit planes of 32 rows (update_planes.cu). Below one block of
 // rows the planes are mostly empty and the staged kernel's two launches are the shorter way.
-constexpr int kStreamUpdateMinBatch = 32;
-bool streamUpdateEligible(const UpdateProblem &p);
+constexpr int kPlaneUpdateMinRows = 32;
+bool planeUpdateEligible(const UpdateProblem &p);
 // kernel selection of the pulsed update: 0 = automatic, 1 = always the staged kernel, 2 = the
 // bit-plane kernel whenever the pulse type allows it (any batch size)
 void setUpdatePath(int mode);

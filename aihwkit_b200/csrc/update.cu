@@ -559,11 +559,11 @@ template <int KIND> static void launchUpdateDense(const UpdateProblem &p, cudaSt
 static int g_update_path = 0;
 void setUpdatePath(int mode) { g_update_path = mode; }
 
-bool streamUpdateEligible(const UpdateProblem &p) {
+bool planeUpdateEligible(const UpdateProblem &p) {
   if (g_update_path == 1 || p.up.pulse_type != AB200_PULSE_STOCHASTIC_COMPRESSED) {
     return false;
   }
-  return g_update_path == 2 || p.m * (p.nseg > 0 ? p.nseg : 1) >= kStreamUpdateMinBatch;
+  return g_update_path == 2 || p.m * (p.nseg > 0 ? p.nseg : 1) >= kPlaneUpdateMinRows;
 }
 
 void launchPulsePrepare(const UpdateProblem &p, cudaStream_t stream) {

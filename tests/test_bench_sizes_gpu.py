@@ -83,7 +83,7 @@ def test_softbounds_update_conv_tile_stochastic_statistics():
     from aihwkit_b200.rpu_base import tiles as T
 
     rng = np.random.default_rng(32)
-    x_size, d_size, m = 2304, 256, 1536  # large enough for the streaming update kernel
+    x_size, d_size, m = 2304, 256, 1536  # large enough for the bit-plane update kernel
     p = H.training_params(noise=True, pulse_det=False)
     dp = H.device("sb", True, dw_min=0.001, w_max=0.6, w_min=-0.6, dw_min_dtod=0.3)
     cfg = p._config(x_size, d_size, dp, seed=5)
@@ -300,7 +300,7 @@ def test_conv_tile_indexed_on_whole_images():
                                                   ("sbr", 256, 256, 1100)])
 def test_streaming_update_equals_staged_update(kind, x_size, d_size, m):
     """The two kernels of the stochastic pulsed update - blocks of samples staged per weight tile,
-    and the stream over the samples of each x-line that large batches take - see the same pulse
+    and the bit planes that batches of 32 rows and more take - see the same pulse
     trains (same noise key and call counter) and apply the same pulses in the same per-weight
     order: without device noise their results are identical bit for bit."""
     from aihwkit_b200 import _cabi

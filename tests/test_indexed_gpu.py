@@ -290,7 +290,7 @@ def test_indexed_update_equals_update_on_the_unfolded_matrix(which, n_img):
     """update_indexed (the pulse preparation gathers its samples from the images; a compound cuts
     the batch at its transfers) against update on the unfolded matrix with the same seed and
     stochastic pulses: the same samples, the same trains, the same weights and hidden planes bit
-    for bit - small batches (staged kernel) and large ones (streaming kernel)."""
+    for bit - small batches (staged kernel) and large ones (bit planes)."""
     from aihwkit_b200.rpu_base import tiles as T
     from oracle import analog_tile_oracle as O
 

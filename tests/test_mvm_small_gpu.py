@@ -29,8 +29,8 @@ def test_perfect_io_against_float64(m, x_size, d_size):
 @pytest.mark.parametrize("out_size,in_size,max_tile,m", [
     (96, 64, 64, 3), (33, 200, 70, 7), (700, 130, 64, 16), (1536, 384, 192, 21), (100, 2300, 64, 2)])
 def test_mapped_layer_against_its_tiles_one_by_one(out_size, in_size, max_tile, m):
-    """Scaled tiles, bias and all noise on: the layer in one launch against single tiles with the same
-    weights, noise streams and rows, added up in the order of the in-splits."""
+    """Scaled tiles, bias and all noise on: the layer in one launch of the fp32 kernel for small batches against the
+    tensor-core path of the same layer, with the same weights and noise streams."""
     from aihwkit_b200 import _cabi
     from aihwkit_b200.rpu_base import tiles as T
 

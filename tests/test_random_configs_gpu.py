@@ -237,7 +237,7 @@ def test_random_compound_against_reference(seed):
 def test_random_stochastic_updates_agree_between_the_two_kernels(seed):
     """Stochastic pulse trains at random ragged sizes, train lengths (one to four 31-slot
     segments) and device kinds, also through a Tiki-Taka compound: the staged kernel and the
-    streaming kernel see the same trains and apply the same pulses in the same per-weight order,
+    bit-plane kernel see the same trains and apply the same pulses in the same per-weight order,
     so without device noise the weights (and the fast tile) agree bit for bit; and they move."""
     from aihwkit_b200 import _cabi
     from aihwkit_b200.rpu_base import tiles as T

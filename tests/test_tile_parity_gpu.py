@@ -786,7 +786,7 @@ def test_stochastic_rounding_of_pulse_probabilities():
 def test_pulse_counters_account_for_the_weight_change(pulse_det, m, bl):
     """count_pulses: with a noise-free ConstantStep device far from its bounds the weight change
     of every element is (pulses up) * step_up - (pulses down) * step_down, through the staged and
-    the streaming update kernel, one and several train segments, stochastic and implicit pulses;
+    the bit-plane update kernel, one and several train segments, stochastic and implicit pulses;
     the counters add up over calls and are empty for a device that does not count."""
     from aihwkit_b200.rpu_base import tiles as T
 
