@@ -60,9 +60,10 @@ def _pool(task, refill, key):
     return z.reshape(-1).astype(np.float32)
 
 
-def _apply_task(w, hi, lo, up, down, counts, dirs, rows, std, task, key):
+def _apply_task(w, hi, lo, up, down, counts, dirs, rows, std, task, key, rule=None):
     """One x-line and up to 32 d-lines: ``counts`` / ``dirs`` ``[row, lane]``, ``rows`` those in which the
-    x-line pulsed.  Returns the number of pulses of the busiest weight."""
+    x-line pulsed; ``rule(lane, w, down, std * z)``: the weight after a pulse, ConstantStep by default.
+    Returns the number of pulses of the busiest weight."""
     one, n_lanes = np.float32(1), w.size
     state = {"pool": None, "pos": 256, "refills": 0}
 
@@ -80,6 +81,9 @@ def _apply_task(w, hi, lo, up, down, counts, dirs, rows, std, task, key):
             for k in range(max(n)):
                 lanes = [l for l in range(n_lanes) if k < n[l]]
                 for l, z in zip(lanes, take(len(lanes))):
+                    if rule is not None:
+                        w[l] = rule(l, w[l], q[l][r][1], np.float32(std) * z)
+                        continue
                     f = one + np.float32(std) * z
                     w[l] = w[l] - f * down[l] if q[l][r][1] else w[l] + f * up[l]
                     w[l] = max(min(w[l], hi[l]), lo[l])
@@ -165,6 +169,113 @@ def test_pulses_and_noise_event_by_event(x_size, d_size, m, bl, scale, layout):
     # cosine are approximations); a Gaussian given to another pulse moves a weight by about 6e-4
     assert np.abs(got - w).max() <= busiest * 2.0 ** -24
     assert busiest > 3
+
+
+def _rule(kind, mult, col):
+    """Linear step (SoftBounds) and SoftBoundsReference, noise multiplied with the step or added to it; ``col``: the
+    parameters of the lanes by name."""
+    one = np.float32(1)
+
+    def linear(l, w, down, xi):
+        sl, sc = (col["slope_down"][l], col["dwmin_down"][l]) if down else (col["slope_up"][l], col["dwmin_up"][l])
+        dw = (sl * w + sc) * (one + xi) if mult else sl * w + sc * (one + xi)
+        return max(min(w - dw if down else w + dw, col["max_bound"][l]), col["min_bound"][l])
+
+    def reference(l, w, down, xi):
+        sc, bound = ((col["dwmin_down"][l], col["min_bound"][l]) if down
+                     else (col["dwmin_up"][l], col["max_bound"][l]))
+        w = w + col["reference"][l]
+        rest = one - w / bound
+        dw = sc * rest * (one + xi) if mult else sc * (rest + xi)
+        return max(min(w - dw if down else w + dw, col["max_bound"][l]), col["min_bound"][l]) - col["reference"][l]
+
+    return linear if kind in ("ls", "sb") else reference
+
+
+@pytest.mark.parametrize("kind", ["ls", "sb", "sbr"])
+@pytest.mark.parametrize("mult", [False, True])
+@pytest.mark.parametrize("x_size,d_size,m", [(3, 33, 70), (5, 31, 140)])
+def test_noise_multiplied_or_added_event_by_event(kind, mult, x_size, d_size, m):
+    from aihwkit_b200.rpu_base import devices as D
+    from aihwkit_b200.rpu_base import tiles as T
+    from tests import helpers as H
+
+    rng = np.random.default_rng(m)
+    bl, dw_min, std = 3, 0.01, 0.3
+    p = D.AnalogTileParameter()
+    p.update.pulse_type, p.update.desired_bl = D.PulseType.StochasticCompressed, bl
+    p.update.update_management = p.update.update_bl_management = False
+    p.update.fixed_bl = True
+    dp = H.device(kind, True, dw_min=dw_min, dw_min_std=std, mult_noise=mult)
+    if kind == "ls":
+        dp.gamma_up, dp.gamma_down = 0.3, 0.4
+    t = T.AnalogTile(p._config(x_size, d_size, dp, seed=17), cuda_device=0)
+    t.set_seed(1234567)
+    key = (1234567, 0x5BD1E995)
+    t.set_learning_rate(dw_min * bl)  # strength 1
+    x = (rng.uniform(0.4, 0.9, (m, x_size)) * rng.choice([-1, 1], (m, x_size))).astype(np.float32)
+    d = (rng.uniform(0.4, 0.9, (m, d_size)) * rng.choice([-1, 1], (m, d_size))).astype(np.float32)
+    names = t.get_hidden_parameter_names()
+    hp = dict(zip(names, t.get_hidden_parameters().numpy()))
+    w = np.clip(rng.uniform(-0.3, 0.3, (d_size, x_size)), hp["min_bound"], hp["max_bound"]).astype(np.float32)
+    t.set_weights(torch.from_numpy(w))
+    t.update(torch.from_numpy(x).cuda(), torch.from_numpy(d).cuda())
+    got = t.get_weights().numpy()
+
+    unit = np.full(m, np.sqrt(np.float32(dw_min * bl) / (np.float32(dw_min) * np.float32(bl))), np.float32)
+    lengths = np.full(m, bl)
+    px, pd = _trains(x, unit, lengths, bl, key, TAG_X), _trains(d, unit, lengths, bl, key, TAG_D)
+    busiest = 0
+    for j in range(x_size):
+        counts = (px[:, j, None] & pd).sum(-1)
+        rows = np.flatnonzero(px[:, j].any(-1))
+        dirs = (x[:, j, None] > 0) == (d > 0)
+        for i0 in range(0, d_size, 32):
+            s = slice(i0, min(i0 + 32, d_size))
+            col = w[s, j].copy()
+            rule = _rule(kind, mult, {n: v[s, j] for n, v in hp.items()})
+            busiest = max(busiest, _apply_task(col, None, None, None, None, counts[:, s], dirs[:, s], rows, std,
+                                               j * ((d_size + 31) // 32) + i0 // 32, key, rule))
+            w[s, j] = col
+    # two roundings of values below 2 per pulse (the weight, and the weight without its reference) may fall the other
+    # way where the device's Gaussian differs in its last bits; one that belongs to another pulse, or the other form
+    # of the noise, moves a weight by about 3e-3
+    assert np.abs(got - w).max() <= busiest * 2.0 ** -22
+    assert busiest > 20
+
+
+@pytest.mark.parametrize("omega", [0.0, 0.6])
+@pytest.mark.parametrize("kind", ["cs", "sb", "sbr"])
+def test_noisy_tiles_of_a_layer_share_launches(kind, omega):
+    """Device noise on: twelve tiles in shared launches against the same tiles as layers of one tile each."""
+    from aihwkit_b200.rpu_base import tiles as T
+    from tests import helpers as H
+
+    g = torch.Generator().manual_seed(3)
+    out_size, in_size, m = 200, 130, 65
+    p = H.training_params(noise=False, pulse_det=False)
+    cfg = p._config(64, 64, H.device(kind, True, dw_min=0.002, dw_min_dtod=0.3), seed=5)
+    w = torch.rand(out_size, in_size, generator=g) - 0.5
+    x = (torch.rand(m, in_size, generator=g) * 2 - 1).cuda()
+    d = (torch.randn(m, out_size, generator=g) * 0.2).cuda()
+
+    def run(**block):
+        layer = T.TileArray(cfg, out_size, in_size, 64, 64, cuda_device=0, **block)
+        layer.set_seed(9)
+        layer.set_weights(w, weight_scaling_omega=omega)
+        layer.set_learning_rate(0.05)
+        for _ in range(2):
+            layer.update(x, d)
+        return layer.get_weights(), layer.num_in_splits, layer.num_out_splits
+
+    whole, n_in, n_out = run()
+    assert n_in * n_out == 12
+    parts = torch.zeros_like(whole)
+    for i in range(n_in):
+        for o in range(n_out):
+            parts += run(in_split_range=(i, i + 1), out_split_range=(o, o + 1))[0]
+    assert torch.equal(whole, parts)
+    assert (whole - w).abs().max() > 1e-3
 
 
 @pytest.mark.parametrize("out_size,in_size,max_tile,m,omega", [
