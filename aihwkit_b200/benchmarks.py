@@ -16,8 +16,10 @@ Configurations (seeded synthetic inputs with the stated shapes and distributions
 Prints one JSON line: columns/s for the whole step and per phase, and for the update kernel the
 achieved HBM bandwidth on its algorithmic bytes `x*d*(8+P) + 4*m*(x+d)` against the measured copy
 bandwidth (P = per-element parameter bytes: 16 ConstantStep, 24 SoftBounds / SoftBoundsReference).
-For large batches the update is bound by the coincidence arithmetic (x*d*m AND+popc), not by HBM;
-the line then also reports coincidence pairs per second.
+Large batches are far from that bound: the update spends its time on instructions, one Gaussian and one
+device rule per pulse and the bookkeeping of 32 rows at a time around them (profiles of
+pulsedUpdatePlanesKernel: 0.75 of the issue slots). The line reports the rate of (row, weight) pairs beside the
+bandwidth; how many pulses a pair brings depends on the data, so that rate has no peak of its own.
 """
 
 from __future__ import annotations
@@ -115,8 +117,6 @@ def run(config: int, steps: int = 20, warmup: int = 3, batch: int = 0, indexed: 
     """One benchmark line (a dict) for configuration 0, 2 or 3.  ``on_line(line, cfg, x, d, lr)``,
     when given, may extend it (``bench.py --config N`` adds the CPU baseline of the compiled
     reference there)."""
-    import ctypes as C
-
     import torch
 
     from . import _cabi
@@ -214,8 +214,6 @@ def run(config: int, steps: int = 20, warmup: int = 3, batch: int = 0, indexed: 
     mvm_bytes = 4 * m * (x_size + d_size) + 4 * x_size * d_size
     flops = 2.0 * m * x_size * d_size
     pairs = float(x_size) * d_size * m
-    popc = C.c_double(0.0)
-    _cabi.check(lib.ab200_measure_popc_peak(0, C.byref(popc)))
 
     def mvm_roofline(t_ms, n_launch):
         tf = flops / (t_ms * 1e-3) / 1e12
@@ -240,13 +238,11 @@ def run(config: int, steps: int = 20, warmup: int = 3, batch: int = 0, indexed: 
         "forward_roofline": mvm_roofline(t_f, launches[0]),
         "backward_roofline": mvm_roofline(t_b, launches[1]),
         "update_roofline": {
-            "bound": "integer" if pairs / (popc.value or 1.0) > upd_bytes / (hbm * 1e9) else "hbm",
+            "bound": "hbm" if upd_bytes / (t_u * 1e-3) / 1e9 / hbm > 0.5 else "instructions and latency",
             "algorithmic_bytes": upd_bytes,
             "achieved": upd_bytes / (t_u * 1e-3) / 1e9, "peak": hbm, "unit": "GB/s",
             "frac": upd_bytes / (t_u * 1e-3) / 1e9 / hbm, "peak_source": src,
             "coincidence_pairs_per_s": pairs / (t_u * 1e-3),
-            "popc_pairs_per_s_peak": popc.value,
-            "frac_of_popc_peak": pairs / (t_u * 1e-3) / (popc.value or 1.0),
             "launches": launches[2], "launch_floor_ms": launches[2] * floor_us * 1e-3,
         },
         "peak_sources": {"hbm": src, "bf16": bf16_src},
