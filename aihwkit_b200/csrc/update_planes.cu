@@ -306,7 +306,10 @@ __device__ __noinline__ void refillPool(PhiloxKey key, uint64_t pair, uint32_t c
 // refill; the busiest lane sets the number of rounds, 0.66 of the lanes have an event in one. A list of
 // {coincidences, directions} words in shared memory instead of the queue of bits took 7 % fewer instructions
 // and the same time (24 instead of 32 warps per SM).
-template <int KIND, bool NOISY, bool MULT, int N>
+//
+// SHORT: a range of one row, of a batch that transfers cut up; x-lines without a pulse in it are left out before
+// their weights are read.
+template <int KIND, bool NOISY, bool MULT, int N, bool SHORT>
 __global__ void __launch_bounds__(32 * UP_WARPS, 8)
     pulsedUpdatePlanesKernel(const __grid_constant__ UpdateBatch<N> batch) {
   const UpdateProblem &p = AB200_BATCH_TILE(blockIdx.y);
@@ -323,6 +326,14 @@ __global__ void __launch_bounds__(32 * UP_WARPS, 8)
   const int i = dblk * 32 + lane;
   const bool i_ok = i < p.d_size;
   const long long idx = (long long)j * p.d_size + (i_ok ? i : 0);
+  if (SHORT && *p.plane_max <= 3) {
+    // an x-line without a pulse in the range leaves the weights and their parameters where they are
+    const uint4 xv = reinterpret_cast<const uint4 *>(p.xw)[(long long)(p.s_begin >> 5) * 8 * p.x_size + j];
+    const uint32_t rows = (0xffffffffu << (p.s_begin & 31)) & (0xffffffffu >> (31 - ((p.s_end - 1) & 31)));
+    if (((xv.y | xv.z | xv.w) & rows) == 0u) {
+      return;
+    }
+  }
   float w = 0.0f;
   PulseStep<KIND> step;
   {
@@ -590,8 +601,15 @@ static void launchPlanesInstance(const UpdateBatch<N> &batch, int n, cudaStream_
     const UpdateProblem &p = batch.tile[k];
     blocks = std::max(blocks, (long long)((p.d_size + 31) / 32) * ((p.x_size + UP_WARPS - 1) / UP_WARPS));
   }
-  AB200_CUDA(launchChained(pulsedUpdatePlanesKernel<KIND, NOISY, MULT, N>, dim3((unsigned)blocks, n),
-                           dim3(32 * UP_WARPS), 0, stream, batch));
+  auto kernel = pulsedUpdatePlanesKernel<KIND, NOISY, MULT, N, false>;
+  const UpdateProblem &p = batch.tile[0];
+  // Weights and parameters of a large tile are most of what a launch over one row takes: a transfer after every row,
+  // us per 64 rows, 1024 x 1024 2764 -> 2481, 512 x 512 1096 -> 1077. In small tiles and with more rows the look at the
+  // line first costs more than it spares (64 x 64 566 -> 599; 1024 x 1024, a transfer after five rows, 627 -> 643).
+  if (N == 1 && p.m > 1 && p.s_end - p.s_begin == 1 && (long long)p.x_size * p.d_size >= 1 << 18) {
+    kernel = pulsedUpdatePlanesKernel<KIND, NOISY, MULT, N, N == 1>;
+  }
+  AB200_CUDA(launchChained(kernel, dim3((unsigned)blocks, n), dim3(32 * UP_WARPS), 0, stream, batch));
 }
 
 template <int KIND, int N> static void launchPlanesKind(const UpdateBatch<N> &batch, int n, cudaStream_t stream) {

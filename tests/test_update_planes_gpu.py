@@ -373,3 +373,32 @@ def test_scaled_gradients_take_no_memory_of_their_own():
     layer.update(x, d)
     torch.cuda.synchronize()
     assert before - torch.cuda.mem_get_info()[0] < m * tile * 4
+
+
+@pytest.mark.parametrize("x_size,d_size,m,every", [(512, 512, 40, 1.0), (300, 1000, 37, 1.0), (300, 1000, 70, 7.0)])
+def test_ranges_of_one_row_in_large_tiles(x_size, d_size, m, every):
+    """A transfer after every row, in tiles whose lines are looked at before their weights are read, and longer ranges
+    of the same: against the staged kernel, device noise off, bit for bit, the slow tile included."""
+    from aihwkit_b200 import _cabi
+    from aihwkit_b200.rpu_base import tiles as T
+    from tests import helpers as H
+
+    g = torch.Generator().manual_seed(m)
+    p = H.training_params(noise=False, pulse_det=False)
+    x = (torch.rand(m, x_size, generator=g) * 2 - 1).cuda()
+    x[torch.rand(m, x_size, generator=g).cuda() < 0.3] = 0.0
+    d = (torch.randn(m, d_size, generator=g) * 0.2).cuda()
+    out = []
+    lib = _cabi.lib()
+    try:
+        for path in (0, 1):
+            _cabi.check(lib.ab200_set_update_path(path))
+            t = T.AnalogTile(p._config(x_size, d_size, H.transfer_device(False, transfer_every=every,
+                                                                         units_in_mbatch=False), seed=3), cuda_device=0)
+            t.set_learning_rate(0.05)
+            t.update(x, d)
+            out.append((t.get_weights(), t.get_hidden_parameters()))
+    finally:
+        _cabi.check(lib.ab200_set_update_path(0))
+    assert torch.equal(out[0][0], out[1][0]) and torch.equal(out[0][1], out[1][1])
+    assert out[0][1].abs().sum() > 0
