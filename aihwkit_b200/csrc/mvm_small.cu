@@ -10,8 +10,9 @@
 // digital bias.
 //
 // Measured, 16 rows: 768 -> 3072 on 2 x 6 tiles 267 -> 15.4 us (24 launches -> 1), 1024 x 1024 42 -> 17.5 us, one row
-// through 512 x 512 20 -> 5.4 us on the GPU. Bound by latency: of a step's about 10 k cycles the loads take
-// 3 k, the product 4 k, quantising 1 k; the rest is the output stage of a tile.
+// through 512 x 512 20 -> 5.4 us on the GPU. Bound by latency: a chain of load, reduce, quantise, product and output
+// stage on sixteen warps per SM, 0.4 of the issue slots used; waits for shared memory, for the instruction before
+// and at the barriers about alike.
 //
 // Weights, products and sums stay fp32. Element-wise semantics are the helpers of mvm_common.cuh, with the
 // noise counters of the other kernels.
@@ -377,8 +378,8 @@ int smallMvmMaxCtas(int in_size) {
   // Four rounds of one CTA per SM; with more, the 64 x 64 tiles of the general kernel fill the GPU as well and
   // load less per product. 2048 x 2048, forward, this kernel against the general one: 16 rows (64 CTAs) 28
   // against 91 us, 64 rows (256) 56 against 179; 4096 x 4096, 32 rows (256) 109 against 367.
-  // Short rows leave most of a CTA's 512 features empty: 64 x 64, 4000 rows (500 CTAs) 22.6 against 17.9 us, but
-  // 128 x 128, 1000 rows (252) 13.3 against 15.4.
+  // Short rows give a CTA little to hide its barriers behind: 64 x 64, 4000 rows (500 CTAs) 13.9 against 15.5 us, but
+  // transposed 16.4 against 12.0, and 32 x 300, 900 rows (570) 13.8 against 11.2.
   return (in_size > 128 ? 4 : 2) * smCount();
 }
 

